@@ -312,7 +312,7 @@ def _exact_grid(g, steps):
     def table(v):  # a media-table value per cell
         if g.media is None:
             return v[0]
-        return torch.where(g.media > 0, v[1], v[0]).double()
+        return torch.tensor(v, dtype=torch.float64, device="cuda")[g.media.long()]
 
     K = g.K.double() if g.K is not None else table(list(m.K))
     phi = g.phi.double() if g.phi is not None else table(list(m.m))
