@@ -41,7 +41,8 @@ enum { GBF_SOURCE_DIRICHLET_PATCH = 0, /* reference: S2 = S2_gr on the top patch
 enum { GBF_BC_REFERENCE = 0,           /* reference Border_S2/Border_P1 rules           */
        GBF_BC_HYDROSTATIC_SIDES = 1 }; /* Dirichlet hydrostatic P on i/k sides,
                                           no-flow bottom face for both phases          */
-enum { GBF_PREC_F64 = 0,               /* plain FP64 state and arithmetic               */
+enum { GBF_PREC_F64 = 0,               /* FP64 state; a step's increments to FP64 accuracy of
+                                          the state (FP32 pairs where that is faster)   */
        GBF_PREC_SPLIT = 1,             /* FP32 P,S,K,fluxes; phase masses at least as precise
                                           as FP64: FP32-pair defects over the state's exact
                                           FP32-product mass; after the FP32 Newton step one
@@ -87,7 +88,9 @@ typedef struct gbf_model {
   int bc_mode;                    /* GBF_BC_* */
   double kv;                      /* vertical/horizontal permeability ratio (1 = isotropic) */
   double newton_tol;              /* 0: always run newton_iterations (reference);
-                                     >0: stop once |dS| and |dP|/P_atm fall below it */
+                                     >0: stop once |dS| and |dP|/P_atm fall below it.
+                                     FP64 domains and ensembles of 7 or more iterations
+                                     solve to round-off whatever its value */
 } gbf_model;
 
 /*
@@ -190,7 +193,7 @@ int gbf_boundary_f64_noalloc(const gbf_model* m, gbf_arrays d_arrays, void* stre
 
 /* ------------------------------------------------------- single domain ----
  * One grid whose state lives in HBM between steps. `precision` is
- * GBF_PREC_F64 (plain FP64: two passes per step — properties, then fluxes,
+ * GBF_PREC_F64 (FP64 state: two passes per step — properties, then fluxes,
  * mass update and Newton fused — plus a face pass for the boundaries) or
  * GBF_PREC_SPLIT (FP32 P, S, K, phi and fluxes; per-cell phase masses at
  * least as precise as FP64, as FP32-pair defects), GBF_PREC_SPLIT_DF (the

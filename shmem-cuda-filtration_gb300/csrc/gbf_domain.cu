@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "gbf_domain.h"
+#include "gbf_f64_pair.cuh"
 #include "gbf_split.h"
 
 GbfDerived gbf_derive(const gbf_model& m) {
@@ -45,6 +46,13 @@ namespace {
 int alloc_f64_work(gbf_domain* d) {
   const size_t n = gbf_geo(d->m).n, b = n * sizeof(double);
   int s = GBF_OK;
+  if (gbf_pair_applies(d->m)) {
+    s |= gbf_domain_alloc(d, (void**)&d->pair_work, 4 * n * sizeof(float2));
+    s |= gbf_domain_alloc(d, (void**)&d->pair_rows, sizeof(GbfPairRow) * (size_t)d->m.ny);
+    if (!s) s |= gbf_pair_fill_rows(d->m, d->pair_rows, d->stream);
+    d->pair_consts.reset(new GbfPairConsts(gbf_pair_consts(d->m)));
+    return s ? GBF_ERR_NOMEM : GBF_OK;
+  }
   s |= gbf_domain_alloc(d, (void**)&d->L1, b);
   s |= gbf_domain_alloc(d, (void**)&d->L2, b);
   s |= gbf_domain_alloc(d, (void**)&d->ro1, b);
@@ -82,10 +90,24 @@ void free_all(gbf_domain* d) {
 int f64_step(gbf_domain* d, int props_flags) {
   const int nxt = d->cur ^ 1;
   GbfF64Step s = {};
+  GbfPairWork pw = {};
+  if (d->pair_work) {
+    const size_t n = gbf_geo(d->m).n;
+    pw.D = d->pair_work;
+    pw.L1 = pw.D + n;
+    pw.L2 = pw.L1 + n;
+    pw.Pk = pw.L2 + n;
+    pw.rows = d->pair_rows;
+  }
   if (d->borrowed) {
-    const size_t b = gbf_geo(d->m).n * sizeof(double);
-    GBF_CUDA(cudaMemcpyAsync(d->P[1], d->P[0], b, cudaMemcpyDeviceToDevice, d->stream));
-    GBF_CUDA(cudaMemcpyAsync(d->S[1], d->S[0], b, cudaMemcpyDeviceToDevice, d->stream));
+    if (d->pair_work) {  // pass 1 reads the caller's arrays and leaves the copy
+      pw.P_from = d->P[0];
+      pw.S_from = d->S[0];
+    } else {
+      const size_t b = gbf_geo(d->m).n * sizeof(double);
+      GBF_CUDA(cudaMemcpyAsync(d->P[1], d->P[0], b, cudaMemcpyDeviceToDevice, d->stream));
+      GBF_CUDA(cudaMemcpyAsync(d->S[1], d->S[0], b, cudaMemcpyDeviceToDevice, d->stream));
+    }
     s.P = d->P[1];
     s.S = d->S[1];
     s.Pn = d->P[0];
@@ -114,7 +136,8 @@ int f64_step(gbf_domain* d, int props_flags) {
     s.ro1 = d->caller.ro1;
     s.ro2 = d->caller.ro2;
   }
-  int st = gbf_f64_launch_step(d->m, d->d, d->cells, s, props_flags, mass_out, d->stream, &d->timer);
+  int st = gbf_f64_launch_step(d->m, d->d, d->cells, s, d->pair_consts.get(), d->pair_work ? &pw : nullptr, props_flags,
+                               mass_out, d->stream, &d->timer);
   if (st) return st;
   if (d->borrowed)
     d->lazy_dirty = true;
@@ -423,6 +446,17 @@ int gbf_domain_download(gbf_domain* d, int field, double* host) {
   const size_t n = gbf_geo(d->m).n, b = n * sizeof(double);
   if (d->precision != GBF_PREC_F64) return gbf_split_download(d, field, host);
   const double* src = nullptr;
+  if (d->pair_work && (field == GBF_FIELD_RO1 || field == GBF_FIELD_RO2)) {
+    // the densities of the state the last step started from (the other buffer)
+    double* tmp = nullptr;
+    GBF_CUDA(cudaMallocAsync((void**)&tmp, b, d->stream));
+    int s = gbf_density_launch(d->m, field == GBF_FIELD_RO1 ? 1 : 2, d->P[d->steps > 0 ? d->cur ^ 1 : d->cur], tmp,
+                               d->stream);
+    if (!s) s = gbf_cuda_check(cudaMemcpyAsync(host, tmp, b, cudaMemcpyDeviceToHost, d->stream), "copy density");
+    cudaFreeAsync(tmp, d->stream);
+    if (!s) s = gbf_cuda_check(cudaStreamSynchronize(d->stream), "gbf_domain_download");
+    return s;
+  }
   switch (field) {
     case GBF_FIELD_P1: src = d->P[d->cur]; break;
     case GBF_FIELD_S2: src = d->S[d->cur]; break;
@@ -587,6 +621,10 @@ int gbf_dropin_defer(gbf_domain* d, const gbf_model& m, int stage) {
     if (int s = gbf_dropin_writeback(d)) return s;
     d->m = m;
     d->d = gbf_derive(m);
+    if (d->pair_work) {  // fused mode: its constants and row table
+      *d->pair_consts = gbf_pair_consts(m);
+      if (int s = gbf_pair_fill_rows(m, d->pair_rows, d->stream)) return s;
+    }
     if (d->precision != GBF_PREC_F64) {  // split mode: its row constants, and the state formed anew
       if (int s = gbf_split_fill_rows(d->m, d->split_rows, d->stream)) return s;
       d->split_stale = true;

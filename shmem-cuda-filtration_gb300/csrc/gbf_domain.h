@@ -2,6 +2,7 @@
 // shared by the FP64, split-precision and drop-in code (not installed).
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "gbf_internal.h"
@@ -40,10 +41,14 @@ struct GbfF64Step {
 // Device status bits (OR-ed by kernels, read by gbf_domain_status).
 enum { GBF_DEV_NONFINITE = 1u, GBF_DEV_TIMEOUT = 2u };
 
-// FP64 launchers (gbf_f64.cu).
+// FP64 launchers (gbf_f64.cu). `pair` (with its constants): the step in
+// increment form (gbf_f64_pair.cuh); NULL: the plain FP64 passes.
+struct GbfPairConsts;
+struct GbfPairWork;
 unsigned gbf_f64_flux_grid(const gbf_model& m);
 int gbf_f64_launch_step(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells, const GbfF64Step& s,
-                        int props_flags, double* mass_out, cudaStream_t st, GbfTimer* tm);
+                        const GbfPairConsts* pc, const GbfPairWork* pair, int props_flags, double* mass_out,
+                        cudaStream_t st, GbfTimer* tm);
 
 struct gbf_domain {
   gbf_model m;
@@ -59,7 +64,11 @@ struct gbf_domain {
   // FP64 state and props
   double *P[2] = {nullptr, nullptr}, *S[2] = {nullptr, nullptr};
   int cur = 0;
-  double *L1 = nullptr, *L2 = nullptr, *ro1 = nullptr, *ro2 = nullptr, *lnSe = nullptr;
+  double *L1 = nullptr, *L2 = nullptr, *ro1 = nullptr, *ro2 = nullptr, *lnSe = nullptr;  // plain FP64 passes
+  // the pair step (gbf_f64_pair.cuh): constants, work arrays, row table
+  std::unique_ptr<GbfPairConsts> pair_consts;
+  float2* pair_work = nullptr;  // D, L1, L2, P_k: n each
+  struct GbfPairRow* pair_rows = nullptr;
   gbf_arrays outs = {};  // optional reference arrays (velocity, masses, Xi, P2)
   // split-precision state (gbf_split.cu)
   float *Pf[2] = {nullptr, nullptr}, *Sf[2] = {nullptr, nullptr};
@@ -104,6 +113,9 @@ int gbf_domain_alloc(gbf_domain* d, void** p, size_t bytes);
 // and S NULL, from a split state (dPf, Sf); boundary cells 0 (gbf_eager.cu).
 int gbf_roS_old_launch(const gbf_model& m, const double* P, const double* S, const float* dPf, const float* Sf,
                        double* o1, double* o2, cudaStream_t st);
+
+// The density of phase 1 or 2 of a pressure field (gbf_f64.cu).
+int gbf_density_launch(const gbf_model& m, int phase, const double* P, double* out, cudaStream_t st);
 
 // Drop-in helpers (gbf_domain.cu).
 // precision: GBF_PREC_F64 (the fused mode) or a split form (the split mode).

@@ -5,8 +5,9 @@
 // (member, x-tile, y-tile, k-range) of all members; CTAs take tiles from an
 // atomic counter (dynamic balance of uneven members) and run the z-marching
 // tile of gbf_split_tile.cuh with the member's constants copied to shared
-// memory. Plain FP64: the two passes of gbf_f64_cell.cuh over packed chunk
-// lists of all members' cells. Then one face pass over all members'
+// memory. Plain FP64: the two passes of gbf_f64_pair.cuh (or, for models of
+// fewer than 7 Newton iterations, gbf_f64_cell.cuh) over packed chunk lists of
+// all members' cells. Then one face pass over all members'
 // boundary cells and one per-member phase-mass reduction. A step is a CUDA
 // graph (counter reset, step, faces, masses), captured once per buffer parity.
 //
@@ -20,6 +21,7 @@
 #include <vector>
 
 #include "gbf_f64_cell.cuh"
+#include "gbf_f64_pair.cuh"
 #include "gbf_split_tile.cuh"
 
 namespace {
@@ -35,6 +37,8 @@ struct EnsMember {
   float* Sf[2];
   double *M1, *M2;
   double *L1, *L2, *ro1, *ro2, *lnSe;
+  GbfPairConsts pc64;  // the pair step (gbf_f64_pair.cuh; pw.D NULL: the plain FP64 passes)
+  GbfPairWork pw;
   int part_begin, part_end;  // this member's slots in the partial-sum array
   double k1v;                // defect form: water-mass part left out of the tiles' sums (gbf_defect_k1)
   unsigned long long off;    // first cell of this member in the packed all-members layout
@@ -63,7 +67,9 @@ const bool kShapePairs[kShapes] = {false, false, false, true, true, true};
 // grid whose nx is 16 more than a multiple of 32 (nx >= 48).
 constexpr int kWideTX = 48, kWideTY = 10;
 bool mixed_wide_tail(int nx) { return nx >= 48 && nx % 32 > 0 && nx % 32 <= 16; }
-constexpr int kChunkCells = 16384, kBoundaryChunk = 4096, kThreads = 256;
+// Chunks of 4096 cells: with 16384, seven million cells are 440 blocks, less
+// than one wave of the FP64 passes (363 us against 226 for the flux pass).
+constexpr int kChunkCells = 4096, kBoundaryChunk = 4096, kThreads = 256;
 
 // ------------------------------------------------------------ split kernels
 
@@ -321,16 +327,19 @@ __device__ __forceinline__ GbfF64Step ens_f64_step(const EnsMember& me, int cur)
   return s;
 }
 
+// A member's descriptor to shared memory.
+__device__ __forceinline__ void ens_copy_member(EnsMember& me, const EnsMember* src_) {
+  const int* src = reinterpret_cast<const int*>(src_);
+  int* dst = reinterpret_cast<int*>(&me);
+  for (int q = threadIdx.x; q < (int)(sizeof(EnsMember) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(kThreads) k_ens_f64_props(const EnsMember* __restrict__ mem,
                                                             const EnsChunk* __restrict__ chunks, int cur) {
   __shared__ EnsMember me;
   const EnsChunk ch = chunks[blockIdx.x];
-  {
-    const int* src = reinterpret_cast<const int*>(mem + ch.member);
-    int* dst = reinterpret_cast<int*>(&me);
-    for (int q = threadIdx.x; q < (int)(sizeof(EnsMember) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
-  }
-  __syncthreads();
+  ens_copy_member(me, mem + ch.member);
   const GbfGeo g = gbf_geo(me.m);
   const GbfF64Step s = ens_f64_step(me, cur);
   for (unsigned c = ch.begin + threadIdx.x; c < ch.end; c += blockDim.x) gbf_f64_props_cell(me.m, me.d, me.cells, s, 0, g, c);
@@ -341,12 +350,7 @@ __global__ void __launch_bounds__(kThreads) k_ens_f64_flux_newton(const EnsMembe
                                                                   double* partials, unsigned* status) {
   __shared__ EnsMember me;
   const EnsChunk ch = chunks[blockIdx.x];
-  {
-    const int* src = reinterpret_cast<const int*>(mem + ch.member);
-    int* dst = reinterpret_cast<int*>(&me);
-    for (int q = threadIdx.x; q < (int)(sizeof(EnsMember) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
-  }
-  __syncthreads();
+  ens_copy_member(me, mem + ch.member);
   const GbfGeo g = gbf_geo(me.m);
   const GbfF64Step s = ens_f64_step(me, cur);
   const unsigned ix = g.nx - 2, iy = g.ny - 2;
@@ -367,6 +371,44 @@ __global__ void __launch_bounds__(kThreads) k_ens_f64_boundary(const EnsMember* 
   const GbfGeo g = gbf_geo(me.m);
   const GbfF64Step s = ens_f64_step(me, cur);
   for (unsigned t = ch.begin + threadIdx.x; t < ch.end; t += blockDim.x) gbf_f64_boundary_cell(me.m, s, g, t);
+}
+
+// The pair step's two passes over the same chunk lists.
+__global__ void __launch_bounds__(kThreads) k_ens_pair_props(const EnsMember* __restrict__ mem,
+                                                             const EnsChunk* __restrict__ chunks, int cur) {
+  __shared__ EnsMember me;
+  const EnsChunk ch = chunks[blockIdx.x];
+  ens_copy_member(me, mem + ch.member);
+  const GbfF64Step s = ens_f64_step(me, cur);
+  for (unsigned c = ch.begin + threadIdx.x; c < ch.end; c += blockDim.x)
+    gbf_pair_props_cell<false>(me.pc64, me.cells, s, me.pw, c);
+}
+
+template <bool MASS>
+__global__ void __launch_bounds__(kThreads, 4) k_ens_pair_step(const EnsMember* __restrict__ mem,
+                                                            const EnsChunk* __restrict__ chunks, int cur,
+                                                            double* partials, unsigned* status) {
+  __shared__ EnsMember me;
+  const EnsChunk ch = chunks[blockIdx.x];
+  ens_copy_member(me, mem + ch.member);
+  const GbfF64Step s = ens_f64_step(me, cur);
+  const GbfPairConsts& C = me.pc64;
+  GbfPairMass acc;
+  unsigned bad = 0;
+  for (unsigned t = ch.begin + threadIdx.x; t < ch.end; t += blockDim.x) {
+    const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
+    const unsigned i = 1u + t - r * C.dix.d, j = 1u + r - q * C.diy.d, k = 1u + q;
+    gbf_pair_step_cell<MASS>(C, me.cells, s, me.pw, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc,
+                             bad);
+  }
+  if (bad) atomicOr(status, GBF_DEV_NONFINITE);
+  if (MASS) gbf_block_sum2<kThreads>(acc.m1 - pf_to_double(acc.r1), acc.m2, me.d.V, partials + 2 * blockIdx.x);
+}
+
+__global__ void k_ens_pair_rows(const EnsMember* __restrict__ mem) {
+  const EnsMember& me = mem[blockIdx.x];
+  GbfPairRow* rows = const_cast<GbfPairRow*>(me.pw.rows);
+  for (int j = threadIdx.x; j < me.m.ny; j += blockDim.x) rows[j] = gbf_pair_row(me.m, j);
 }
 
 // Per-member phase masses of this step: one block per member sums its
@@ -491,6 +533,7 @@ struct gbf_ensemble {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int cur = 0;
+  bool pair = false;       // FP64: the pair step (every member's model qualifies)
   bool any_patch = false;  // a split member under a Dirichlet patch: PATCH tiles and the step's pre-pass
   int shape = kShape32x8;
   std::map<int, int> kchunk_by_edge;  // fusion depth per member edge (0 = default rule)
@@ -784,6 +827,20 @@ int launch_split_step(gbf_ensemble* e, double* partials, cudaStream_t st, const 
 }
 
 // Enqueue one step on `st` (also used under stream capture).
+// The FP64 passes over chunks [p0, p0 + np) of the cells and [f0, f0 + nf) of the interior cells.
+void enqueue_f64(gbf_ensemble* e, int p0, int np, int f0, int nf, int cur, double* partials, cudaStream_t st,
+                 GbfTimer* tm) {
+  cudaEvent_t ev = gbf_timer_begin(tm, st);
+  if (e->pair) k_ens_pair_props<<<(unsigned)np, kThreads, 0, st>>>(e->d_mem, e->d_props + p0, cur);
+  else k_ens_f64_props<<<(unsigned)np, kThreads, 0, st>>>(e->d_mem, e->d_props + p0, cur);
+  gbf_timer_end(tm, GBF_K_ENS_PROPS, ev, st);
+  ev = gbf_timer_begin(tm, st);
+  if (!e->pair) k_ens_f64_flux_newton<<<(unsigned)nf, kThreads, 0, st>>>(e->d_mem, e->d_flux + f0, cur, partials, e->d_status);
+  else if (partials) k_ens_pair_step<true><<<(unsigned)nf, kThreads, 0, st>>>(e->d_mem, e->d_flux + f0, cur, partials, e->d_status);
+  else k_ens_pair_step<false><<<(unsigned)nf, kThreads, 0, st>>>(e->d_mem, e->d_flux + f0, cur, nullptr, e->d_status);
+  gbf_timer_end(tm, GBF_K_ENS_FLUX_NEWTON, ev, st);
+}
+
 int enqueue_step(gbf_ensemble* e, cudaStream_t st) {
   const bool mass = (e->out_flags & GBF_OUT_MASS) && e->d_mass_hist;
   double* partials = mass ? e->d_partials : nullptr;
@@ -803,13 +860,7 @@ int enqueue_step(gbf_ensemble* e, cudaStream_t st) {
       k_ens_split_boundary<<<(unsigned)e->bnd.size(), kThreads, 0, st>>>(e->d_mem, e->d_bnd, e->cur);
     gbf_timer_end(tm, GBF_K_ENS_BOUNDARY, ev, st);
   } else {
-    ev = gbf_timer_begin(tm, st);
-    k_ens_f64_props<<<(unsigned)e->props.size(), kThreads, 0, st>>>(e->d_mem, e->d_props, e->cur);
-    gbf_timer_end(tm, GBF_K_ENS_PROPS, ev, st);
-    ev = gbf_timer_begin(tm, st);
-    k_ens_f64_flux_newton<<<(unsigned)e->flux.size(), kThreads, 0, st>>>(e->d_mem, e->d_flux, e->cur, partials,
-                                                                         e->d_status);
-    gbf_timer_end(tm, GBF_K_ENS_FLUX_NEWTON, ev, st);
+    enqueue_f64(e, 0, (int)e->props.size(), 0, (int)e->flux.size(), e->cur, partials, st, tm);
     ev = gbf_timer_begin(tm, st);
     k_ens_f64_boundary<<<(unsigned)e->bnd.size(), kThreads, 0, st>>>(e->d_mem, e->d_bnd, e->cur);
     gbf_timer_end(tm, GBF_K_ENS_BOUNDARY, ev, st);
@@ -867,9 +918,7 @@ int enqueue_group_step(gbf_ensemble* e, int r0, int r1, int cur, unsigned* count
     else
       k_ens_split_boundary<<<(unsigned)(b.bnd - a.bnd), kThreads, 0, st>>>(e->d_mem, e->d_bnd + a.bnd, cur);
   } else {
-    k_ens_f64_props<<<(unsigned)(b.props - a.props), kThreads, 0, st>>>(e->d_mem, e->d_props + a.props, cur);
-    k_ens_f64_flux_newton<<<(unsigned)(b.flux - a.flux), kThreads, 0, st>>>(e->d_mem, e->d_flux + a.flux, cur,
-                                                                           nullptr, e->d_status);
+    enqueue_f64(e, a.props, b.props - a.props, a.flux, b.flux - a.flux, cur, nullptr, st, nullptr);
     k_ens_f64_boundary<<<(unsigned)(b.bnd - a.bnd), kThreads, 0, st>>>(e->d_mem, e->d_bnd + a.bnd, cur);
   }
   cudaError_t err = cudaGetLastError();
@@ -939,6 +988,8 @@ int gbf_ensemble_create(int n, const gbf_model* models, const gbf_cells* host_ce
   if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess) s = gbf_fail(GBF_ERR_CUDA, "stream");
   e->own_stream = true;
   const bool split = precision != GBF_PREC_F64;
+  e->pair = !split;
+  for (int r = 0; r < n; r++) e->pair = e->pair && gbf_pair_applies(models[r]);
   for (int r = 0; r < n && !s; r++) {
     const gbf_model& m = models[r];
     const size_t nc = gbf_geo(m).n;
@@ -981,8 +1032,15 @@ int gbf_ensemble_create(int n, const gbf_model* models, const gbf_cells* host_ce
         s |= ens_alloc(e, (void**)&me.P[b], nc * sizeof(double));
         s |= ens_alloc(e, (void**)&me.S[b], nc * sizeof(double));
       }
-      double** w[] = {&me.L1, &me.L2, &me.ro1, &me.ro2, &me.lnSe};
-      for (double** p : w) s |= ens_alloc(e, (void**)p, nc * sizeof(double));
+      if (e->pair) {
+        me.pc64 = gbf_pair_consts(m);
+        float2** w[] = {&me.pw.D, &me.pw.L1, &me.pw.L2, &me.pw.Pk};
+        for (float2** p : w) s |= ens_alloc(e, (void**)p, nc * sizeof(float2));
+        s |= ens_alloc(e, (void**)&me.pw.rows, sizeof(GbfPairRow) * (size_t)m.ny);
+      } else {
+        double** w[] = {&me.L1, &me.L2, &me.ro1, &me.ro2, &me.lnSe};
+        for (double** p : w) s |= ens_alloc(e, (void**)p, nc * sizeof(double));
+      }
     }
   }
   if (!s) s |= ens_alloc(e, (void**)&e->d_counter, sizeof(unsigned));
@@ -995,6 +1053,10 @@ int gbf_ensemble_create(int n, const gbf_model* models, const gbf_cells* host_ce
   }
   if (!s && e->precision != GBF_PREC_F64) {  // the members' row-constant tables, once
     k_ens_rows<<<e->n, 64>>>(e->d_mem);
+    s = gbf_cuda_check(cudaDeviceSynchronize(), "gbf_ensemble_create rows");
+  }
+  if (!s && e->pair) {  // likewise the pair step's
+    k_ens_pair_rows<<<e->n, 64>>>(e->d_mem);
     s = gbf_cuda_check(cudaDeviceSynchronize(), "gbf_ensemble_create rows");
   }
   if (s) {

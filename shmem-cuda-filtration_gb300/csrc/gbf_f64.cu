@@ -1,24 +1,32 @@
-// gbf_f64.cu — plain FP64 step of one domain, fused into two passes plus a
-// face pass (per-cell code in gbf_f64_cell.cuh).
+// gbf_f64.cu — FP64 step of one domain: two passes plus a face pass.
 //
-// GB300 executes FP64 at about 1/64 of its FP32 rate (measured 1.2 TFLOP/s
-// DFMA against 6.4 TB/s of HBM), so a plain FP64 step is bound by the FP64
-// pipe, not by memory: the design minimises FP64 instructions per cell and
-// spends bytes freely to do so.
-//   pass 1 (k_f64_props, every cell): one log and two exp per cell for the
-//     Brooks-Corey relative permeabilities (cpu.cpp:57-74), the densities,
-//     and L = Xi * ro per phase; ln(S_e) is kept for the Newton step.
-//   pass 2 (k_f64_flux_newton, interior cells): upwinded face fluxes with
-//     gravity (cpu.cpp:218-291) and the 2x2 Newton (cpu.cpp:293-320) fused;
-//     the first iteration reuses ln(S_e) from pass 1 and the iteration stops
-//     once the update is at round-off (model.newton_tol), at most
-//     model.newton_iterations times. Writes the next state (ping-pong) and,
-//     optionally, per-block phase-mass partial sums.
+// GB300 executes FP64 at about 1/58 of its FP32 rate (measured 1.2 TFLOP/s
+// DFMA against 6.7 TB/s of HBM): any step whose arithmetic is FP64 is bound
+// by that pipe (measured 8.73 ms a step at 256^3: 85% of it active, DRAM at
+// 4%). The step therefore forms its increments in FP32 pairs
+// (gbf_f64_pair.cuh) and touches the FP64 pipe for five additions a cell:
+//   pass 1 (k_pair_props, every cell): pressure against the row's hydrostatic
+//     value, mobility x density of both phases, capillary pressure, as pairs
+//     (32 bytes a cell written);
+//   pass 2 (k_pair_step, interior cells): upwinded face fluxes with gravity
+//     (cpu.cpp:218-291) and the 2x2 Newton (cpu.cpp:293-320) in increments,
+//     the next FP64 state (ping-pong), phase-mass partial sums on request.
+// Two passes, not one tile: a cell's properties cost half of its fluxes and
+// Newton, so they are not computed again for halos, and the 64 bytes a cell
+// that this moves beside the state are hidden behind the arithmetic. Both are
+// bound by instruction issue (pass 1 with the FP64 pipe 61% busy); 256^3,
+// heterogeneous, a quarter of the cells with DNAPL: pass 1 223 us, pass 2 440
+// us (2.3 and 2.6 TB/s of their 52 and 68 bytes a cell), where the FP64
+// passes took 2460 and 6270. Pass 2 takes 64 registers for four blocks an SM:
+// at three (80 registers) its latencies show, 808 us; at five and six it spills
+// (627, 764).
 //   face pass (k_f64_boundary): the reference's sweep-ordered boundary
 //     values (cpu.cpp:44-54, 323-403) into the next state.
-// Every cell's properties are computed once per step (no halo recomputation),
-// which is what an FP64-bound kernel wants.
+// A model with fewer Newton iterations than the reference's 7 runs the plain
+// FP64 passes (k_f64_props, k_f64_flux_newton; per-cell code in
+// gbf_f64_cell.cuh): its iterates stop before convergence.
 #include "gbf_f64_cell.cuh"
+#include "gbf_f64_pair.cuh"
 
 namespace {
 
@@ -44,6 +52,37 @@ __global__ void __launch_bounds__(kThreads) k_f64_flux_newton(const gbf_model m,
   }
   if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
   if (s.mass_partials) gbf_block_sum2<kThreads>(msum1, msum2, d.V, s.mass_partials + 2 * blockIdx.x);
+}
+
+template <bool DROPIN>
+__global__ void __launch_bounds__(kThreads) k_pair_props(const GbfPairConsts C, const gbf_cells cells,
+                                                         const GbfF64Step s, const GbfPairWork w) {
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < C.n; c += gridDim.x * blockDim.x)
+    gbf_pair_props_cell<DROPIN>(C, cells, s, w, c);
+}
+
+template <bool MASS>
+__global__ void __launch_bounds__(kThreads, 4) k_pair_step(const GbfPairConsts C, const gbf_cells cells,
+                                                        const GbfF64Step s, const GbfPairWork w, double V) {
+  GbfPairMass acc;
+  unsigned bad = 0;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < C.nint; t += gridDim.x * blockDim.x) {
+    const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
+    const unsigned i = 1u + t - r * C.dix.d, j = 1u + r - q * C.diy.d, k = 1u + q;
+    gbf_pair_step_cell<MASS>(C, cells, s, w, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc, bad);
+  }
+  if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
+  if (MASS) gbf_block_sum2<kThreads>(acc.m1 - pf_to_double(acc.r1), acc.m2, V, s.mass_partials + 2 * blockIdx.x);
+}
+
+__global__ void __launch_bounds__(kThreads) k_density(double ro0, double beta, double Patm, const double* P,
+                                                      double* out, size_t n) {
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
+    out[c] = ro0 * (1. + beta * (P[c] - Patm));
+}
+
+__global__ void k_pair_rows(const gbf_model m, GbfPairRow* rows) {
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m.ny; j += gridDim.x * blockDim.x) rows[j] = gbf_pair_row(m, j);
 }
 
 __global__ void __launch_bounds__(kThreads) k_f64_boundary(const gbf_model m, const GbfF64Step s) {
@@ -75,20 +114,114 @@ unsigned gbf_f64_flux_grid(const gbf_model& m) {
   return gbf_grid_for(nint, kThreads, 4);
 }
 
+GbfPairConsts gbf_pair_consts(const gbf_model& m) {
+  GbfPairConsts C = {};
+  const GbfDerived d = gbf_derive(m);
+  C.nx = m.nx; C.ny = m.ny; C.nz = m.nz;
+  C.noflow = m.bc_mode == GBF_BC_HYDROSTATIC_SIDES;
+  C.pl = (unsigned)m.nx * (unsigned)m.ny;
+  C.n = C.pl * (unsigned)m.nz;
+  C.nint = (unsigned)(m.nx - 2) * (unsigned)(m.ny - 2) * (unsigned)(m.nz - 2);
+  C.dnx = gbf_fast_div((unsigned)m.nx);
+  C.dny = gbf_fast_div((unsigned)m.ny);
+  C.dix = gbf_fast_div((unsigned)m.nx - 2);
+  C.diy = gbf_fast_div((unsigned)m.ny - 2);
+  if (d.src != 0.) {
+    C.rn = m.rate_cells;
+    C.ri0 = m.nx / 2 - m.rate_cells / 2;
+    C.rk0 = m.nz / 2 - m.rate_cells / 2;
+  }
+  C.max_iter = m.newton_iterations;
+  C.Patm = (float)fabs(m.P_atm);
+  // 2^e that brings the water mobility x density of media 0 to about 1
+  int e = 0;
+  const double L = m.K[0] * m.ro01 / m.mu1;
+  if (L > 0. && isfinite(L)) frexp(L, &e);
+  e = e < -60 ? -60 : e > 60 ? 60 : e;
+  const double sc = ldexp(1.0, -e), log2e = 1.4426950408889634074;
+  C.k1 = pf_const(m.ro01 * m.beta1);
+  C.k2 = pf_const(m.ro02 * m.beta2);
+  C.rk1 = pf_const(1.0 / (m.ro01 * m.beta1));
+  C.ro1 = pf_const(m.ro01);
+  C.ro2 = pf_const(m.ro02);
+  C.g1 = pf_const(m.g * m.h2 * m.ro01 * m.beta1);
+  C.g2 = pf_const(m.g * m.h2 * m.ro02 * m.beta2);
+  C.ghd = pf_const(m.g * m.h2 * (m.ro02 - m.ro01));
+  C.wx = pf_const(m.dt / (m.h1 * m.h1) / sc);
+  C.wy = pf_const(m.dt * m.kv / (m.h2 * m.h2) / sc);
+  C.wz = pf_const(m.dt / (m.h3 * m.h3) / sc);
+  C.c1 = pf_const(sc / m.mu1);
+  C.c2 = pf_const(sc / m.mu2);
+  C.dtsrc_d = m.dt * d.src;
+  C.rro2_d = 1.0 / m.ro02;
+  for (int md = 0; md < 2; md++) {
+    C.K[md] = pf_const(m.K[md]);
+    C.phi_d[md] = m.m[md];
+    C.phip[md] = pf_const(m.m[md]);
+    C.rphi[md] = pf_const(1.0 / m.m[md]);
+    C.inv[md] = pf_const(d.inv_1mswr[md]);
+    C.inv_d[md] = d.inv_1mswr[md];
+    C.E1[md] = d.e1[md] * log2e;
+    C.E2[md] = d.e2[md] * log2e;
+    C.E3[md] = d.m_inv_lam[md] * log2e;
+    C.E1f[md] = (float)C.E1[md];
+    C.E2f[md] = (float)C.E2[md];
+    C.E3p[md] = pf_const(C.E3[md]);
+    C.pd[md] = pf_const(m.P_d[md]);
+    C.ilam[md] = pf_const(d.inv_lam_1mswr[md]);
+    for (int n = 1; n <= 4; n++) C.taylor[md][n - 1] = (float)((1.0 / m.lambda[md] + n) / (n + 1));
+  }
+  C.ro1_d = m.ro01; C.ro2_d = m.ro02; C.beta1_d = m.beta1; C.beta2_d = m.beta2; C.Patm_d = m.P_atm;
+  C.k1_d = m.ro01 * m.beta1; C.k2_d = m.ro02 * m.beta2;
+  return C;
+}
+
+int gbf_density_launch(const gbf_model& m, int phase, const double* P, double* out, cudaStream_t st) {
+  const size_t n = gbf_geo(m).n;
+  k_density<<<gbf_grid_for(n, kThreads), kThreads, 0, st>>>(phase == 1 ? m.ro01 : m.ro02, phase == 1 ? m.beta1 : m.beta2,
+                                                           m.P_atm, P, out, n);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? GBF_OK : gbf_cuda_check(e, "gbf_density_launch");
+}
+
+int gbf_pair_fill_rows(const gbf_model& m, GbfPairRow* rows, cudaStream_t st) {
+  k_pair_rows<<<gbf_grid_for((size_t)m.ny, kThreads), kThreads, 0, st>>>(m, rows);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? GBF_OK : gbf_cuda_check(e, "gbf_pair_fill_rows");
+}
+
 int gbf_f64_launch_step(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells, const GbfF64Step& s,
-                        int props_flags, double* mass_out, cudaStream_t st, GbfTimer* tm) {
+                        const GbfPairConsts* pc, const GbfPairWork* pair, int props_flags, double* mass_out,
+                        cudaStream_t st, GbfTimer* tm) {
   const GbfGeo g = gbf_geo(m);
-  cudaEvent_t e = gbf_timer_begin(tm, st);
-  k_f64_props<<<gbf_grid_for(g.n, kThreads, 4), kThreads, 0, st>>>(m, d, cells, s, props_flags);
-  gbf_timer_end(tm, GBF_K_PROPS, e, st);
   const unsigned fg = gbf_f64_flux_grid(m);
+  const bool mass = s.mass_partials && mass_out;
+  cudaEvent_t e = gbf_timer_begin(tm, st);
+  if (pair) {
+    const unsigned pg = gbf_grid_for(g.n, kThreads, 8);
+    if (pair->P_from) k_pair_props<true><<<pg, kThreads, 0, st>>>(*pc, cells, s, *pair);
+    else k_pair_props<false><<<pg, kThreads, 0, st>>>(*pc, cells, s, *pair);
+    if (props_flags) {  // the outputs P2, Xi, u of the state the step starts from
+      GbfF64Step o = s;
+      o.L1 = nullptr;
+      k_f64_props<<<gbf_grid_for(g.n, kThreads, 4), kThreads, 0, st>>>(m, d, cells, o, props_flags);
+    }
+  } else {
+    k_f64_props<<<gbf_grid_for(g.n, kThreads, 4), kThreads, 0, st>>>(m, d, cells, s, props_flags);
+  }
+  gbf_timer_end(tm, GBF_K_PROPS, e, st);
   e = gbf_timer_begin(tm, st);
-  k_f64_flux_newton<<<fg, kThreads, 0, st>>>(m, d, cells, s);
+  if (pair) {
+    if (mass) k_pair_step<true><<<fg, kThreads, 0, st>>>(*pc, cells, s, *pair, d.V);
+    else k_pair_step<false><<<fg, kThreads, 0, st>>>(*pc, cells, s, *pair, d.V);
+  } else {
+    k_f64_flux_newton<<<fg, kThreads, 0, st>>>(m, d, cells, s);
+  }
   gbf_timer_end(tm, GBF_K_FLUX_NEWTON, e, st);
   e = gbf_timer_begin(tm, st);
   k_f64_boundary<<<gbf_grid_for(gbf_boundary_count(g), kThreads, 4), kThreads, 0, st>>>(m, s);
   gbf_timer_end(tm, GBF_K_BOUNDARY, e, st);
-  if (s.mass_partials && mass_out) {
+  if (mass) {
     e = gbf_timer_begin(tm, st);
     gbf_k_mass_tail<<<1, 256, 0, st>>>(s.mass_partials, (int)fg, mass_out);
     gbf_timer_end(tm, GBF_K_MASS_TAIL, e, st);

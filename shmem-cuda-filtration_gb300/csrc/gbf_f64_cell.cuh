@@ -16,7 +16,7 @@ __device__ __forceinline__ void gbf_f64_props_cell(const gbf_model& m, const Gbf
   const int md = gbf_media_at(cells, c);
   const double K = cells.K ? (double)cells.K[c] : m.K[md];
   const double S2 = s.S[c], P1 = s.P[c];
-  const double S_e = (1. - S2 - m.S_wr[md]) * d.inv_1mswr[md];
+  const double S_e = (1. - S2 - m.S_wr[md]) / (1. - m.S_wr[md]);  // a division: exactly 1 at S = 0, where kr2 is 0
   const double l = log(S_e);
   const double k1 = exp(d.e1[md] * l);
   const double k2 = (1. - S_e) * (1. - S_e) * (1. - exp(d.e2[md] * l));
@@ -24,11 +24,13 @@ __device__ __forceinline__ void gbf_f64_props_cell(const gbf_model& m, const Gbf
   const double Xi2 = K * k2 * d.neg_inv_mu2;
   const double ro1 = m.ro01 * (1. + m.beta1 * (P1 - m.P_atm));
   const double ro2 = m.ro02 * (1. + m.beta2 * (P1 - m.P_atm));  // P2 = P1 (P_k = 0, cpu.cpp:63)
-  s.L1[c] = Xi1 * ro1;
-  s.L2[c] = Xi2 * ro2;
-  s.ro1[c] = ro1;
-  s.ro2[c] = ro2;
-  s.lnSe[c] = l;
+  if (s.L1) {  // NULL: only the outputs below (beside the pair step)
+    s.L1[c] = Xi1 * ro1;
+    s.L2[c] = Xi2 * ro2;
+    s.ro1[c] = ro1;
+    s.ro2[c] = ro2;
+    s.lnSe[c] = l;
+  }
   if (flags & GBF_PF_WRITE_XI_P2) {
     s.Xi1[c] = Xi1;
     s.Xi2[c] = Xi2;
@@ -167,8 +169,10 @@ __device__ __forceinline__ void gbf_f64_boundary_cell(const gbf_model& m, const 
   int i, j, k;
   gbf_boundary_cell(g, t, i, j, k);
   const size_t c = gbf_idx(g, i, j, k);
-  const double* ro1 = s.ro1;
-  auto ro1_top = [ro1, &g](int ii) { return ro1[(size_t)ii + (size_t)g.nx]; };
+  const double* P = s.P;  // the start-of-step density of (i, 1, 0)
+  auto ro1_top = [P, &m, &g](int ii) {
+    return __dmul_rn(m.ro01, __fma_rn(m.beta1, __dsub_rn(P[(size_t)ii + (size_t)g.nx], m.P_atm), 1.));
+  };
   s.Sn[c] = gbf_sweep_S<double>(m, g, s.Sn, s.S, i, j, k);
   s.Pn[c] = gbf_sweep_P<double>(m, g, s.Pn, s.P, i, j, k, ro1_top);
 }
