@@ -47,6 +47,7 @@ struct EnsMember {
   GbfPatchConsts pc;
   float2* patch;
   GbfRowConst* rows;  // split forms: the row constants of the state conversions (ny entries)
+  GbfFastDiv dnx, dny;
 };
 
 struct EnsChunk {
@@ -454,27 +455,43 @@ __global__ void __launch_bounds__(64) k_ens_split_patch(const EnsMember* __restr
 
 // Packed all-members FP64 state (staging) -> every member's current buffer
 // (and the next buffer's faces, which the next step rewrites), one chunk
-// (member, cell range) per block.
+// (member, cell range) per block, the loads of four cells a thread in flight
+// together. MR: the split form's masses, or kLoadF64.
+constexpr int kLoadF64 = -1, kLoadPer = 4;
+template <int MR>
 __global__ void __launch_bounds__(kThreads) k_ens_load(const EnsMember* __restrict__ mem,
                                                        const EnsChunk* __restrict__ chunks, int cur,
                                                        const double* __restrict__ P_all,
-                                                       const double* __restrict__ S_all, int precision) {
+                                                       const double* __restrict__ S_all) {
+  __shared__ EnsMember me;
   const EnsChunk ch = chunks[blockIdx.x];
-  const EnsMember& me = mem[ch.member];
-  const gbf_model& m = me.m;
-  for (unsigned c = ch.begin + threadIdx.x; c < ch.end; c += blockDim.x) {
-    const double p = P_all[me.off + c], s = S_all[me.off + c];
-    if (precision == GBF_PREC_F64) {
-      me.P[cur][c] = p;
-      me.S[cur][c] = s;
-    } else {
-      const int j = (int)((c / (unsigned)m.nx) % (unsigned)m.ny);
-      float dPf, Sf;
-      gbf_split_init_cell(m, p, s, me.rows[j], dPf, Sf, me.M1, me.M2, c, gbf_mass_rep(precision));
-      me.dPf[cur][c] = dPf;
-      me.Sf[cur][c] = Sf;
-      me.dPf[cur ^ 1][c] = dPf;
-      me.Sf[cur ^ 1][c] = Sf;
+  ens_copy_member(me, mem + ch.member);
+  for (unsigned b = ch.begin + threadIdx.x; b < ch.end; b += kLoadPer * kThreads) {
+    double p[kLoadPer], s[kLoadPer];
+#pragma unroll
+    for (int u = 0; u < kLoadPer; u++) {
+      const unsigned c = b + u * kThreads;
+      if (c < ch.end) {
+        p[u] = P_all[me.off + c];
+        s[u] = S_all[me.off + c];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kLoadPer; u++) {
+      const unsigned c = b + u * kThreads;
+      if (c >= ch.end) continue;
+      if constexpr (MR == kLoadF64) {
+        me.P[cur][c] = p[u];
+        me.S[cur][c] = s[u];
+      } else {
+        const unsigned r = gbf_div(c, me.dnx), j = r - gbf_div(r, me.dny) * me.dny.d;
+        float dPf, Sf;
+        gbf_split_init_cell<MR, true>(me.m, p[u], s[u], me.rows[j], dPf, Sf, me.M1, me.M2, c);
+        me.dPf[cur][c] = dPf;
+        me.Sf[cur][c] = Sf;
+        me.dPf[cur ^ 1][c] = dPf;
+        me.Sf[cur ^ 1][c] = Sf;
+      }
     }
   }
 }
@@ -487,21 +504,26 @@ __global__ void k_ens_rows(const EnsMember* __restrict__ mem) {
 }
 
 // Every member's current state -> packed all-members FP64 arrays.
+template <bool F64>
 __global__ void __launch_bounds__(kThreads) k_ens_store(const EnsMember* __restrict__ mem,
                                                         const EnsChunk* __restrict__ chunks, int cur,
-                                                        double* __restrict__ P_all, double* __restrict__ S_all,
-                                                        int precision) {
+                                                        double* __restrict__ P_all, double* __restrict__ S_all) {
   const EnsChunk ch = chunks[blockIdx.x];
   const EnsMember& me = mem[ch.member];
-  const gbf_model& m = me.m;
-  for (unsigned c = ch.begin + threadIdx.x; c < ch.end; c += blockDim.x) {
-    if (precision == GBF_PREC_F64) {
-      P_all[me.off + c] = me.P[cur][c];
-      S_all[me.off + c] = me.S[cur][c];
+  const double *P = me.P[cur], *S = me.S[cur];
+  const float *dPf = me.dPf[cur], *Sf = me.Sf[cur];
+  const GbfFastDiv dnx = me.dnx, dny = me.dny;
+  const GbfRowConst* rows = me.rows;
+  double *Po = P_all + me.off, *So = S_all + me.off;
+#pragma unroll 4
+  for (unsigned c = ch.begin + threadIdx.x; c < ch.end; c += kThreads) {
+    if constexpr (F64) {
+      Po[c] = __ldg(P + c);
+      So[c] = __ldg(S + c);
     } else {
-      const int j = (int)((c / (unsigned)m.nx) % (unsigned)m.ny);
-      P_all[me.off + c] = me.rows[j].phs + (double)me.dPf[cur][c];
-      S_all[me.off + c] = (double)me.Sf[cur][c];
+      const unsigned r = gbf_div(c, dnx), j = r - gbf_div(r, dny) * dny.d;
+      Po[c] = gbf_split_P(__ldg(dPf + c), rows[j]);
+      So[c] = gbf_f2d_all(__ldg(Sf + c));
     }
   }
 }
@@ -590,6 +612,17 @@ bool tma_possible(const gbf_ensemble* e, int TX) {
     if (!(me.cells.K && me.cells.phi && !me.cells.media && gbf_tma_eligible(e->models[r].nx, TX))) return false;
   }
   return true;
+}
+
+// Chunks [a, a + n) of the all-cells list: packed FP64 arrays <-> the members' state.
+void launch_load(gbf_ensemble* e, int a, int n, int cur, const double* P, const double* S, cudaStream_t st) {
+  auto kern = e->precision == GBF_PREC_F64 ? k_ens_load<kLoadF64> : gbf_mass_rep(e->precision) == kMassDefect ? k_ens_load<kMassDefect>
+              : gbf_mass_rep(e->precision) == kMassDF ? k_ens_load<kMassDF> : k_ens_load<kMassDefectDF>;
+  kern<<<(unsigned)n, kThreads, 0, st>>>(e->d_mem, e->d_all + a, cur, P, S);
+}
+void launch_store(gbf_ensemble* e, int a, int n, int cur, double* P, double* S, cudaStream_t st) {
+  auto kern = e->precision == GBF_PREC_F64 ? k_ens_store<true> : k_ens_store<false>;
+  kern<<<(unsigned)n, kThreads, 0, st>>>(e->d_mem, e->d_all + a, cur, P, S);
 }
 
 // Packed work lists of the current tuning.
@@ -1000,6 +1033,8 @@ int gbf_ensemble_create(int n, const gbf_model* models, const gbf_cells* host_ce
     me.m = m;
     me.d = gbf_derive(m);
     me.C = gbf_split_consts(m);
+    me.dnx = gbf_fast_div((unsigned)m.nx);
+    me.dny = gbf_fast_div((unsigned)m.ny);
     if (host_cells) {
       const gbf_cells& hc = host_cells[r];
       if (hc.media && !(s |= ens_alloc(e, (void**)&me.cells.media, nc * sizeof(int))))
@@ -1132,12 +1167,9 @@ int gbf_ensemble_upload(gbf_ensemble* e, int r, const double* P1, const double* 
     GBF_CUDA(cudaMallocAsync((void**)&tmp, 2 * b, e->stream));
     GBF_CUDA(cudaMemcpyAsync(tmp, P1, b, cudaMemcpyDefault, e->stream));
     GBF_CUDA(cudaMemcpyAsync(tmp + nc, S2, b, cudaMemcpyDefault, e->stream));
-    if (int s = gbf_split_init_state(m, me.rows, tmp, tmp + nc, me.dPf[c], me.Sf[c], me.M1, me.M2,
-                                     gbf_mass_rep(e->precision), e->stream))
+    if (int s = gbf_split_init_state(m, me.rows, tmp, tmp + nc, me.dPf, me.Sf, me.M1, me.M2,
+                                     gbf_mass_rep(e->precision), 0, nc, e->stream))
       return s;
-    // the next-state buffer's faces are rewritten every step; start them equal
-    GBF_CUDA(cudaMemcpyAsync(me.dPf[c ^ 1], me.dPf[c], nc * sizeof(float), cudaMemcpyDeviceToDevice, e->stream));
-    GBF_CUDA(cudaMemcpyAsync(me.Sf[c ^ 1], me.Sf[c], nc * sizeof(float), cudaMemcpyDeviceToDevice, e->stream));
     GBF_CUDA(cudaFreeAsync(tmp, e->stream));
   }
   e->steps = 0;
@@ -1169,7 +1201,7 @@ int gbf_ensemble_upload_all(gbf_ensemble* e, const double* P_all, const double* 
     P = e->d_stage;
     S = e->d_stage + e->cells;
   }
-  k_ens_load<<<(unsigned)e->all.size(), kThreads, 0, e->stream>>>(e->d_mem, e->d_all, e->cur, P, S, e->precision);
+  launch_load(e, 0, (int)e->all.size(), e->cur, P, S, e->stream);
   GBF_CUDA(cudaGetLastError());
   e->steps = 0;
   GBF_CUDA(cudaMemsetAsync(e->d_status, 0, sizeof(unsigned), e->stream));
@@ -1187,13 +1219,12 @@ int gbf_ensemble_download_all(gbf_ensemble* e, double* P_all, double* S_all) {
   double* P = (double*)gbf_mapped_host(P_all);
   double* S = (double*)gbf_mapped_host(S_all);
   if (P && S) {
-    k_ens_store<<<(unsigned)e->all.size(), kThreads, 0, e->stream>>>(e->d_mem, e->d_all, e->cur, P, S, e->precision);
+    launch_store(e, 0, (int)e->all.size(), e->cur, P, S, e->stream);
     GBF_CUDA(cudaGetLastError());
   } else {
     if (int s = ensure_stage(e)) return s;
     const size_t b = sizeof(double) * (size_t)e->cells;
-    k_ens_store<<<(unsigned)e->all.size(), kThreads, 0, e->stream>>>(e->d_mem, e->d_all, e->cur, e->d_stage,
-                                                                     e->d_stage + e->cells, e->precision);
+    launch_store(e, 0, (int)e->all.size(), e->cur, e->d_stage, e->d_stage + e->cells, e->stream);
     GBF_CUDA(cudaGetLastError());
     GBF_CUDA(cudaMemcpyAsync(P_all, e->d_stage, b, cudaMemcpyDefault, e->stream));
     GBF_CUDA(cudaMemcpyAsync(S_all, e->d_stage + e->cells, b, cudaMemcpyDefault, e->stream));
@@ -1234,11 +1265,10 @@ int ens_advance_host(gbf_ensemble* e, const double* P_in, const double* S_in, in
   for (int g = 0; g < G; g++) {
     const auto &a = e->starts[first[g]], &b = e->starts[first[g + 1]];
     GBF_CUDA(cudaStreamWaitEvent(cs, e->ev[2 + 2 * g], 0));
-    k_ens_load<<<(unsigned)(b.all - a.all), kThreads, 0, cs>>>(e->d_mem, e->d_all + a.all, c0, stP, stS, e->precision);
+    launch_load(e, a.all, b.all - a.all, c0, stP, stS, cs);
     for (int q = 0; q < nsteps; q++)
       if (int s = enqueue_group_step(e, first[g], first[g + 1], c0 ^ (q & 1), e->d_gcounter + g, cs)) return s;
-    k_ens_store<<<(unsigned)(b.all - a.all), kThreads, 0, cs>>>(e->d_mem, e->d_all + a.all, c0 ^ (nsteps & 1), stP,
-                                                                 stS, e->precision);
+    launch_store(e, a.all, b.all - a.all, c0 ^ (nsteps & 1), stP, stS, cs);
     GBF_CUDA(cudaGetLastError());
     GBF_CUDA(cudaEventRecord(e->ev[3 + 2 * g], cs));
     GBF_CUDA(cudaStreamWaitEvent(e->s_out, e->ev[3 + 2 * g], 0));
@@ -1311,7 +1341,7 @@ int gbf_ensemble_download(gbf_ensemble* e, int r, int field, double* host) {
     double* tmp = nullptr;
     GBF_CUDA(cudaMallocAsync((void**)&tmp, b, e->stream));
     if (int s = gbf_split_state_to_f64(m, me.rows, me.dPf[e->cur], me.Sf[e->cur], field == GBF_FIELD_P1 ? tmp : nullptr,
-                                       field == GBF_FIELD_S2 ? tmp : nullptr, e->stream))
+                                       field == GBF_FIELD_S2 ? tmp : nullptr, 0, nc, e->stream))
       return s;
     GBF_CUDA(cudaMemcpyAsync(host, tmp, b, cudaMemcpyDefault, e->stream));
     GBF_CUDA(cudaFreeAsync(tmp, e->stream));

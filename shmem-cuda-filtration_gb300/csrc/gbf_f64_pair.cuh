@@ -22,20 +22,6 @@
 #include "gbf_domain.h"
 #include "gbf_pair.cuh"
 
-// n / d for n < 2^31 by multiplication.
-struct GbfFastDiv {
-  unsigned d, m;
-  int s;
-};
-inline GbfFastDiv gbf_fast_div(unsigned d) {
-  int l = 0;
-  while ((1ull << l) < d) l++;
-  return {d, (unsigned)(((1ull << (31 + l)) / d) + 1ull), 31 + l};
-}
-__device__ __forceinline__ unsigned gbf_div(unsigned n, const GbfFastDiv& f) {
-  return (unsigned)(((unsigned long long)n * f.m) >> f.s);
-}
-
 // A row's constants: P_hs(j), P_hs(j) - P_atm as a pair, and what rounding
 // leaves of rho01 g h2 minus the rows' differences of P_hs (above, below).
 struct GbfPairRow {

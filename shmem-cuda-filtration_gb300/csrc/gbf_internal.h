@@ -10,6 +10,20 @@
 
 #define GBF_HD __host__ __device__ __forceinline__
 
+// n / d for n < 2^31 by multiplication.
+struct GbfFastDiv {
+  unsigned d, m;
+  int s;
+};
+inline GbfFastDiv gbf_fast_div(unsigned d) {
+  int l = 0;
+  while ((1ull << l) < d) l++;
+  return {d, (unsigned)(((1ull << (31 + l)) / d) + 1ull), 31 + l};
+}
+__device__ __forceinline__ unsigned gbf_div(unsigned n, const GbfFastDiv& f) {
+  return (unsigned)(((unsigned long long)n * f.m) >> f.s);
+}
+
 // ------------------------------------------------------------------ status
 // Sticky status shared by all entry points (single host thread, like the
 // reference). Returns `s` so callers can `return gbf_fail(...)`.

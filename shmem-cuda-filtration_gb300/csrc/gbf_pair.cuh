@@ -117,6 +117,62 @@ __device__ __forceinline__ GbfPf pf_from_double(double d) {
 }
 __device__ __forceinline__ double pf_to_double(GbfPf a) { return __dadd_rn(gbf_f2d(a.h), gbf_f2d(a.l)); }
 
+// The conversions with every input's exact result. (float)d, and (double)(float)d in fd.
+static __device__ __noinline__ float gbf_d2f_general(double d, double* fd) {
+  const float f = (float)d;
+  *fd = (double)f;
+  return f;
+}
+__device__ __forceinline__ float gbf_d2f(double d, double& fd) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const unsigned a = hi & 0x7fffffffu;
+  if (a - (897u << 20) < (253u << 20)) {  // a normal result, whichever way it rounds
+    // round the 53-bit number to 24 bits, ties to even, carrying into the exponent
+    const unsigned t = lo + 0x0fffffffu + ((lo >> 29) & 1u);
+    const unsigned h = hi + (t < lo ? 1u : 0u);
+    fd = __hiloint2double((int)h, (int)(t & 0xe0000000u));
+    return __uint_as_float((hi & 0x80000000u) | (((h & 0x7fffffffu) - (896u << 20)) << 3) | (t >> 29));
+  }
+  if ((a | lo) == 0u) {
+    fd = d;
+    return __uint_as_float(hi);
+  }
+  return gbf_d2f_general(d, &fd);
+}
+// d as an FP32 pair, h = (float)d, l = (float)(d - h) (gbf_df_from_double).
+static __device__ __noinline__ float2 gbf_d2f2_general(double d) {
+  const float h = (float)d;
+  return make_float2(h, (float)(d - (double)h));
+}
+__device__ __forceinline__ float2 gbf_d2f2(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const unsigned a = hi & 0x7fffffffu;
+  if (a - (960u << 20) < (190u << 20)) {  // both parts normal
+    double fd;
+    const float h = gbf_d2f(d, fd);
+    // d - h in units of d's last place, a signed 29-bit integer: its leading
+    // 23 and last 6 bits as FP32 integers, their sum rounded once
+    const int n = (int)lo - __double2loint(fd);
+    const float n1 = __fsub_rn(__uint_as_float(0x4b400000u + (unsigned)(n >> 6)), 12582912.f);
+    const float n2 = __fsub_rn(__uint_as_float(0x4b000000u + ((unsigned)n & 63u)), 8388608.f);
+    const unsigned sc = ((a >> 20) - 948u) << 23;
+    return make_float2(h, __fmul_rn(__fmaf_rn(n1, 64.f, n2), __uint_as_float((hi & 0x80000000u) | sc)));
+  }
+  if ((a | lo) == 0u) return make_float2(__uint_as_float(hi), 0.f);
+  return gbf_d2f2_general(d);
+}
+// (double)f
+__device__ __forceinline__ double gbf_f2d_all(float f) {
+  const unsigned b = __float_as_uint(f), u = b & 0x7fffffffu;
+  unsigned m = u, e = u >= 0x7f800000u ? 0x70000000u : 0x38000000u;
+  if (u < 0x00800000u && u != 0u) {  // subnormal: normalised
+    const int n = __clz((int)u) - 8;
+    m = (u << n) & 0x007fffffu;
+    e = (unsigned)(897 - n) << 20;
+  }
+  return __hiloint2double((int)((b & 0x80000000u) | (u == 0u ? 0u : (m >> 3) + e)), (int)(m << 29));
+}
+
 // ------------------------------------------------------ ln and 2^x tables
 // Table-driven in the manner of Tang (ACM TOMS 15, 1989; 16, 1990), the
 // reduced argument and the last sums in FP64, the polynomials (the part below

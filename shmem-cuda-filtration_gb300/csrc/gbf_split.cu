@@ -223,25 +223,62 @@ __global__ void k_split_mass_tail(const double* partials, int nblocks, double* o
   if (threadIdx.x == 0) { out[0] = red[0][0] + k1v; out[1] = red[1][0]; }
 }
 
-// rows: the grid's row table (GbfRowConst), or NULL to form each row's
-// values per cell (the same values either way).
-__global__ void k_split_init(const gbf_model m, const GbfRowConst* rows, const double* P, const double* S,
-                             float* dPf, float* Sf, double* M1, double* M2, int mr, size_t c0, size_t c1) {
-  const GbfGeo g = gbf_geo(m);
-  for (size_t c = c0 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < c1; c += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)((c / g.nx) % g.ny);
-    if (rows) gbf_split_init_cell(m, P[c], S[c], rows[j], dPf[c], Sf[c], M1, M2, c, mr);
-    else gbf_split_init_cell(m, P[c], S[c], j, dPf[c], Sf[c], M1, M2, c, mr);
+// The state conversions of cells [c0, c1): each block kConvCells consecutive
+// cells, the loads of a thread's cells in flight together.
+constexpr int kConvPer = 4, kConvCells = kConvPer * kThreads;
+template <int MR>
+__global__ void __launch_bounds__(kThreads) k_split_init(const gbf_model m, const GbfFastDiv dnx, const GbfFastDiv dny,
+                                                         const GbfRowConst* rows, const double* P, const double* S,
+                                                         float* dP0, float* dP1, float* S0, float* S1, double* M1,
+                                                         double* M2, unsigned c0, unsigned c1) {
+  const unsigned b = c0 + blockIdx.x * kConvCells + threadIdx.x;
+  double p[kConvPer], s[kConvPer];
+#pragma unroll
+  for (int u = 0; u < kConvPer; u++) {
+    const unsigned c = b + u * kThreads;
+    if (c < c1) {
+      p[u] = P[c];
+      s[u] = S[c];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kConvPer; u++) {
+    const unsigned c = b + u * kThreads;
+    if (c < c1) {
+      const unsigned r = gbf_div(c, dnx), j = r - gbf_div(r, dny) * dny.d;
+      float dp, sf;
+      gbf_split_init_cell<MR, false>(m, p[u], s[u], rows[j], dp, sf, M1, M2, c);
+      dP0[c] = dp;
+      dP1[c] = dp;  // the next-state buffer's faces are rewritten every step; they start equal
+      S0[c] = sf;
+      S1[c] = sf;
+    }
   }
 }
 
-__global__ void k_split_to_f64(const gbf_model m, const GbfRowConst* rows, const float* dPf, const float* Sf,
-                               double* P, double* S, size_t c0, size_t c1) {
-  const GbfGeo g = gbf_geo(m);
-  for (size_t c = c0 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < c1; c += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)((c / g.nx) % g.ny);
-    if (P) P[c] = (rows ? rows[j].phs : gbf_p_hydrostatic(m, j)) + (double)dPf[c];
-    if (S) S[c] = (double)Sf[c];
+__global__ void __launch_bounds__(kThreads) k_split_to_f64(const GbfFastDiv dnx, const GbfFastDiv dny,
+                                                           const GbfRowConst* rows, const float* dPf, const float* Sf,
+                                                           double* P, double* S, unsigned c0, unsigned c1) {
+  const unsigned b = c0 + blockIdx.x * kConvCells + threadIdx.x;
+  float p[kConvPer], s[kConvPer];
+#pragma unroll
+  for (int u = 0; u < kConvPer; u++) {
+    const unsigned c = b + u * kThreads;
+    if (c < c1) {
+      if (P) p[u] = dPf[c];
+      if (S) s[u] = Sf[c];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kConvPer; u++) {
+    const unsigned c = b + u * kThreads;
+    if (c < c1) {
+      if (P) {
+        const unsigned r = gbf_div(c, dnx), j = r - gbf_div(r, dny) * dny.d;
+        P[c] = gbf_split_P(p[u], rows[j]);
+      }
+      if (S) S[c] = gbf_f2d_all(s[u]);
+    }
   }
 }
 
@@ -472,9 +509,13 @@ int gbf_split_fill_rows(const gbf_model& m, GbfRowConst* rows, cudaStream_t st) 
 }
 
 int gbf_split_init_state(const gbf_model& m, const GbfRowConst* rows, const double* P_dev, const double* S_dev,
-                         float* dPf, float* Sf, double* M1, double* M2, int mr, cudaStream_t st) {
-  const size_t n = gbf_geo(m).n;
-  k_split_init<<<gbf_grid_for(n, kThreads, 4), kThreads, 0, st>>>(m, rows, P_dev, S_dev, dPf, Sf, M1, M2, mr, 0, n);
+                         float* const dPf[2], float* const Sf[2], double* M1, double* M2, int mr, size_t c0, size_t c1,
+                         cudaStream_t st) {
+  const GbfFastDiv dnx = gbf_fast_div((unsigned)m.nx), dny = gbf_fast_div((unsigned)m.ny);
+  const unsigned blocks = (unsigned)((c1 - c0 + kConvCells - 1) / kConvCells);
+  auto kern = mr == kMassDefect ? k_split_init<kMassDefect> : mr == kMassDF ? k_split_init<kMassDF> : k_split_init<kMassDefectDF>;
+  kern<<<blocks, kThreads, 0, st>>>(m, dnx, dny, rows, P_dev, S_dev, dPf[0], dPf[1], Sf[0], Sf[1], M1, M2,
+                                    (unsigned)c0, (unsigned)c1);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GBF_OK : gbf_cuda_check(e, "gbf_split_init_state");
 }
@@ -496,12 +537,9 @@ int gbf_split_upload(gbf_domain* d, const double* P1, const double* S2, cudaMemc
     S = tmp + n;
   }
   d->cur = 0;
-  k_split_init<<<gbf_grid_for(n, kThreads, 4), kThreads, 0, d->stream>>>(
-      d->m, d->split_rows, P, S, d->Pf[0], d->Sf[0], d->M1, d->M2, gbf_mass_rep(d->precision), 0, n);
-  GBF_CUDA(cudaGetLastError());
-  // the next-state buffer's faces are rewritten every step; start them equal
-  GBF_CUDA(cudaMemcpyAsync(d->Pf[1], d->Pf[0], n * sizeof(float), cudaMemcpyDeviceToDevice, d->stream));
-  GBF_CUDA(cudaMemcpyAsync(d->Sf[1], d->Sf[0], n * sizeof(float), cudaMemcpyDeviceToDevice, d->stream));
+  if (int e = gbf_split_init_state(d->m, d->split_rows, P, S, d->Pf, d->Sf, d->M1, d->M2, gbf_mass_rep(d->precision), 0,
+                                   n, d->stream))
+    return e;
   if (tmp) GBF_CUDA(cudaFreeAsync(tmp, d->stream));
   return GBF_OK;
 }
@@ -545,10 +583,10 @@ int gbf_split_download(gbf_domain* d, int field, double* host) {
   double* tmp = (double*)gbf_mapped_host(host);  // page-locked: written in place
   const bool staged = tmp == nullptr;
   if (staged) GBF_CUDA(cudaMallocAsync((void**)&tmp, b, d->stream));
-  k_split_to_f64<<<gbf_grid_for(n, kThreads, 4), kThreads, 0, d->stream>>>(
-      d->m, d->split_rows, d->Pf[d->cur], d->Sf[d->cur], field == GBF_FIELD_P1 ? tmp : nullptr,
-      field == GBF_FIELD_S2 ? tmp : nullptr, 0, n);
-  GBF_CUDA(cudaGetLastError());
+  if (int e = gbf_split_state_to_f64(d->m, d->split_rows, d->Pf[d->cur], d->Sf[d->cur],
+                                     field == GBF_FIELD_P1 ? tmp : nullptr, field == GBF_FIELD_S2 ? tmp : nullptr, 0, n,
+                                     d->stream))
+    return e;
   if (staged) {
     GBF_CUDA(cudaMemcpyAsync(host, tmp, b, cudaMemcpyDeviceToHost, d->stream));
     GBF_CUDA(cudaFreeAsync(tmp, d->stream));
@@ -558,9 +596,10 @@ int gbf_split_download(gbf_domain* d, int field, double* host) {
 }
 
 int gbf_split_state_to_f64(const gbf_model& m, const GbfRowConst* rows, const float* dPf, const float* Sf, double* P,
-                           double* S, cudaStream_t st) {
-  k_split_to_f64<<<gbf_grid_for(gbf_geo(m).n, kThreads, 4), kThreads, 0, st>>>(m, rows, dPf, Sf, P, S, 0,
-                                                                                gbf_geo(m).n);
+                           double* S, size_t c0, size_t c1, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((c1 - c0 + kConvCells - 1) / kConvCells);
+  k_split_to_f64<<<blocks, kThreads, 0, st>>>(gbf_fast_div((unsigned)m.nx), gbf_fast_div((unsigned)m.ny), rows, dPf, Sf,
+                                              P, S, (unsigned)c0, (unsigned)c1);
   GBF_CUDA(cudaGetLastError());
   return GBF_OK;
 }
@@ -639,10 +678,7 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
     if (q < ns) {  // slab q in: FP64 -> split state, both buffers
       const size_t c0 = (size_t)pa(q) * pl, c1 = (size_t)pb(q) * pl;
       GBF_CUDA(cudaStreamWaitEvent(cs, d->pipe_ev[2 + q], 0));
-      k_split_init<<<gbf_grid_for(c1 - c0, kThreads, 4), kThreads, 0, cs>>>(m, d->split_rows, stP, stS, d->Pf[0],
-                                                                          d->Sf[0], d->M1, d->M2, mr, c0, c1);
-      GBF_CUDA(cudaMemcpyAsync(d->Pf[1] + c0, d->Pf[0] + c0, (c1 - c0) * sizeof(float), cudaMemcpyDeviceToDevice, cs));
-      GBF_CUDA(cudaMemcpyAsync(d->Sf[1] + c0, d->Sf[0] + c0, (c1 - c0) * sizeof(float), cudaMemcpyDeviceToDevice, cs));
+      if (int e = gbf_split_init_state(m, d->split_rows, stP, stS, d->Pf, d->Sf, d->M1, d->M2, mr, c0, c1, cs)) return e;
     }
     if (q > 0) {  // slab q - 1: its chunk layer of the step, its boundary cells, out
       const int r = q - 1;
@@ -651,8 +687,7 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
       if (Gr.mass_partials) Gr.mass_partials += 2 * (size_t)tiles * r;
       if (int s = launch_chunks(C, Gr, mr, maps, 0, cs, kp, r, 1)) return s;
       k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, cs>>>(m, G, C.H, nb, pa(r), pb(r));
-      k_split_to_f64<<<gbf_grid_for(c1 - c0, kThreads, 4), kThreads, 0, cs>>>(m, d->split_rows, d->Pf[1], d->Sf[1],
-                                                                            stP, stS, c0, c1);
+      if (int e = gbf_split_state_to_f64(m, d->split_rows, d->Pf[1], d->Sf[1], stP, stS, c0, c1, cs)) return e;
       GBF_CUDA(cudaGetLastError());
       GBF_CUDA(cudaEventRecord(d->pipe_ev[2 + ns + r], cs));
       GBF_CUDA(cudaStreamWaitEvent(d->pipe_out, d->pipe_ev[2 + ns + r], 0));

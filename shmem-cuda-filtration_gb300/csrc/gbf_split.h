@@ -55,7 +55,7 @@ GbfPatchConsts gbf_patch_consts(const gbf_model& m);
 // row arithmetic once per row instead of once per cell.
 struct GbfRowConst {
   double phs;
-  float c1, c2;
+  double c1, c2;  // FP32 numbers
 };
 // Fill rows[0, ny) for the model (stream-ordered on st).
 int gbf_split_fill_rows(const gbf_model& m, GbfRowConst* rows, cudaStream_t st);
@@ -103,14 +103,14 @@ int gbf_split_launches_per_step(gbf_domain* d);
 // large enough for two slabs of about 1M cells: gbf_split_pipelined).
 int gbf_split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, double* P_out, double* S_out);
 bool gbf_split_pipelined(const gbf_model& m);
-// FP64 (P, S) of every cell from a split state (device arrays; either output
-// may be NULL; rows: the grid's row table, or NULL to form each row's values
-// per cell).
+// FP64 (P, S) of cells [c0, c1) from a split state (device arrays; either
+// output may be NULL).
 int gbf_split_state_to_f64(const gbf_model& m, const GbfRowConst* rows, const float* dPf, const float* Sf, double* P,
-                           double* S, cudaStream_t st);
-// FP32 state and wide masses of one grid from FP64 device arrays (rows as above).
+                           double* S, size_t c0, size_t c1, cudaStream_t st);
+// FP32 state (both buffers) and masses of cells [c0, c1) of a grid from FP64 device arrays.
 int gbf_split_init_state(const gbf_model& m, const GbfRowConst* rows, const double* P_dev, const double* S_dev,
-                         float* dPf, float* Sf, double* M1, double* M2, int mr, cudaStream_t st);
+                         float* const dPf[2], float* const Sf[2], double* M1, double* M2, int mr, size_t c0, size_t c1,
+                         cudaStream_t st);
 // V sum over interior cells of c1(j) phi (the defect form's water mass of a
 // fully water-saturated grid at the row densities): the part of the phase-1
 // mass the tiles' sums leave out. Written to *k1v_host; 0 for other forms.

@@ -6,6 +6,7 @@
 
 #include <type_traits>
 
+#include "gbf_pair.cuh"
 #include "gbf_split.h"
 #include "gbf_tma.h"
 
@@ -1243,40 +1244,54 @@ __device__ bool split_tile(const GbfSplitConsts& C, const GbfSplitGrid& G, int i
   return true;
 }
 
-// Split state of one cell from FP64 P, S: dP = P - P_hs(j), S in FP32 and
-// the phase masses ro1 (1 - S2), ro2 S2 with P2 = P1 (cpu.cpp:72-73, 224-225)
-// in the representation `mr` (defect form: minus c1 (1 - S), c2 S of the
-// FP32 S, products that are exact in FP64).
 // A row's constants for the state conversions (GbfRowConst), as
 // gbf_p_hydrostatic and gbf_defect_row give them.
 __device__ __forceinline__ GbfRowConst gbf_row_const(const gbf_model& m, int j) {
   const GbfDefectRow w = gbf_defect_row(m, j);
-  return {gbf_p_hydrostatic(m, j), w.c1, w.c2};
+  return {gbf_p_hydrostatic(m, j), (double)w.c1, (double)w.c2};
 }
+// Masses of a cell with DNAPL (gbf_split_init_cell), A1 = ro1. A call, so that
+// its FP64 instructions are not issued predicated off for the other cells.
+template <int MR, bool PACKED>
+__device__ __noinline__ double2 gbf_split_wet_masses(double A1, double ro02, double beta2, double pa, double s,
+                                                     double Sd, double c1, double c2) {
+  const double B = __dsub_rn(1., s), A2 = __dmul_rn(ro02, __fma_rn(beta2, pa, 1.));
+  if (!gbf_is_defect(MR)) return make_double2(__dmul_rn(A1, B), __dmul_rn(A2, s));
+  if (PACKED)
+    return make_double2(__fma_rn(-c1, __dsub_rn(1., Sd), __dmul_rn(A1, B)), __fma_rn(-c2, Sd, __dmul_rn(A2, s)));
+  return make_double2(__fma_rn(A1, B, -__dmul_rn(c1, __dsub_rn(1., Sd))), __fma_rn(A2, s, -__dmul_rn(c2, Sd)));
+}
+// Split state of one cell from FP64 P, S: dP = P - P_hs(j), S in FP32 and
+// the phase masses ro1 (1 - S2), ro2 S2 with P2 = P1 (cpu.cpp:72-73, 224-225)
+// in the representation MR (defect forms: minus c1 (1 - S), c2 S of the FP32
+// S, products that are exact in FP64). Bound by the FP64 pipe: its
+// conversions (11 of 25 such instructions a cell) are integer operations
+// (gbf_pair.cuh), and cells without DNAPL take 5 of the 13 others. 256^3, a
+// fifth of the cells with DNAPL: 818 us and a copy of the state -> 230 us
+// with both buffers written. PACKED: the ensembles' packed transfers round
+// the product ro1 (1 - S) and fuse c1 (1 - S); single grids the other way round
+// (1e-13 of a density apart, each as it has always been).
+template <int MR, bool PACKED>
 __device__ __forceinline__ void gbf_split_init_cell(const gbf_model& m, double p, double s, const GbfRowConst& rc,
-                                                    float& dPf, float& Sf, double* M1, double* M2, size_t c, int mr) {
-  dPf = (float)(p - rc.phs);
-  Sf = (float)s;
-  const double m1 = m.ro01 * (1. + m.beta1 * (p - m.P_atm)) * (1. - s);
-  const double m2 = m.ro02 * (1. + m.beta2 * (p - m.P_atm)) * s;
-  if (mr == kMassDefect) {
-    reinterpret_cast<float*>(M1)[c] = (float)(m1 - (double)rc.c1 * (1. - (double)Sf));
-    reinterpret_cast<float*>(M2)[c] = (float)(m2 - (double)rc.c2 * (double)Sf);
-  } else if (mr == kMassDefectDF) {
-    reinterpret_cast<float2*>(M1)[c] = gbf_df_from_double(m1 - (double)rc.c1 * (1. - (double)Sf));
-    reinterpret_cast<float2*>(M2)[c] = gbf_df_from_double(m2 - (double)rc.c2 * (double)Sf);
-  } else if (mr == kMassDF) {
-    reinterpret_cast<float2*>(M1)[c] = gbf_df_from_double(m1);
-    reinterpret_cast<float2*>(M2)[c] = gbf_df_from_double(m2);
+                                                    float& dPf, float& Sf, double* M1, double* M2, size_t c) {
+  double x, Sd;
+  dPf = gbf_d2f(__dsub_rn(p, rc.phs), x);
+  Sf = gbf_d2f(s, Sd);
+  const double pa = __dsub_rn(p, m.P_atm);
+  const double A1 = __dmul_rn(m.ro01, __fma_rn(m.beta1, pa, 1.));
+  double2 w;
+  if (gbf_is_zero(s)) w = make_double2(gbf_is_defect(MR) ? __dsub_rn(A1, rc.c1) : A1, 0.);
+  else w = gbf_split_wet_masses<MR, PACKED>(A1, m.ro02, m.beta2, pa, s, Sd, rc.c1, rc.c2);
+  if (MR == kMassDefect) {
+    reinterpret_cast<float*>(M1)[c] = gbf_d2f(w.x, x);
+    reinterpret_cast<float*>(M2)[c] = gbf_d2f(w.y, x);
   } else {
-    M1[c] = m1;
-    M2[c] = m2;
+    reinterpret_cast<float2*>(M1)[c] = gbf_d2f2(w.x);
+    reinterpret_cast<float2*>(M2)[c] = gbf_d2f2(w.y);
   }
 }
-__device__ __forceinline__ void gbf_split_init_cell(const gbf_model& m, double p, double s, int j, float& dPf,
-                                                    float& Sf, double* M1, double* M2, size_t c, int mr) {
-  gbf_split_init_cell(m, p, s, gbf_row_const(m, j), dPf, Sf, M1, M2, c, mr);
-}
+// FP64 (P, S) of a cell.
+__device__ __forceinline__ double gbf_split_P(float dPf, const GbfRowConst& rc) { return __dadd_rn(rc.phs, gbf_f2d_all(dPf)); }
 
 // Value the reference's boundary sweep leaves in P1 (cpu.cpp:366-403), in
 // the dP = P - P_hs(j) representation: copies within a row keep dP, the top
