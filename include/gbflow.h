@@ -255,8 +255,10 @@ int gbf_domain_kernel_times(gbf_domain* d, double* ms, int* launches, int nkinds
 int gbf_kernel_kinds(void);
 const char* gbf_kernel_name(int kind);
 /* Split kernels stage their x-y planes by TMA (cp.async.bulk.tensor) where a
-   grid qualifies (FP32 K field, no media table, nx % 4 == 0), else by plain
-   loads. 0 forces plain loads for domains and ensembles created afterwards
+   grid qualifies, else by plain loads. Domains: K and porosity fields without
+   a media table, or the media table (or one medium) without either field, any
+   size (their rows are padded to 16 bytes on the device). Ensembles: every
+   member with FP32 K and porosity fields, no media table, nx % 4 == 0. 0 forces plain loads for domains and ensembles created afterwards
    (and ensemble tile lists rebuilt afterwards); default 1. Negative `on`
    leaves the setting as it is. Returns the setting in force before the call. */
 int gbf_set_tma(int on);

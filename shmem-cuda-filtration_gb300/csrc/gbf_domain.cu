@@ -356,8 +356,8 @@ int gbf_domain_save(gbf_domain* d, const char* path, int step) {
     GBF_CUDA(cudaMallocAsync((void**)&tmp, 2 * n * sizeof(double), d->stream));
     const int prev = d->cur ^ 1;
     int s = d->precision == GBF_PREC_F64
-                ? gbf_roS_old_launch(d->m, d->P[prev], d->S[prev], nullptr, nullptr, tmp, tmp + n, d->stream)
-                : gbf_roS_old_launch(d->m, nullptr, nullptr, d->Pf[prev], d->Sf[prev], tmp, tmp + n, d->stream);
+                ? gbf_roS_old_launch(d->m, d->P[prev], d->S[prev], nullptr, nullptr, 0, tmp, tmp + n, d->stream)
+                : gbf_roS_old_launch(d->m, nullptr, nullptr, d->Pf[prev], d->Sf[prev], d->px, tmp, tmp + n, d->stream);
     if (!s) s = gbf_cuda_check(cudaMemcpyAsync(old.data(), tmp, 2 * n * sizeof(double), cudaMemcpyDeviceToHost,
                                                d->stream), "copy roS_old");
     cudaFreeAsync(tmp, d->stream);
@@ -394,7 +394,7 @@ int gbf_domain_write_plots(gbf_domain* d, const char* dir, double t) {
     a.u2y = w + 11 * n; a.u2z = w + 12 * n;
     const int prev = d->cur ^ 1;
     int s = d->precision == GBF_PREC_F64 ? gbf_cuda_check(cudaMemcpyAsync(a.P1, d->P[prev], b, cudaMemcpyDeviceToDevice, d->stream), "copy P")
-                                         : gbf_split_state_to_f64(m, d->split_rows, d->Pf[prev], d->Sf[prev], a.P1, a.S2, 0, n, d->stream);
+                                         : gbf_split_state_to_f64(m, d->px, d->split_rows, d->Pf[prev], d->Sf[prev], a.P1, a.S2, 0, n, d->stream);
     if (!s && d->precision == GBF_PREC_F64)
       s = gbf_cuda_check(cudaMemcpyAsync(a.S2, d->S[prev], b, cudaMemcpyDeviceToDevice, d->stream), "copy S");
     if (!s) s = gbf_props_f64(&m, a, d->cells, d->stream);
@@ -549,7 +549,7 @@ int gbf_dropin_materialize(gbf_domain* d) {
   a.P1 = d->P[1];
   a.S2 = d->S[1];
   if (d->precision != GBF_PREC_F64) {  // split mode: the step-start state is the other split buffer
-    if (int s = gbf_split_state_to_f64(d->m, d->split_rows, d->Pf[d->cur ^ 1], d->Sf[d->cur ^ 1], d->P[1], d->S[1],
+    if (int s = gbf_split_state_to_f64(d->m, d->px, d->split_rows, d->Pf[d->cur ^ 1], d->Sf[d->cur ^ 1], d->P[1], d->S[1],
                                        0, gbf_geo(d->m).n, d->stream))
       return s;
   }
@@ -579,7 +579,7 @@ void gbf_domain_detach_dropin(gbf_domain* d) {
 int gbf_dropin_writeback(gbf_domain* d) {
   if (!d || !d->caller_stale) return GBF_OK;
   d->caller_stale = false;
-  return gbf_split_state_to_f64(d->m, d->split_rows, d->Pf[d->cur], d->Sf[d->cur], d->caller.P1, d->caller.S2, 0,
+  return gbf_split_state_to_f64(d->m, d->px, d->split_rows, d->Pf[d->cur], d->Sf[d->cur], d->caller.P1, d->caller.S2, 0,
                                 gbf_geo(d->m).n, d->stream);
 }
 

@@ -73,6 +73,9 @@ struct gbf_domain {
   // split-precision state (gbf_split.cu)
   float *Pf[2] = {nullptr, nullptr}, *Sf[2] = {nullptr, nullptr};
   double *M1 = nullptr, *M2 = nullptr;
+  int split_plan[3] = {0, 0, 0};  // GbfSplitPlan of the grid
+  int px = 0;              // row pitch of the split state and of split_cells (cells)
+  gbf_cells split_cells = {nullptr, nullptr, nullptr};  // the cells in rows of that pitch (cells itself where px = nx)
   double* split_partials = nullptr;
   float2* split_patch = nullptr;  // the Dirichlet patch's FP64 inflow (split forms; NULL without a patch)
   struct GbfRowConst* split_rows = nullptr;  // the split state conversions' row table (ny entries)
@@ -111,7 +114,7 @@ int gbf_domain_alloc(gbf_domain* d, void** p, size_t bytes);
 
 // roS1_old, roS2_old of interior cells from an FP64 state (P, S) or, with P
 // and S NULL, from a split state (dPf, Sf); boundary cells 0 (gbf_eager.cu).
-int gbf_roS_old_launch(const gbf_model& m, const double* P, const double* S, const float* dPf, const float* Sf,
+int gbf_roS_old_launch(const gbf_model& m, const double* P, const double* S, const float* dPf, const float* Sf, int px,
                        double* o1, double* o2, cudaStream_t st);
 
 // The density of phase 1 or 2 of a pressure field (gbf_f64.cu).

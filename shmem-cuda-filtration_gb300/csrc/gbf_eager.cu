@@ -307,7 +307,8 @@ int launched(const char* where) {
 // the split state (dP from the hydrostatic profile, S in FP32) when P is NULL.
 // Boundary cells get 0.
 __global__ void __launch_bounds__(kThreads) k_roS_old(const gbf_model m, const double* P, const double* S,
-                                                      const float* dPf, const float* Sf, double* o1, double* o2) {
+                                                      const float* dPf, const float* Sf, int px, double* o1,
+                                                      double* o2) {
   const GbfGeo g = gbf_geo(m);
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < g.n; c += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(c % g.nx), j = (int)((c / g.nx) % g.ny), k = (int)(c / g.pl);
@@ -316,8 +317,9 @@ __global__ void __launch_bounds__(kThreads) k_roS_old(const gbf_model m, const d
       o2[c] = 0.;
       continue;
     }
-    const double p = P ? P[c] : gbf_p_hydrostatic(m, j) + (double)dPf[c];
-    const double s = S ? S[c] : (double)Sf[c];
+    const size_t q = c + (size_t)(px - g.nx) * ((size_t)j + (size_t)k * g.ny);  // the split state's rows are px apart
+    const double p = P ? P[c] : gbf_p_hydrostatic(m, j) + (double)dPf[q];
+    const double s = S ? S[c] : (double)Sf[q];
     const double ro1 = m.ro01 * (1. + (m.beta1) * (p - m.P_atm));
     const double ro2 = m.ro02 * (1. + (m.beta2) * (p - m.P_atm));
     o1[c] = ro1 * (1 - s);
@@ -327,9 +329,9 @@ __global__ void __launch_bounds__(kThreads) k_roS_old(const gbf_model m, const d
 
 }  // namespace
 
-int gbf_roS_old_launch(const gbf_model& m, const double* P, const double* S, const float* dPf, const float* Sf,
+int gbf_roS_old_launch(const gbf_model& m, const double* P, const double* S, const float* dPf, const float* Sf, int px,
                        double* o1, double* o2, cudaStream_t st) {
-  k_roS_old<<<gbf_grid_for(gbf_geo(m).n, kThreads), kThreads, 0, st>>>(m, P, S, dPf, Sf, o1, o2);
+  k_roS_old<<<gbf_grid_for(gbf_geo(m).n, kThreads), kThreads, 0, st>>>(m, P, S, dPf, Sf, px, o1, o2);
   GBF_CUDA(cudaGetLastError());
   return GBF_OK;
 }

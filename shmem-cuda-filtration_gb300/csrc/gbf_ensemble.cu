@@ -732,13 +732,13 @@ int build_lists(gbf_ensemble* e) {
     // split_tile_x2 boxes: halo {tx + 8, ty + 2}, rows {tx, ty}
     auto pair_maps = [&](GbfTmaSet& q, const EnsMember& me, const gbf_model& m, int tx, int ty) {
       for (int b = 0; b < 2; b++) {
-        enc |= gbf_tma_encode_box(&q.dP[b], me.dPf[b], 4, m.nx, m.ny, m.nz, tx + 8, ty + 2);
-        enc |= gbf_tma_encode_box(&q.S[b], me.Sf[b], 4, m.nx, m.ny, m.nz, tx + 8, ty + 2);
+        enc |= gbf_tma_encode_box(&q.dP[b], me.dPf[b], 4, m.nx, m.ny, m.nz, m.nx, tx + 8, ty + 2);
+        enc |= gbf_tma_encode_box(&q.S[b], me.Sf[b], 4, m.nx, m.ny, m.nz, m.nx, tx + 8, ty + 2);
       }
-      enc |= gbf_tma_encode_box(&q.K, me.cells.K, 4, m.nx, m.ny, m.nz, tx + 8, ty + 2);
-      enc |= gbf_tma_encode_box(&q.M1, me.M1, mb, m.nx, m.ny, m.nz, tx, ty);
-      enc |= gbf_tma_encode_box(&q.M2, me.M2, mb, m.nx, m.ny, m.nz, tx, ty);
-      enc |= gbf_tma_encode_box(&q.phi, me.cells.phi, 4, m.nx, m.ny, m.nz, tx, ty);
+      enc |= gbf_tma_encode_box(&q.K, me.cells.K, 4, m.nx, m.ny, m.nz, m.nx, tx + 8, ty + 2);
+      enc |= gbf_tma_encode_box(&q.M1, me.M1, mb, m.nx, m.ny, m.nz, m.nx, tx, ty);
+      enc |= gbf_tma_encode_box(&q.M2, me.M2, mb, m.nx, m.ny, m.nz, m.nx, tx, ty);
+      enc |= gbf_tma_encode_box(&q.phi, me.cells.phi, 4, m.nx, m.ny, m.nz, m.nx, tx, ty);
     };
     for (int r = 0; r < e->n && !enc; r++) {
       const EnsMember& me = e->h_mem[r];
@@ -1167,7 +1167,7 @@ int gbf_ensemble_upload(gbf_ensemble* e, int r, const double* P1, const double* 
     GBF_CUDA(cudaMallocAsync((void**)&tmp, 2 * b, e->stream));
     GBF_CUDA(cudaMemcpyAsync(tmp, P1, b, cudaMemcpyDefault, e->stream));
     GBF_CUDA(cudaMemcpyAsync(tmp + nc, S2, b, cudaMemcpyDefault, e->stream));
-    if (int s = gbf_split_init_state(m, me.rows, tmp, tmp + nc, me.dPf, me.Sf, me.M1, me.M2,
+    if (int s = gbf_split_init_state(m, m.nx, me.rows, tmp, tmp + nc, me.dPf, me.Sf, me.M1, me.M2,
                                      gbf_mass_rep(e->precision), 0, nc, e->stream))
       return s;
     GBF_CUDA(cudaFreeAsync(tmp, e->stream));
@@ -1340,7 +1340,7 @@ int gbf_ensemble_download(gbf_ensemble* e, int r, int field, double* host) {
   } else {
     double* tmp = nullptr;
     GBF_CUDA(cudaMallocAsync((void**)&tmp, b, e->stream));
-    if (int s = gbf_split_state_to_f64(m, me.rows, me.dPf[e->cur], me.Sf[e->cur], field == GBF_FIELD_P1 ? tmp : nullptr,
+    if (int s = gbf_split_state_to_f64(m, m.nx, me.rows, me.dPf[e->cur], me.Sf[e->cur], field == GBF_FIELD_P1 ? tmp : nullptr,
                                        field == GBF_FIELD_S2 ? tmp : nullptr, 0, nc, e->stream))
       return s;
     GBF_CUDA(cudaMemcpyAsync(host, tmp, b, cudaMemcpyDefault, e->stream));

@@ -38,18 +38,21 @@ const void* gbf_mapped_host(const void* p);
 // ---------------------------------------------------------------- geometry
 struct GbfGeo {
   int nx, ny, nz;
-  size_t pl;  // nx * ny
+  int px;     // row pitch in cells: nx, or more for the split state of grids whose rows are padded
+  size_t pl;  // px * ny
   size_t n;   // nx * ny * nz
 };
 
-GBF_HD GbfGeo gbf_geo(const gbf_model& m) {
+GBF_HD GbfGeo gbf_geo(const gbf_model& m, int px) {
   GbfGeo g;
   g.nx = m.nx; g.ny = m.ny; g.nz = m.nz;
-  g.pl = (size_t)m.nx * (size_t)m.ny;
-  g.n = g.pl * (size_t)m.nz;
+  g.px = px;
+  g.pl = (size_t)px * (size_t)m.ny;
+  g.n = (size_t)m.nx * (size_t)m.ny * (size_t)m.nz;
   return g;
 }
-GBF_HD size_t gbf_idx(const GbfGeo& g, int i, int j, int k) { return (size_t)i + (size_t)j * g.nx + (size_t)k * g.pl; }
+GBF_HD GbfGeo gbf_geo(const gbf_model& m) { return gbf_geo(m, m.nx); }
+GBF_HD size_t gbf_idx(const GbfGeo& g, int i, int j, int k) { return (size_t)i + (size_t)j * g.px + (size_t)k * g.pl; }
 GBF_HD bool gbf_is_boundary(const GbfGeo& g, int i, int j, int k) {
   return i == 0 || i == g.nx - 1 || j == 0 || j == g.ny - 1 || k == 0 || k == g.nz - 1;
 }
@@ -59,11 +62,13 @@ GBF_HD bool gbf_is_boundary(const GbfGeo& g, int i, int j, int k) {
 //   [.., + 2*nx*(nz-2))               faces j = 0 and j = ny-1 (k interior)
 //   [.., + 2*(ny-2)*(nz-2))           faces i = 0 and i = nx-1 (j, k interior)
 GBF_HD size_t gbf_boundary_count(const GbfGeo& g) {
-  return 2 * g.pl + 2 * (size_t)g.nx * (g.nz - 2) + 2 * (size_t)(g.ny - 2) * (g.nz - 2);
+  return 2 * (size_t)g.nx * g.ny + 2 * (size_t)g.nx * (g.nz - 2) + 2 * (size_t)(g.ny - 2) * (g.nz - 2);
 }
 // The first two groups only: every boundary cell but the x faces with j, k
 // interior (which the x-pair split tile writes itself).
-GBF_HD size_t gbf_boundary_count_no_xfaces(const GbfGeo& g) { return 2 * g.pl + 2 * (size_t)g.nx * (g.nz - 2); }
+GBF_HD size_t gbf_boundary_count_no_xfaces(const GbfGeo& g) {
+  return 2 * (size_t)g.nx * g.ny + 2 * (size_t)g.nx * (g.nz - 2);
+}
 // The same cells as rows of nx cells at (j, k), "face rows":
 //   r in [0, 2 ny)                  k = 0 (r < ny) or nz - 1, j = r mod ny
 //   r in [2 ny, 2 ny + 2 (nz - 2))  j = 0 or ny - 1, k = 1 + (r - 2 ny) mod (nz - 2)
@@ -84,7 +89,7 @@ GBF_HD void gbf_face_row(const GbfGeo& g, int r, int& j, int& k) {
 // division is emulated on the GPU.
 GBF_HD void gbf_boundary_cell(const GbfGeo& g, size_t id_, int& i, int& j, int& k) {
   unsigned id = (unsigned)id_;
-  const unsigned nx = (unsigned)g.nx, pl = (unsigned)g.pl;
+  const unsigned nx = (unsigned)g.nx, pl = nx * (unsigned)g.ny;
   const unsigned a = 2u * pl;
   if (id < a) {
     k = id < pl ? 0 : g.nz - 1;

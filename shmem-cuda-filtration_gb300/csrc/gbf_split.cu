@@ -19,7 +19,7 @@
 
 #include <algorithm>
 
-#include "gbf_split_tile.cuh"
+#include "gbf_split_x2.cuh"
 
 GbfPatchConsts gbf_patch_consts(const gbf_model& m) {
   GbfPatchConsts P = {};
@@ -39,8 +39,9 @@ GbfPatchConsts gbf_patch_consts(const gbf_model& m) {
   return P;
 }
 
-GbfSplitConsts gbf_split_consts(const gbf_model& m) {
+GbfSplitConsts gbf_split_consts(const gbf_model& m, int px) {
   GbfSplitConsts C = {};
+  C.px = px;
   C.nx = m.nx; C.ny = m.ny; C.nz = m.nz;
   C.noflow_bottom = (m.bc_mode == GBF_BC_HYDROSTATIC_SIDES);
   const double V = m.h1 * m.h2 * m.h3;
@@ -110,11 +111,6 @@ constexpr int kThreads = 256;
 
 int tiles_x(const GbfSplitConsts& C) { return (C.nx - 2 + kSplitTX - 1) / kSplitTX; }
 int tiles_y(const GbfSplitConsts& C) { return (C.ny - 2 + kSplitTY - 1) / kSplitTY; }
-// x-pair tiles (TMA staging): 64 x 8 cells from x0 = 64 t, t such that x0 <= nx - 2
-constexpr int kPairTX = 64, kPairTY = 8;
-__host__ __device__ int tiles_x2(const GbfSplitConsts& C) { return (C.nx - 1 + kPairTX - 1) / kPairTX; }
-__host__ __device__ int tiles_y2(const GbfSplitConsts& C) { return (C.ny - 2 + kPairTY - 1) / kPairTY; }
-
 // The plain-load tile on one grid (grids without TMA staging). Block b runs
 // tile b mod (tiles of a chunk layer) of the k chunk kc0 + b / (tiles of a
 // layer), kchunk planes from 1 + kchunk kc; G.mass_partials is that launch's
@@ -135,42 +131,11 @@ __global__ void __launch_bounds__(kSplitThreads, 4) k_split_step(const GbfSplitC
   if constexpr (CFL) split_block_cfl<kSplitThreads>(acc.cfl1, acc.cfl2, G.cfl_out);
 }
 
-// The x-pair tile on one grid: one tile (64 x 8 cells, a k range) per CTA,
-// blocks mapped to tiles and k chunks as in k_split_step.
-template <int MR, bool CFL, bool PATCH>
-__global__ void __launch_bounds__(kPairTX / 2 * kPairTY, gbf_pair_ctas(MR)) k_split_step_x2(const GbfSplitConsts C,
-                                                                         const GbfSplitGrid G, const int kchunk,
-                                                                         const int kc0, const GbfTmaSet* maps,
-                                                                         int buf) {
-  extern __shared__ __align__(128) unsigned char dyn[];
-  using Cta = GbfPairCta<kPairTX, kPairTY, MR>;
-  Cta& cta = *reinterpret_cast<Cta*>(dyn);
-  if (gbf_smem_u32(dyn) & 127u) {  // the TMA destinations need it; never expected to fire
-    if (threadIdx.x == 0) atomicOr(G.status, GBF_DEV_TIMEOUT);
-    return;
-  }
-  const int ntx = tiles_x2(C), nty = tiles_y2(C);
-  const int b = blockIdx.x;
-  const int tx = b % ntx, ty = (b / ntx) % nty, kc = kc0 + b / (ntx * nty);
-  const int k0 = 1 + kc * kchunk;
-  const int k1 = min(k0 + kchunk, C.nz - 1);
-  if (threadIdx.x == 0) gbf_pair_bars_init(cta.bars);
-  __syncthreads();
-  unsigned phases = 0;
-  GbfSplitAcc<MR> acc;
-  split_tile_x2<MR, kPairTX, kPairTY, CFL, kPairTX / 2 * kPairTY, PATCH>(C, G, kPairTX * tx, 1 + kPairTY * ty, k0,
-                                                                         k1, cta.bars, cta.body, acc, maps, buf,
-                                                                         &phases);
-  if (acc.bad) atomicOr(G.status, GBF_DEV_NONFINITE);
-  if (G.mass_partials) split_block_mass<MR, kPairTX / 2 * kPairTY>(acc, C.V, G.mass_partials + 2 * blockIdx.x);
-  if constexpr (CFL) split_block_cfl<kPairTX / 2 * kPairTY>(acc.cfl1, acc.cfl2, G.cfl_out);
-}
-
 // Boundary cells [0, nb) of gbf_boundary_cell's enumeration (all, or all but
 // the x faces that the x-pair tile writes).
-__global__ void __launch_bounds__(kThreads) k_split_boundary(const gbf_model m, const GbfSplitGrid G, float H,
+__global__ void __launch_bounds__(kThreads) k_split_boundary(const gbf_model m, int px, const GbfSplitGrid G, float H,
                                                              size_t nb, int k_lo, int k_hi) {
-  const GbfGeo g = gbf_geo(m);
+  const GbfGeo g = gbf_geo(m, px);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb; t += (size_t)gridDim.x * blockDim.x) {
     int i, j, k;
     gbf_boundary_cell(g, t, i, j, k);
@@ -227,9 +192,9 @@ __global__ void k_split_mass_tail(const double* partials, int nblocks, double* o
 // cells, the loads of a thread's cells in flight together.
 constexpr int kConvPer = 4, kConvCells = kConvPer * kThreads;
 template <int MR>
-__global__ void __launch_bounds__(kThreads) k_split_init(const gbf_model m, const GbfFastDiv dnx, const GbfFastDiv dny,
-                                                         const GbfRowConst* rows, const double* P, const double* S,
-                                                         float* dP0, float* dP1, float* S0, float* S1, double* M1,
+__global__ void __launch_bounds__(kThreads) k_split_init(const gbf_model m, int px, const GbfFastDiv dnx,
+                                                         const GbfFastDiv dny, const GbfRowConst* rows, const double* P,
+                                                         const double* S, float* dP0, float* dP1, float* S0, float* S1, double* M1,
                                                          double* M2, unsigned c0, unsigned c1) {
   const unsigned b = c0 + blockIdx.x * kConvCells + threadIdx.x;
   double p[kConvPer], s[kConvPer];
@@ -245,19 +210,19 @@ __global__ void __launch_bounds__(kThreads) k_split_init(const gbf_model m, cons
   for (int u = 0; u < kConvPer; u++) {
     const unsigned c = b + u * kThreads;
     if (c < c1) {
-      const unsigned r = gbf_div(c, dnx), j = r - gbf_div(r, dny) * dny.d;
+      const unsigned r = gbf_div(c, dnx), j = r - gbf_div(r, dny) * dny.d, q = c + r * (unsigned)(px - m.nx);
       float dp, sf;
-      gbf_split_init_cell<MR, false>(m, p[u], s[u], rows[j], dp, sf, M1, M2, c);
-      dP0[c] = dp;
-      dP1[c] = dp;  // the next-state buffer's faces are rewritten every step; they start equal
-      S0[c] = sf;
-      S1[c] = sf;
+      gbf_split_init_cell<MR, false>(m, p[u], s[u], rows[j], dp, sf, M1, M2, q);
+      dP0[q] = dp;
+      dP1[q] = dp;  // the next-state buffer's faces are rewritten every step; they start equal
+      S0[q] = sf;
+      S1[q] = sf;
     }
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_split_to_f64(const GbfFastDiv dnx, const GbfFastDiv dny,
-                                                           const GbfRowConst* rows, const float* dPf, const float* Sf,
+__global__ void __launch_bounds__(kThreads) k_split_to_f64(unsigned pad, const GbfFastDiv dnx,
+                                                           const GbfFastDiv dny, const GbfRowConst* rows, const float* dPf, const float* Sf,
                                                            double* P, double* S, unsigned c0, unsigned c1) {
   const unsigned b = c0 + blockIdx.x * kConvCells + threadIdx.x;
   float p[kConvPer], s[kConvPer];
@@ -265,8 +230,9 @@ __global__ void __launch_bounds__(kThreads) k_split_to_f64(const GbfFastDiv dnx,
   for (int u = 0; u < kConvPer; u++) {
     const unsigned c = b + u * kThreads;
     if (c < c1) {
-      if (P) p[u] = dPf[c];
-      if (S) s[u] = Sf[c];
+      const unsigned q = pad ? c + gbf_div(c, dnx) * pad : c;  // pad: the padding of a row
+      if (P) p[u] = dPf[q];
+      if (S) s[u] = Sf[q];
     }
   }
 #pragma unroll
@@ -294,48 +260,68 @@ __global__ void k_split_rows(const gbf_model m, GbfRowConst* rows) {
 // at least 16 planes (or the whole column), take the one with the fewest
 // plane-times: waves x (planes per CTA + about 1.5 for the prologue, which
 // builds the first plane and loads the plane below it). Grids that fill
-// less than one wave may go down to 8 planes per CTA.
-int gbf_split_kchunk_waves(long long tiles, int nzi, long long slots) {
-  if (nzi < 1) return 1;
+// less than one wave may go down to 2 planes per CTA: there the planes a CTA
+// marches through are the step's latency (40^3: 8 planes 19.4 us a step, 2
+// planes 13.0).
+int gbf_split_kchunk_waves(long long tiles, int nzi, long long slots, double* cost_out = nullptr) {
+  if (nzi < 1) nzi = 1;
   if (slots < 1) slots = 1;
-  const int max_chunks = (nzi + 7) / 8;
+  const int max_chunks = (nzi + 1) / 2;
   int best = nzi;
   double best_cost = 1e300;
   for (int chunks = 1; chunks <= max_chunks; chunks++) {
     const int kc = (nzi + chunks - 1) / chunks;
     const long long ctas = tiles * ((nzi + kc - 1) / kc);
-    if (chunks > 1 && kc < 16 && (kc < 8 || ctas > slots)) continue;
+    if (chunks > 1 && kc < 16 && ctas > slots) continue;
     const double cost = (double)((ctas + slots - 1) / slots) * (kc + 1.5);
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
       best = kc;
     }
   }
+  if (cost_out) *cost_out = best_cost;
   return best;
 }
 
-// Resident CTAs per SM of the two single-grid tiles (launch bounds and shared memory: the 32x8
-// plain-load tile 4, the x-pair tile gbf_pair_ctas: 3 in the defect form, else 2).
-int gbf_split_kchunk(const GbfSplitConsts& C) {
-  return gbf_split_kchunk_waves((long long)tiles_x(C) * tiles_y(C), C.nz - 2, 4LL * gbf_num_sms());
+namespace {
+constexpr int kPairTX[kPairShapes] = {64, 32, 16}, kPairTY[kPairShapes] = {8, 16, 32};
+long long pair_tiles(const GbfSplitConsts& C, int shape) {
+  return (long long)((C.nx - 1 + kPairTX[shape] - 1) / kPairTX[shape]) *
+         ((C.ny - 2 + kPairTY[shape] - 1) / kPairTY[shape]);
 }
-int gbf_split_kchunk_x2(const GbfSplitConsts& C, int mr) {
-  return gbf_split_kchunk_waves((long long)tiles_x2(C) * tiles_y2(C), C.nz - 2,
-                                (long long)gbf_pair_ctas(mr) * gbf_num_sms());
+}  // namespace
+
+// Resident CTAs per SM (launch bounds and shared memory): the 32x8 plain-load
+// tile 4, the x-pair tiles gbf_pair_ctas: 3 in the defect form (2 in the 16x32
+// shape, 77 KB of shared memory), else 2. The x-pair shape is the one with the
+// fewest plane-times: a grid's rows fill 64 lanes badly where nx is just above
+// a multiple of 64 or small (13x300x280: 68.6 us a step with 64x8, 29.7 with
+// 16x32; 151x97x83: 31.2 and 29.3 with 32x16), and the three cost the same a
+// plane.
+GbfSplitPlan gbf_split_plan(const GbfSplitConsts& C, int mr, bool tma) {
+  const long long sms = gbf_num_sms();
+  if (!tma) {
+    const int kc = gbf_split_kchunk_waves((long long)tiles_x(C) * tiles_y(C), C.nz - 2, 4 * sms);
+    return {0, kc, kc};
+  }
+  GbfSplitPlan plan = {};
+  double best = 1e300;
+  for (int shape = 0; shape < kPairShapes; shape++) {
+    const int ctas = mr == kMassDefect && shape == kPair16x32 ? 2 : gbf_pair_ctas(mr);
+    double cost;
+    const int kc = gbf_split_kchunk_waves(pair_tiles(C, shape), C.nz - 2, ctas * sms, &cost);
+    if (shape == kPair64x8) plan.kchunk_cfl = kc;
+    if (cost < best - 1e-9) {
+      best = cost;
+      plan.shape = shape;
+      plan.kchunk = kc;
+    }
+  }
+  return plan;
 }
 
 // The step tiles of k chunks [kc0, kc0 + nkc) (kchunk planes each): the
 // x-pair tile with TMA staging (maps), else the plain-load tile.
-template <int MR, bool CFL, bool PATCH>
-int launch_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, const GbfTmaSet* maps, int buf, cudaStream_t st,
-              int kchunk, int kc0, int nkc) {
-  const unsigned blocks = (unsigned)(tiles_x2(C) * tiles_y2(C) * nkc);
-  const int bytes = (int)sizeof(GbfPairCta<kPairTX, kPairTY, MR>);
-  GBF_CUDA(cudaFuncSetAttribute(k_split_step_x2<MR, CFL, PATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  k_split_step_x2<MR, CFL, PATCH><<<blocks, kPairTX / 2 * kPairTY, bytes, st>>>(C, G, kchunk, kc0, maps, buf);
-  return GBF_OK;
-}
-
 namespace {
 // The Dirichlet patch's pre-pass, one thread per patch cell (gbf_split_patch_cell).
 __global__ void __launch_bounds__(kThreads) k_split_patch(const GbfSplitConsts C, const GbfPatchConsts P,
@@ -346,57 +332,56 @@ __global__ void __launch_bounds__(kThreads) k_split_patch(const GbfSplitConsts C
 }  // namespace
 
 template <int MR, bool PATCH>
-int launch_tiles(const GbfSplitConsts& C, const GbfSplitGrid& G, const GbfTmaSet* maps, int buf, cudaStream_t st,
-                 int kchunk, int kc0, int nkc) {
-  const bool cfl = G.cfl_out != nullptr;
-  if (maps)
-    return cfl ? launch_x2<MR, true, PATCH>(C, G, maps, buf, st, kchunk, kc0, nkc)
-               : launch_x2<MR, false, PATCH>(C, G, maps, buf, st, kchunk, kc0, nkc);
+int launch_plain(const GbfSplitConsts& C, const GbfSplitGrid& G, cudaStream_t st, int kchunk, int kc0, int nkc) {
   const unsigned blocks = (unsigned)(tiles_x(C) * tiles_y(C) * nkc);
-  if (cfl) k_split_step<MR, true, PATCH><<<blocks, kSplitThreads, 0, st>>>(C, G, kchunk, kc0);
+  if (G.cfl_out) k_split_step<MR, true, PATCH><<<blocks, kSplitThreads, 0, st>>>(C, G, kchunk, kc0);
   else k_split_step<MR, false, PATCH><<<blocks, kSplitThreads, 0, st>>>(C, G, kchunk, kc0);
   return GBF_OK;
 }
 
-// The tiles under a Dirichlet patch (G.patch_in set) are the PATCH instantiations.
-int launch_chunks(const GbfSplitConsts& C, const GbfSplitGrid& G, int mr, const GbfTmaSet* maps, int buf,
+// The step tiles of k chunks [kc0, kc0 + nkc) (kchunk planes each): the
+// x-pair tile with TMA staging (maps), else the plain-load tile. Under a
+// Dirichlet patch (G.patch_in set) the PATCH instantiations.
+int launch_chunks(const GbfSplitConsts& C, const GbfSplitGrid& G, int mr, int shape, const GbfTmaSet* maps, int buf,
                   cudaStream_t st, int kchunk, int kc0, int nkc) {
+  if (maps) {
+    if (shape != kPair64x8) maps++;
+    return G.K ? gbf_launch_x2_fields(shape, C, G, mr, maps, buf, st, kchunk, kc0, nkc)
+               : gbf_launch_x2_table(shape, C, G, mr, maps, buf, st, kchunk, kc0, nkc);
+  }
   auto form = [&](auto tag) {
     constexpr int MR = decltype(tag)::value;
-    return G.patch_in ? launch_tiles<MR, true>(C, G, maps, buf, st, kchunk, kc0, nkc)
-                      : launch_tiles<MR, false>(C, G, maps, buf, st, kchunk, kc0, nkc);
+    return G.patch_in ? launch_plain<MR, true>(C, G, st, kchunk, kc0, nkc) : launch_plain<MR, false>(C, G, st, kchunk, kc0, nkc);
   };
   return mr == kMassDefect ? form(std::integral_constant<int, kMassDefect>{})
          : mr == kMassDF   ? form(std::integral_constant<int, kMassDF>{})
                            : form(std::integral_constant<int, kMassDefectDF>{});
 }
-// A step's k chunking: kchunk planes a chunk, and the tiles of a chunk layer.
-int step_kchunk(const GbfSplitConsts& C, int mr, const GbfTmaSet* maps) {
-  return maps ? gbf_split_kchunk_x2(C, mr) : gbf_split_kchunk(C);
-}
-long long layer_tiles(const GbfSplitConsts& C, const GbfTmaSet* maps) {
-  return maps ? (long long)tiles_x2(C) * tiles_y2(C) : (long long)tiles_x(C) * tiles_y(C);
+// The shape of a step's tiles (CFL numbers: 64x8), and the tiles of a chunk layer.
+int step_shape(const GbfSplitGrid& G, const GbfSplitPlan& plan) { return G.cfl_out ? kPair64x8 : plan.shape; }
+long long layer_tiles(const GbfSplitConsts& C, int shape, const GbfTmaSet* maps) {
+  return maps ? pair_tiles(C, shape) : (long long)tiles_x(C) * tiles_y(C);
 }
 
 int gbf_split_launch_domain(const gbf_model& m, const GbfSplitConsts& C, const GbfSplitGrid& G, int mr,
                             double* mass_out, cudaStream_t st, GbfTimer* tm, const GbfTmaSet* maps, int buf,
-                            double k1v) {
-  const int kchunk = step_kchunk(C, mr, maps);
+                            double k1v, const GbfSplitPlan& plan) {
+  const int shape = step_shape(G, plan), kchunk = G.cfl_out ? plan.kchunk_cfl : plan.kchunk;
   const int nkc = (C.nz - 2 + kchunk - 1) / kchunk;
-  const unsigned blocks = (unsigned)(layer_tiles(C, maps) * nkc);
+  const unsigned blocks = (unsigned)(layer_tiles(C, shape, maps) * nkc);
   cudaEvent_t e = gbf_timer_begin(tm, st);
   if (G.patch_in) {  // the Dirichlet patch's FP64 inflow, timed with the step kernel
     const GbfPatchConsts P = gbf_patch_consts(m);
     k_split_patch<<<gbf_grid_for((size_t)P.n * P.n, kThreads), kThreads, 0, st>>>(C, P, G);
   }
   // TMA staging (maps): the x-pair tile; else the plain-load tile
-  if (int s = launch_chunks(C, G, mr, maps, buf, st, kchunk, 0, nkc)) return s;
+  if (int s = launch_chunks(C, G, mr, shape, maps, buf, st, kchunk, 0, nkc)) return s;
   gbf_timer_end(tm, GBF_K_SPLIT_STEP, e, st);
   e = gbf_timer_begin(tm, st);
   // one cell per thread (row segments, as the ensembles' face pass walks
   // them, measured 8.6 -> 10.4 us on 256^3: too few warps for a latency-bound pass)
   const size_t nb = maps ? gbf_boundary_count_no_xfaces(gbf_geo(m)) : gbf_boundary_count(gbf_geo(m));
-  k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, st>>>(m, G, C.H, nb, 0, C.nz);
+  k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, st>>>(m, C.px, G, C.H, nb, 0, C.nz);
   gbf_timer_end(tm, GBF_K_SPLIT_BOUNDARY, e, st);
   if (G.mass_partials && mass_out) {
     e = gbf_timer_begin(tm, st);
@@ -407,7 +392,6 @@ int gbf_split_launch_domain(const gbf_model& m, const GbfSplitConsts& C, const G
   return err == cudaSuccess ? GBF_OK : gbf_cuda_check(err, "gbf_split_launch_domain");
 }
 
-// Mass-partial slots: the larger of the two tilings' CTA counts.
 // The host-resident pipeline's slabs (gbf_split_advance_host): one k chunk
 // layer of the step each, about 1M cells (16 MB each way) or more, so that a
 // slab's copies outlast its few launches, at most 16, at least 4 planes.
@@ -425,19 +409,56 @@ bool gbf_split_pipelined(const gbf_model& m) {
   return pipe_slabs(C) >= 2 && (C.nz - 2 + pipe_kchunk(C) - 1) / pipe_kchunk(C) >= 2;
 }
 
+// Mass-partial slots: the largest CTA count of the grid's launches.
 unsigned gbf_split_blocks(const gbf_model& m, int mr) {
   const GbfSplitConsts C = gbf_split_consts(m);
-  const int kchunk = gbf_split_kchunk(C), kc2 = gbf_split_kchunk_x2(C, mr), kp = pipe_kchunk(C);
-  const unsigned a = (unsigned)(tiles_x(C) * tiles_y(C) * ((C.nz - 2 + kchunk - 1) / kchunk));
-  const unsigned b = (unsigned)(tiles_x2(C) * tiles_y2(C) * ((C.nz - 2 + kc2 - 1) / kc2));
-  const unsigned p = (unsigned)(std::max(tiles_x(C) * tiles_y(C), tiles_x2(C) * tiles_y2(C)) * ((C.nz - 2 + kp - 1) / kp));
-  return std::max(a, std::max(b, p));
+  const GbfSplitPlan a = gbf_split_plan(C, mr, false), b = gbf_split_plan(C, mr, true);
+  const int kp = pipe_kchunk(C);
+  auto ctas = [&](long long tiles, int kc) { return tiles * ((C.nz - 2 + kc - 1) / kc); };
+  long long most = ctas((long long)tiles_x(C) * tiles_y(C), std::min(a.kchunk, kp));
+  most = std::max(most, ctas(pair_tiles(C, kPair64x8), std::min(b.kchunk_cfl, kp)));
+  return (unsigned)std::max(most, ctas(pair_tiles(C, b.shape), std::min(b.kchunk, kp)));
 }
 
 // ----------------------------------------------------------------- host side
 
+// A field of the caller's cells (nx a row) to rows px apart.
+__global__ void __launch_bounds__(kThreads) k_split_pitch(const unsigned* src, unsigned* dst, GbfFastDiv dnx, unsigned pad,
+                                                          unsigned n) {
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
+    dst[c + gbf_div(c, dnx) * pad] = src[c];
+}
+static int pitch_field(gbf_domain* d, const void* src, const void* dst) {
+  const unsigned n = (unsigned)gbf_geo(d->m).n;
+  k_split_pitch<<<gbf_grid_for(n, kThreads), kThreads, 0, d->stream>>>((const unsigned*)src, (unsigned*)dst,
+                                                                       gbf_fast_div((unsigned)d->m.nx),
+                                                                       (unsigned)(d->px - d->m.nx), n);
+  GBF_CUDA(cudaGetLastError());
+  return GBF_OK;
+}
+int gbf_split_pitch_media(gbf_domain* d) {
+  if (d->split_cells.media == d->cells.media) return GBF_OK;
+  return pitch_field(d, d->cells.media, d->split_cells.media);
+}
+
 int gbf_split_alloc(gbf_domain* d) {
-  const size_t n = gbf_geo(d->m).n;
+  const gbf_model& m = d->m;
+  // Grids with K and porosity fields and no media table, or with the media
+  // table (or one medium) and no field, run the x-pair tile: TMA staging wants
+  // rows of whole 16-byte units, so the split state's and the fields' rows are
+  // padded to that. Measured against the plain-load tile, us a step: 256^3 of
+  // the media table under the Dirichlet patch 322 -> 214, 255x253x251 with
+  // fields 271 -> 193, 67x45x150 of the table 36.5 -> 31.4, 40^3 15.1 -> 13.0.
+  const bool fields = d->cells.K && d->cells.phi && !d->cells.media, table = !d->cells.K && !d->cells.phi;
+  const int pitch = (m.nx + 3) / 4 * 4;
+  const bool tma = (fields || table) && gbf_tma_eligible(pitch, 64) &&
+                   (double)pitch * m.ny * m.nz < 2147483648.0;
+  d->px = tma ? pitch : m.nx;
+  const GbfSplitPlan plan = gbf_split_plan(gbf_split_consts(m), gbf_mass_rep(d->precision), tma);
+  d->split_plan[0] = plan.shape;
+  d->split_plan[1] = plan.kchunk;
+  d->split_plan[2] = plan.kchunk_cfl;
+  const size_t n = (size_t)d->px * m.ny * m.nz;
   int s = GBF_OK;
   for (int b = 0; b < 2 && !s; b++) {
     s |= gbf_domain_alloc(d, (void**)&d->Pf[b], n * sizeof(float));
@@ -447,6 +468,17 @@ int gbf_split_alloc(gbf_domain* d) {
   const int mb = gbf_mass_bytes(gbf_mass_rep(d->precision));
   if (!s) s |= gbf_domain_alloc(d, (void**)&d->M1, n * mb);
   if (!s) s |= gbf_domain_alloc(d, (void**)&d->M2, n * mb);
+  d->split_cells = d->cells;
+  if (!s && d->px != m.nx) {  // the cell fields in padded rows
+    auto padded = [&](const void* src, const void** dst) {
+      if (!src || s) return;
+      s |= gbf_domain_alloc(d, (void**)dst, n * 4);
+      if (!s) s |= pitch_field(d, src, *dst);
+    };
+    padded(d->cells.K, (const void**)&d->split_cells.K);
+    padded(d->cells.phi, (const void**)&d->split_cells.phi);
+    padded(d->cells.media, (const void**)&d->split_cells.media);
+  }
   // the defect form's water-mass part left out of the tiles' sums
   d->defect_k1v = 0.0;
   if (!s && gbf_is_defect(gbf_mass_rep(d->precision)))
@@ -463,27 +495,31 @@ int gbf_split_alloc(gbf_domain* d) {
     if (!s) s |= gbf_cuda_check(cudaMemset(d->split_patch, 0, sizeof(float2) * (size_t)pn * pn), "gbf_split_alloc");
   }
   if (s) return GBF_ERR_NOMEM;
-  // TMA plane loads: FP32 K and phi fields, no media table, rows of whole 16-byte units
-  const gbf_model& m = d->m;
-  if (d->cells.K && d->cells.phi && !d->cells.media && gbf_tma_eligible(m.nx, kPairTX)) {
-    // boxes of the x-pair tile: halo planes {TX + 8, TY + 2}, interior rows {TX, TY}
-    GbfTmaSet h;
+  if (tma) {
+    // boxes of the x-pair tile, 64x8 and the plan's: halo planes {TX + 8, TY + 2}
+    // (K, or the media indices), interior rows {TX, TY}
+    GbfTmaSet h[2] = {};
     int e = GBF_OK;
-    const int hx = kPairTX + 8, hy = kPairTY + 2;
-    for (int b = 0; b < 2 && !e; b++) {
-      e |= gbf_tma_encode_box(&h.dP[b], d->Pf[b], 4, m.nx, m.ny, m.nz, hx, hy);
-      e |= gbf_tma_encode_box(&h.S[b], d->Sf[b], 4, m.nx, m.ny, m.nz, hx, hy);
+    const int px = d->px, shapes[2] = {kPair64x8, d->split_plan[0]};
+    const gbf_cells& c = d->split_cells;
+    const void* k = fields ? (const void*)c.K : (const void*)c.media;
+    for (int q = 0; q < 2 && !e; q++) {
+      const int tx = kPairTX[shapes[q]], ty = kPairTY[shapes[q]];
+      auto box = [&](void* map, const void* base, int eb, int bx, int by) {
+        if (!e) e |= gbf_tma_encode_box(map, base, eb, m.nx, m.ny, m.nz, px, bx, by);
+      };
+      for (int b = 0; b < 2; b++) {
+        box(&h[q].dP[b], d->Pf[b], 4, tx + 8, ty + 2);
+        box(&h[q].S[b], d->Sf[b], 4, tx + 8, ty + 2);
+      }
+      if (k) box(&h[q].K, k, 4, tx + 8, ty + 2);
+      box(&h[q].M1, d->M1, mb, tx, ty);
+      box(&h[q].M2, d->M2, mb, tx, ty);
+      if (fields) box(&h[q].phi, c.phi, 4, tx, ty);
     }
-    if (!e) e |= gbf_tma_encode_box(&h.K, d->cells.K, 4, m.nx, m.ny, m.nz, hx, hy);
-    if (!e) e |= gbf_tma_encode_box(&h.M1, d->M1, mb, m.nx, m.ny, m.nz, kPairTX, kPairTY);
-    if (!e) e |= gbf_tma_encode_box(&h.M2, d->M2, mb, m.nx, m.ny, m.nz, kPairTX, kPairTY);
-    if (!e) e |= gbf_tma_encode_box(&h.phi, d->cells.phi, 4, m.nx, m.ny, m.nz, kPairTX, kPairTY);
-    if (!e && !gbf_domain_alloc(d, &d->tma, sizeof(GbfTmaSet))) {
-      GBF_CUDA(cudaMemcpy(d->tma, &h, sizeof(GbfTmaSet), cudaMemcpyHostToDevice));
-    } else {
-      d->tma = nullptr;  // plain loads
-      gbf_clear_status();
-    }
+    if (!e) e |= gbf_domain_alloc(d, &d->tma, sizeof(h));
+    if (e) return GBF_ERR_CUDA;
+    GBF_CUDA(cudaMemcpy(d->tma, h, sizeof(h), cudaMemcpyHostToDevice));
   }
   return GBF_OK;
 }
@@ -508,13 +544,13 @@ int gbf_split_fill_rows(const gbf_model& m, GbfRowConst* rows, cudaStream_t st) 
   return e == cudaSuccess ? GBF_OK : gbf_cuda_check(e, "gbf_split_fill_rows");
 }
 
-int gbf_split_init_state(const gbf_model& m, const GbfRowConst* rows, const double* P_dev, const double* S_dev,
+int gbf_split_init_state(const gbf_model& m, int px, const GbfRowConst* rows, const double* P_dev, const double* S_dev,
                          float* const dPf[2], float* const Sf[2], double* M1, double* M2, int mr, size_t c0, size_t c1,
                          cudaStream_t st) {
   const GbfFastDiv dnx = gbf_fast_div((unsigned)m.nx), dny = gbf_fast_div((unsigned)m.ny);
   const unsigned blocks = (unsigned)((c1 - c0 + kConvCells - 1) / kConvCells);
   auto kern = mr == kMassDefect ? k_split_init<kMassDefect> : mr == kMassDF ? k_split_init<kMassDF> : k_split_init<kMassDefectDF>;
-  kern<<<blocks, kThreads, 0, st>>>(m, dnx, dny, rows, P_dev, S_dev, dPf[0], dPf[1], Sf[0], Sf[1], M1, M2,
+  kern<<<blocks, kThreads, 0, st>>>(m, px, dnx, dny, rows, P_dev, S_dev, dPf[0], dPf[1], Sf[0], Sf[1], M1, M2,
                                     (unsigned)c0, (unsigned)c1);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GBF_OK : gbf_cuda_check(e, "gbf_split_init_state");
@@ -537,7 +573,7 @@ int gbf_split_upload(gbf_domain* d, const double* P1, const double* S2, cudaMemc
     S = tmp + n;
   }
   d->cur = 0;
-  if (int e = gbf_split_init_state(d->m, d->split_rows, P, S, d->Pf, d->Sf, d->M1, d->M2, gbf_mass_rep(d->precision), 0,
+  if (int e = gbf_split_init_state(d->m, d->px, d->split_rows, P, S, d->Pf, d->Sf, d->M1, d->M2, gbf_mass_rep(d->precision), 0,
                                    n, d->stream))
     return e;
   if (tmp) GBF_CUDA(cudaFreeAsync(tmp, d->stream));
@@ -551,9 +587,11 @@ int gbf_split_step(gbf_domain* d) {
   G.S = d->Sf[d->cur];
   G.dPn = d->Pf[nxt];
   G.Sn = d->Sf[nxt];
-  G.K = d->cells.K;
-  G.phi = d->cells.phi;
-  G.media = d->cells.media;
+  if (d->borrowed)  // the caller's media array: read as it is now
+    if (int e = gbf_split_pitch_media(d)) return e;
+  G.K = d->split_cells.K;
+  G.phi = d->split_cells.phi;
+  G.media = d->split_cells.media;
   G.M1 = d->M1;
   G.M2 = d->M2;
   G.mass_partials = nullptr;
@@ -567,9 +605,10 @@ int gbf_split_step(gbf_domain* d) {
     if ((d->out_flags & GBF_OUT_CFL) && d->cfl_hist) G.cfl_out = d->cfl_hist + 2 * d->mass_count;
     d->mass_count++;
   }
-  const GbfSplitConsts C = gbf_split_consts(d->m);
+  const GbfSplitConsts C = gbf_split_consts(d->m, d->px);
   int s = gbf_split_launch_domain(d->m, C, G, gbf_mass_rep(d->precision), mass_out, d->stream, &d->timer,
-                                  (const GbfTmaSet*)d->tma, d->cur, d->defect_k1v);
+                                  (const GbfTmaSet*)d->tma, d->cur, d->defect_k1v,
+                                  {d->split_plan[0], d->split_plan[1], d->split_plan[2]});
   if (s) return s;
   d->cur = nxt;
   d->steps++;
@@ -583,7 +622,7 @@ int gbf_split_download(gbf_domain* d, int field, double* host) {
   double* tmp = (double*)gbf_mapped_host(host);  // page-locked: written in place
   const bool staged = tmp == nullptr;
   if (staged) GBF_CUDA(cudaMallocAsync((void**)&tmp, b, d->stream));
-  if (int e = gbf_split_state_to_f64(d->m, d->split_rows, d->Pf[d->cur], d->Sf[d->cur],
+  if (int e = gbf_split_state_to_f64(d->m, d->px, d->split_rows, d->Pf[d->cur], d->Sf[d->cur],
                                      field == GBF_FIELD_P1 ? tmp : nullptr, field == GBF_FIELD_S2 ? tmp : nullptr, 0, n,
                                      d->stream))
     return e;
@@ -595,11 +634,12 @@ int gbf_split_download(gbf_domain* d, int field, double* host) {
   return GBF_OK;
 }
 
-int gbf_split_state_to_f64(const gbf_model& m, const GbfRowConst* rows, const float* dPf, const float* Sf, double* P,
+int gbf_split_state_to_f64(const gbf_model& m, int px, const GbfRowConst* rows, const float* dPf, const float* Sf, double* P,
                            double* S, size_t c0, size_t c1, cudaStream_t st) {
   const unsigned blocks = (unsigned)((c1 - c0 + kConvCells - 1) / kConvCells);
-  k_split_to_f64<<<blocks, kThreads, 0, st>>>(gbf_fast_div((unsigned)m.nx), gbf_fast_div((unsigned)m.ny), rows, dPf, Sf,
-                                              P, S, (unsigned)c0, (unsigned)c1);
+  k_split_to_f64<<<blocks, kThreads, 0, st>>>((unsigned)(px - m.nx), gbf_fast_div((unsigned)m.nx),
+                                              gbf_fast_div((unsigned)m.ny), rows, dPf, Sf, P, S, (unsigned)c0,
+                                              (unsigned)c1);
   GBF_CUDA(cudaGetLastError());
   return GBF_OK;
 }
@@ -618,7 +658,7 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
   const GbfGeo g = gbf_geo(m);
   const size_t n = g.n, pl = g.pl;
   const int mr = gbf_mass_rep(d->precision);
-  const GbfSplitConsts C = gbf_split_consts(m);
+  const GbfSplitConsts C = gbf_split_consts(m, d->px);
   const GbfTmaSet* maps = (const GbfTmaSet*)d->tma;
   const int kp = pipe_kchunk(C), ns = (C.nz - 2 + kp - 1) / kp;  // slabs = k chunks
   auto pa = [&](int q) { return q == 0 ? 0 : 1 + q * kp; };
@@ -656,9 +696,9 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
   G.S = d->Sf[0];
   G.dPn = d->Pf[1];
   G.Sn = d->Sf[1];
-  G.K = d->cells.K;
-  G.phi = d->cells.phi;
-  G.media = d->cells.media;
+  G.K = d->split_cells.K;
+  G.phi = d->split_cells.phi;
+  G.media = d->split_cells.media;
   G.M1 = d->M1;
   G.M2 = d->M2;
   G.mass_partials = nullptr;
@@ -672,22 +712,23 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
     if ((d->out_flags & GBF_OUT_CFL) && d->cfl_hist) G.cfl_out = d->cfl_hist;
     d->mass_count = 1;
   }
-  const long long tiles = layer_tiles(C, maps);
+  const int shape = G.cfl_out ? kPair64x8 : d->split_plan[0];
+  const long long tiles = layer_tiles(C, shape, maps);
   const size_t nb = maps ? gbf_boundary_count_no_xfaces(g) : gbf_boundary_count(g);
   for (int q = 0; q <= ns; q++) {
     if (q < ns) {  // slab q in: FP64 -> split state, both buffers
       const size_t c0 = (size_t)pa(q) * pl, c1 = (size_t)pb(q) * pl;
       GBF_CUDA(cudaStreamWaitEvent(cs, d->pipe_ev[2 + q], 0));
-      if (int e = gbf_split_init_state(m, d->split_rows, stP, stS, d->Pf, d->Sf, d->M1, d->M2, mr, c0, c1, cs)) return e;
+      if (int e = gbf_split_init_state(m, d->px, d->split_rows, stP, stS, d->Pf, d->Sf, d->M1, d->M2, mr, c0, c1, cs)) return e;
     }
     if (q > 0) {  // slab q - 1: its chunk layer of the step, its boundary cells, out
       const int r = q - 1;
       const size_t c0 = (size_t)pa(r) * pl, c1 = (size_t)pb(r) * pl;
       GbfSplitGrid Gr = G;
       if (Gr.mass_partials) Gr.mass_partials += 2 * (size_t)tiles * r;
-      if (int s = launch_chunks(C, Gr, mr, maps, 0, cs, kp, r, 1)) return s;
-      k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, cs>>>(m, G, C.H, nb, pa(r), pb(r));
-      if (int e = gbf_split_state_to_f64(m, d->split_rows, d->Pf[1], d->Sf[1], stP, stS, c0, c1, cs)) return e;
+      if (int s = launch_chunks(C, Gr, mr, shape, maps, 0, cs, kp, r, 1)) return s;
+      k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, cs>>>(m, C.px, G, C.H, nb, pa(r), pb(r));
+      if (int e = gbf_split_state_to_f64(m, d->px, d->split_rows, d->Pf[1], d->Sf[1], stP, stS, c0, c1, cs)) return e;
       GBF_CUDA(cudaGetLastError());
       GBF_CUDA(cudaEventRecord(d->pipe_ev[2 + ns + r], cs));
       GBF_CUDA(cudaStreamWaitEvent(d->pipe_out, d->pipe_ev[2 + ns + r], 0));

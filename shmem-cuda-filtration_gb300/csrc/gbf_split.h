@@ -8,6 +8,7 @@
 // the FP32 arithmetic; FP64 and FP32-pair copies for the wide residual.
 struct GbfSplitConsts {
   int nx, ny, nz;
+  int px;  // row pitch of the grid's arrays in cells (nx, or nx rounded up to 16 bytes: gbf_split_pitch)
   int noflow_bottom;  // GBF_BC_HYDROSTATIC_SIDES: no-flow bottom face and hydrostatic P on the i and k sides
   int ri0, rk0, rn;  // the source's cells on the j = 1 layer: the rate injection's or those under the Dirichlet patch (rn = 0: none)
   float H;  // rho01 g h2: hydrostatic pressure step per cell (main.cpp:114)
@@ -33,7 +34,8 @@ struct GbfSplitConsts {
   float2 m_df[2], dtsrc_m_df[2];
   double ro01b1_d, ro02b2_d;  // rho01 beta1, rho02 beta2 (the defect form's row densities)
 };
-GbfSplitConsts gbf_split_consts(const gbf_model& m);
+GbfSplitConsts gbf_split_consts(const gbf_model& m, int px);
+inline GbfSplitConsts gbf_split_consts(const gbf_model& m) { return gbf_split_consts(m, m.nx); }
 
 // The reference's Dirichlet patch (GBF_SOURCE_DIRICHLET_PATCH): top-face cells
 // i in [i0, i0 + n), k in [k0, k0 + n) that hold S2_gr and P_atm (cpu.cpp:346).
@@ -103,12 +105,12 @@ int gbf_split_launches_per_step(gbf_domain* d);
 // large enough for two slabs of about 1M cells: gbf_split_pipelined).
 int gbf_split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, double* P_out, double* S_out);
 bool gbf_split_pipelined(const gbf_model& m);
-// FP64 (P, S) of cells [c0, c1) from a split state (device arrays; either
-// output may be NULL).
-int gbf_split_state_to_f64(const gbf_model& m, const GbfRowConst* rows, const float* dPf, const float* Sf, double* P,
+// FP64 (P, S) of cells [c0, c1) from a split state of row pitch px (device
+// arrays; cells numbered without the padding; either output may be NULL).
+int gbf_split_state_to_f64(const gbf_model& m, int px, const GbfRowConst* rows, const float* dPf, const float* Sf, double* P,
                            double* S, size_t c0, size_t c1, cudaStream_t st);
 // FP32 state (both buffers) and masses of cells [c0, c1) of a grid from FP64 device arrays.
-int gbf_split_init_state(const gbf_model& m, const GbfRowConst* rows, const double* P_dev, const double* S_dev,
+int gbf_split_init_state(const gbf_model& m, int px, const GbfRowConst* rows, const double* P_dev, const double* S_dev,
                          float* const dPf[2], float* const Sf[2], double* M1, double* M2, int mr, size_t c0, size_t c1,
                          cudaStream_t st);
 // V sum over interior cells of c1(j) phi (the defect form's water mass of a
@@ -116,9 +118,19 @@ int gbf_split_init_state(const gbf_model& m, const GbfRowConst* rows, const doub
 // mass the tiles' sums leave out. Written to *k1v_host; 0 for other forms.
 int gbf_defect_k1(const gbf_model& m, const float* phi_dev, const int* media_dev, double* k1v_host,
                   cudaStream_t st);
+// The x-pair tile's shapes on single grids (cells in x by rows; 256 threads,
+// about equal halos each).
+enum { kPair64x8 = 0, kPair32x16, kPair16x32, kPairShapes };
+// How a grid's step is cut: the tile's shape (x-pair tiles) and the k planes
+// of a CTA; and, for steps with CFL numbers (64x8 only), those of that shape.
+struct GbfSplitPlan {
+  int shape, kchunk, kchunk_cfl;
+};
+GbfSplitPlan gbf_split_plan(const GbfSplitConsts& C, int mr, bool tma);
 struct GbfTmaSet;
-// `maps` (device memory; boxes of the x-pair tile) selects the x-pair TMA
-// tile for state buffer `buf`; without it the plain-load 32x8 tile runs.
+// `maps` (device memory; the 64x8 boxes, then those of the plan's shape)
+// selects the x-pair TMA tile for state buffer `buf`; without it the
+// plain-load 32x8 tile runs.
 int gbf_split_launch_domain(const gbf_model& m, const GbfSplitConsts& C, const GbfSplitGrid& G, int mr,
                             double* mass_out, cudaStream_t st, GbfTimer* tm, const GbfTmaSet* maps, int buf,
-                            double k1v);
+                            double k1v, const GbfSplitPlan& plan);

@@ -355,14 +355,15 @@ __device__ __forceinline__ float split_rcp(float x) {
 // Mobility x density of both phases at one cell (FP32): Brooks-Corey kr
 // (cpu.cpp:60-62) from one log2 and two exp2, Xi = -K kr / mu, densities at
 // P2 = P1 (cpu.cpp:63, 72-73).
+__device__ __forceinline__ float split_of(const float (&t)[2], int md) { return md ? t[1] : t[0]; }
 __device__ __forceinline__ void split_props(const GbfSplitConsts& C, int md, float K, float dP, float S, int j,
                                             float& L1, float& L2) {
   const float Pp = fmaf((float)j, C.H, dP);  // P - P_atm
-  const float Se = fmaf(S, C.se_b[md], 1.f);  // (1 - S - S_wr) / (1 - S_wr)
+  const float Se = fmaf(S, split_of(C.se_b, md), 1.f);  // (1 - S - S_wr) / (1 - S_wr)
   const float l2 = split_lg2(Se);
-  const float kr1 = split_ex2(C.e1[md] * l2);
+  const float kr1 = split_ex2(split_of(C.e1, md) * l2);
   const float om = 1.f - Se;
-  const float kr2 = om * om * (1.f - split_ex2(C.e2[md] * l2));
+  const float kr2 = om * om * (1.f - split_ex2(split_of(C.e2, md) * l2));
   L1 = K * kr1 * C.nmr1 * fmaf(C.beta1, Pp, 1.f);  // nmr = -rho0 / mu
   L2 = K * kr2 * C.nmr2 * fmaf(C.beta2, Pp, 1.f);
 }
@@ -382,9 +383,9 @@ __device__ __forceinline__ float split_face(float x, float Lminus, float Lplus) 
 
 // Brooks-Corey capillary pressure P_d S_e^(-1/lambda) and its S-derivative (cpu.cpp:303-308).
 __device__ __forceinline__ float split_Pk(const GbfSplitConsts& C, int md, float S, float& dPk_dS) {
-  const float Se = __fmaf_rn(S, C.se_b[md], 1.f);
-  const float Pk = __fmul_rn(C.P_d[md], split_ex2(__fmul_rn(C.m_inv_lam[md], split_lg2(Se))));
-  dPk_dS = __fmul_rn(__fmul_rn(Pk, C.inv_lam_1mswr[md]), split_rcp(Se));
+  const float Se = __fmaf_rn(S, split_of(C.se_b, md), 1.f);
+  const float Pk = __fmul_rn(split_of(C.P_d, md), split_ex2(__fmul_rn(split_of(C.m_inv_lam, md), split_lg2(Se))));
+  dPk_dS = __fmul_rn(__fmul_rn(Pk, split_of(C.inv_lam_1mswr, md)), split_rcp(Se));
   return Pk;
 }
 
@@ -559,7 +560,7 @@ template <int MR, int N, bool CFL = false, bool PATCH = false>
 __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCellIn (&in)[N],
                                             const typename MassRep<MR>::T (&M1)[N],
                                             const typename MassRep<MR>::T (&M2)[N], typename WideOf<MR>::T R01,
-                                            typename WideOf<MR>::T R02, const GbfDefectRow& rw, int md,
+                                            typename WideOf<MR>::T R02, const GbfDefectRow& rw, const int (&md)[N],
                                             unsigned rowf, int j, int k, bool phi_field, bool mass,
                                             const bool (&count)[N], GbfSplitAcc<MR>& acc, GbfCellOut<MR> (&o)[N],
                                             const float2* patch_in, int i0) {
@@ -570,6 +571,8 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
   constexpr bool DEF = gbf_is_defect(MR);
   const bool noflow = rowf & 1u;
   auto sp = [](float x) { return L::splat(x); };
+  // a media-table constant of each lane's cell
+  auto mt = [&](const float (&t)[2]) { return L::make([&](int n) { return split_of(t, md[n]); }); };
   // the upwinded face flux of split_face on lane vectors
   // upwind mobility of a face with potential x (split_face), and the face
   // flux as a paired product (FMA operands only) or exactly rounded
@@ -697,7 +700,7 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
 #pragma unroll
     for (int n = 0; n < N; n++) {
       const WT src = phi_field ? W::div_f(W::c(C.dtsrc_d, C.dtsrc_df), in[n].phi)
-                               : W::c(C.dtsrc_m_d[md], C.dtsrc_m_df[md]);
+                               : W::c(md[n] ? C.dtsrc_m_d[1] : C.dtsrc_m_d[0], md[n] ? C.dtsrc_m_df[1] : C.dtsrc_m_df[0]);
       if constexpr (DEF) {
         if (insrc[n]) {
           srcf[n] = src.hi;
@@ -726,14 +729,14 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
   // first (linear) iteration the residual is about rho0 beta |dp ds|; a
   // second iteration runs when that could move S by more than 1e-9.
   // Capillary pressure P_d S_e^(-1/lambda) and its S-derivative (split_Pk).
-  const F Se = vfma(S0, sp(C.se_b[md]), sp(1.f));
+  const F Se = vfma(S0, mt(C.se_b), sp(1.f));
   const F lSe = L::make([&](int n) { return split_lg2(L::get(Se, n)); });
-  const F exS = vmul(sp(C.m_inv_lam[md]), lSe);
+  const F exS = vmul(mt(C.m_inv_lam), lSe);
   const F eS = L::make([&](int n) { return split_ex2(L::get(exS, n)); });
-  const F Pk0 = vmul(sp(C.P_d[md]), eS);  // FMA operands only; its sums below are FMAs
+  const F Pk0 = vmul(mt(C.P_d), eS);  // FMA operands only; its sums below are FMAs
   const F rSe0 = L::make([&](int n) { return split_rcp(L::get(Se, n)); });
-  const F dPk0 = vmul(vmul(Pk0, sp(C.inv_lam_1mswr[md])), rSe0);
-  const F PpPk = vfma(sp(C.P_d[md]), eS, Pp);  // P' + P_k
+  const F dPk0 = vmul(vmul(Pk0, mt(C.inv_lam_1mswr)), rSe0);
+  const F PpPk = vfma(mt(C.P_d), eS, Pp);  // P' + P_k
   const F omS = vsub(sp(1.f), S0);
   F r1, r2;
   if constexpr (DEF) {
@@ -742,7 +745,7 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
     // - dm = + f / phi inside the FMA
     r1 = vfma(vneg(f), nrphi, vfma(vfma(sp(C.ro01b1), dPc, sp(rw.e1)), omS, vneg(D1)));
     r2 = vsub(vfma(vneg(gs), nrphi,
-                   vfma(vfma(sp(C.ro02b2), vfma(sp(C.P_d[md]), eS, dPc), sp(rw.e2)), S0, vneg(D2))),
+                   vfma(vfma(sp(C.ro02b2), vfma(mt(C.P_d), eS, dPc), sp(rw.e2)), S0, vneg(D2))),
               L::make([&](int n) { return srcf[n]; }));
   } else {
     r1 = L::make([&](int n) {
@@ -781,15 +784,15 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
 #pragma unroll
     for (int n = 0; n < N; n++) {
       // from the state the first step reached: its increments as applied
-      const float s0 = in[n].S0, pk0 = __fmul_rn(C.P_d[md], L::get(eS, n));
+      const float s0 = in[n].S0, pk0 = __fmul_rn(split_of(C.P_d, md[n]), L::get(eS, n));
       const float p = __fsub_rn(L::get(dPn, n), in[n].dPc), s = __fsub_rn(L::get(Sn, n), s0);
       // a0, b0 of this lane again (the same operations), not kept across the branch
       const float Ppn = __fmaf_rn((float)j, C.H, in[n].dPc);
       const float a = __fmaf_rn(C.beta1, Ppn, 1.f);
-      const float b = __fmaf_rn(C.beta2, __fmaf_rn(C.P_d[md], L::get(eS, n), Ppn), 1.f);
+      const float b = __fmaf_rn(C.beta2, __fmaf_rn(split_of(C.P_d, md[n]), L::get(eS, n), Ppn), 1.f);
       float dPk1;
       const float S1 = __fadd_rn(s0, s);
-      const float Pk1 = split_Pk(C, md, S1, dPk1);
+      const float Pk1 = split_Pk(C, md[n], S1, dPk1);
       const float dpk = __fadd_rn(p, __fsub_rn(Pk1, pk0));
       const float G1 =
           __fmaf_rn(C.ro01, __fmaf_rn(-a, s, __fmul_rn(__fmul_rn(C.beta1, p), __fsub_rn(1.f, S1))), L::get(r1, n));
@@ -837,10 +840,10 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
       e = vadd(vsub(a, vsub(s, bb)), vsub(b, bb));
     };
     const F S1 = Sn, p1 = dPn;
-    const F Se1 = vfma(S1, sp(C.se_b[md]), sp(1.f));
+    const F Se1 = vfma(S1, mt(C.se_b), sp(1.f));
     const F lS1 = L::make([&](int n) { return split_lg2(L::get(Se1, n)); });
-    const F ex1 = vmul(sp(C.m_inv_lam[md]), lS1);
-    const F Pk1 = vmul_exact(sp(C.P_d[md]), L::make([&](int n) { return split_ex2(L::get(ex1, n)); }));
+    const F ex1 = vmul(mt(C.m_inv_lam), lS1);
+    const F Pk1 = vmul_exact(mt(C.P_d), L::make([&](int n) { return split_ex2(L::get(ex1, n)); }));
     // targets: T' = D + t as (hi, err) beside D's low part
     const F ds1 = vsub(S1, S0);
     const F t1 = vfma(sp(rw.c1), ds1, dm1);
@@ -886,7 +889,7 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
     if (anyfresh) {
       const F rSe1 = L::make([&](int n) { return split_rcp(L::get(Se1, n)); });  // 1 / S_e(S1)
       const F Pp1 = vfma(sp((float)j), sp(C.H), p1);
-      const F dPkf = vmul(vmul(Pk1, sp(C.inv_lam_1mswr[md])), rSe1);
+      const F dPkf = vmul(vmul(Pk1, mt(C.inv_lam_1mswr)), rSe1);
       const F K11f = vmul(sp(C.ro01b1), Bh), mK12f = vmul(sp(C.ro01), vfma(sp(C.beta1), Pp1, sp(1.f)));
       const F K21f = vmul(sp(C.ro02b2), S1);
       const F K22f =
@@ -938,8 +941,8 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
         o[n].M2n = L::get(D2n, n);
       }
       if (mass) {  // phi T with T1 = c1 (1 - S) + D1, T2 = c2 S + D2 + q
-        const F ph = phi_field ? L::make([&](int n) { return in[n].phi; }) : sp(C.m_df[md].x);
-        const F pl = sp(phi_field ? 0.f : C.m_df[md].y);
+        const F ph = L::make([&](int n) { return phi_field ? in[n].phi : md[n] ? C.m_df[1].x : C.m_df[0].x; });
+        const F pl = L::make([&](int n) { return phi_field ? 0.f : md[n] ? C.m_df[1].y : C.m_df[0].y; });
         bool all = true;
 #pragma unroll
         for (int n = 0; n < N; n++) all = all && count[n];
@@ -958,8 +961,8 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
         o[n].M1n = defect_add(M1[n], L::get(i1, n));
         o[n].M2n = defect_add(M2[n], L::get(i2, n));
         if (count[n] && mass) {
-          const float ph = phi_field ? in[n].phi : C.m_df[md].x;
-          const float pl = phi_field ? 0.f : C.m_df[md].y;
+          const float ph = phi_field ? in[n].phi : md[n] ? C.m_df[1].x : C.m_df[0].x;
+          const float pl = phi_field ? 0.f : md[n] ? C.m_df[1].y : C.m_df[0].y;
           acc.add(ph, pl, o[n].Sn, o[n].M1n, o[n].M2n, __fmul_rn(L::get(qa, n), o[n].Sn), !phi_field);
         }
       }
@@ -975,7 +978,7 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
           acc.m1 = W::acc_phi(acc.m1, in[n].phi, T1[n]);
           acc.m2 = W::acc_phi(acc.m2, in[n].phi, T2[n]);
         } else {
-          const WT phw = W::c(C.m_d[md], C.m_df[md]);
+          const WT phw = W::c(md[n] ? C.m_d[1] : C.m_d[0], md[n] ? C.m_df[1] : C.m_df[0]);
           acc.m1 = W::add(acc.m1, W::mul(phw, T1[n]));
           acc.m2 = W::add(acc.m2, W::mul(phw, T2[n]));
         }
@@ -1043,7 +1046,7 @@ __device__ bool split_tile(const GbfSplitConsts& C, const GbfSplitGrid& G, int i
         rP[s] = __ldg(G.dP + c);
         rS[s] = __ldg(G.S + c);
         rM[s] = G.media ? __ldg(G.media + c) : 0;
-        rK[s] = G.K ? __ldg(G.K + c) : C.K[rM[s]];
+        rK[s] = G.K ? __ldg(G.K + c) : split_of(C.K, rM[s]);
       }
     }
   };
@@ -1146,7 +1149,7 @@ __device__ bool split_tile(const GbfSplitConsts& C, const GbfSplitGrid& G, int i
   if (active) {
     const unsigned c = (unsigned)(i + j * nx) + (unsigned)(k0 - 1) * pln;
     const int md = G.media ? G.media[c] : 0;
-    const float Kc = G.K ? G.K[c] : C.K[md];
+    const float Kc = G.K ? G.K[c] : split_of(C.K, md);
     dPm = G.dP[c];
     split_props(C, md, Kc, dPm, G.S[c], j, L1m, L2m);
   }
@@ -1205,7 +1208,7 @@ __device__ bool split_tile(const GbfSplitConsts& C, const GbfSplitGrid& G, int i
     if (active) {
       const unsigned c = (unsigned)(i + j * nx) + (unsigned)k * pln;
       const int md = (!TMA && G.media) ? __ldg(G.media + c) : 0;
-      const float phi = TMA ? raw->phi[sr][fi] : (G.phi ? __ldg(G.phi + c) : C.m[md]);
+      const float phi = TMA ? raw->phi[sr][fi] : (G.phi ? __ldg(G.phi + c) : split_of(C.m, md));
       const MT M1 = TMA ? MassRep<MR>::load(reinterpret_cast<const double*>(raw->m1[sr]), mi)
                         : MassRep<MR>::load(G.M1, c);
       const MT M2 = TMA ? MassRep<MR>::load(reinterpret_cast<const double*>(raw->m2[sr]), mi)
@@ -1222,8 +1225,9 @@ __device__ bool split_tile(const GbfSplitConsts& C, const GbfSplitGrid& G, int i
       const GbfCellIn ins[1] = {in};
       const MT m1s[1] = {M1}, m2s[1] = {M2};
       const bool cnt[1] = {true};
+      const int mds[1] = {md};
       GbfCellOut<MR> os[1];
-      split_cells<MR, 1, CFL, PATCH>(C, ins, m1s, m2s, R01, R02, rw, md, rowf, j, k, G.phi != nullptr,
+      split_cells<MR, 1, CFL, PATCH>(C, ins, m1s, m2s, R01, R02, rw, mds, rowf, j, k, G.phi != nullptr,
                                      G.mass_partials != nullptr, cnt, acc, os, G.patch_in, i);
       G.dPn[c] = os[0].dPn;
       G.Sn[c] = os[0].Sn;
@@ -1314,7 +1318,7 @@ __device__ __forceinline__ float gbf_split_sweep_dP(const gbf_model& m, const Gb
     }
     if (j == g.ny - 1) {
       // start-of-step water density at (i, 1, 0): P - P_atm = dP_old + H
-      const float pp = old[(size_t)i + (size_t)g.nx] + H;
+      const float pp = old[(size_t)i + (size_t)g.px] + H;
       add = (float)(m.ro01 * m.beta1 * m.g * m.h2) * pp;
       has_add = true;
       j = g.ny - 2;
@@ -1531,8 +1535,12 @@ template <> struct WidePair<kMassDefect> {  // FP32 defects: two floats
 // bounded waits and give-up as split_tile<..., TMA = true>; each cell is
 // updated by split_cell, so results equal the other tiles' bit for bit. The
 // CTA has NTB >= TXC / 2 * TY threads; the ones beyond the tile take part in
-// the barriers only.
-template <int MR, int TXC, int TY, bool CFL = false, int NTB = TXC / 2 * TY, bool PATCH = false>
+// the barriers only. TAB: a grid of the media table instead of K and porosity
+// fields; the halo box that holds K holds the cells' media indices (as they
+// are, 4 bytes), or nothing for a grid of one medium (G.media NULL), and the
+// interior rows have no porosity. Rows are C.px cells apart (whole 16-byte
+// units; the padding beyond nx is never read nor written).
+template <int MR, int TXC, int TY, bool CFL = false, int NTB = TXC / 2 * TY, bool PATCH = false, bool TAB = false>
 __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, int x0, int j0, int k0, int k1,
                               GbfPairBars<MR>& bars, GbfPairSmem<TXC, TY, MR>& sm, GbfSplitAcc<MR>& acc,
                               const GbfTmaSet* maps, int buf, unsigned* phases) {
@@ -1546,14 +1554,17 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
   constexpr int NPAIR = PCOLS * HY, SLOTS = (NPAIR + NT - 1) / NT;
   Ring& raw = sm.ring;
   const bool in_tile = NT == NTB || (int)threadIdx.x < NT;
-  const int nx = C.nx, ny = C.ny;
-  const unsigned pln = (unsigned)nx * (unsigned)ny;
+  const int nx = C.nx, ny = C.ny, px = C.px;
+  const unsigned pln = (unsigned)px * (unsigned)ny;
   const int tx = threadIdx.x % THX, ty = threadIdx.x / THX;
   const int ia = x0 + 2 * tx, j = j0 + ty;
   const bool row_ok = in_tile && j <= ny - 2;
   const bool act_a = row_ok && ia >= 1 && ia <= nx - 2;
   const bool act_b = row_ok && ia + 1 <= nx - 2;
   const bool any = row_ok && ia <= nx - 2;  // the pair lies in the grid's row (cell b at most nx - 1)
+  // nx odd: the face cell nx - 1 is beyond the last pair with an interior cell, which writes it
+  const bool odd_face = any && ia + 2 == nx - 1;
+  const bool has_media = TAB && G.media != nullptr;
   const int hc = (ty + 1) * BX + 2 * tx + 4;  // own pair in the plane buffers (even)
   const int mi = ty * TXC + 2 * tx;           // own pair in the rows boxes (even)
 
@@ -1592,19 +1603,19 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
   unsigned pend = 0;
   auto issue = [&](int p, int s) {  // halo planes of plane p into stage s
     if (threadIdx.x == 0) {
-      gbf_mbar_expect_tx(&bars.bar[s], Ring::kHaloBytes);
+      gbf_mbar_expect_tx(&bars.bar[s], !TAB || has_media ? Ring::kHaloBytes : Ring::kHaloBytes / 3u * 2u);
       gbf_tma_plane(raw.v[s][0], &maps->dP[buf], x0 - 4, j0 - 1, p, &bars.bar[s]);
       gbf_tma_plane(raw.v[s][1], &maps->S[buf], x0 - 4, j0 - 1, p, &bars.bar[s]);
-      gbf_tma_plane(raw.v[s][2], &maps->K, x0 - 4, j0 - 1, p, &bars.bar[s]);
+      if (!TAB || has_media) gbf_tma_plane(raw.v[s][2], &maps->K, x0 - 4, j0 - 1, p, &bars.bar[s]);
     }
     pend |= 1u << s;
   };
   auto issue_rows = [&](int p, int s) {  // M1, M2, phi rows of plane p into stage s
     if (threadIdx.x == 0) {
-      gbf_mbar_expect_tx(&bars.mbar[s], Ring::kRowsBytes);
+      gbf_mbar_expect_tx(&bars.mbar[s], TAB ? Ring::kRowsBytes - Ring::NR * 4u : Ring::kRowsBytes);
       gbf_tma_plane(raw.m1[s], &maps->M1, x0, j0, p, &bars.mbar[s]);
       gbf_tma_plane(raw.m2[s], &maps->M2, x0, j0, p, &bars.mbar[s]);
-      gbf_tma_plane(raw.phi[s], &maps->phi, x0, j0, p, &bars.mbar[s]);
+      if (!TAB) gbf_tma_plane(raw.phi[s], &maps->phi, x0, j0, p, &bars.mbar[s]);
     }
     pend |= 1u << (8 + s);
   };
@@ -1626,6 +1637,13 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
     if (threadIdx.x == 0) atomicOr(G.status, GBF_DEV_TIMEOUT);
   };
   float2 s_own = make_float2(0.f, 0.f);  // S of the own pair in the plane built last
+  int2 m_own = make_int2(0, 0);          // TAB: its media
+  // K and media of a pair from the value pair that stands for them
+  auto pair_K = [&](float2 kv, int2& md) -> float2 {
+    if constexpr (!TAB) return kv;
+    md = has_media ? make_int2(__float_as_int(kv.x), __float_as_int(kv.y)) : make_int2(0, 0);
+    return make_float2(split_of(C.K, md.x), split_of(C.K, md.y));
+  };
   auto build = [&](int s) {  // plane buffer s from halo stage s
 #pragma unroll
     for (int q = 0; q < SLOTS; q++) {
@@ -1633,14 +1651,17 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       // slots hold a pair for every thread too where the halo is large enough
       if (q == 0 ? in_tile : ((NT == NTB && (q + 1) * NT <= NPAIR) || hq[q] >= 0)) {
         const int e = q == 0 ? hc : hq[q], jr = q == 0 ? j : hj[q];
-        const float2 p = gbf_ld2(&raw.v[s][0][e]), sv = gbf_ld2(&raw.v[s][1][e]), kv = gbf_ld2(&raw.v[s][2][e]);
+        const float2 p = gbf_ld2(&raw.v[s][0][e]), sv = gbf_ld2(&raw.v[s][1][e]);
+        int2 md = make_int2(0, 0);
+        const float2 kv = pair_K(!TAB || has_media ? gbf_ld2(&raw.v[s][2][e]) : p, md);
         float l1a, l2a, l1b, l2b;
-        split_props(C, 0, kv.x, p.x, sv.x, jr, l1a, l2a);
-        split_props(C, 0, kv.y, p.y, sv.y, jr, l1b, l2b);
+        split_props(C, md.x, kv.x, p.x, sv.x, jr, l1a, l2a);
+        split_props(C, md.y, kv.y, p.y, sv.y, jr, l1b, l2b);
         gbf_st2(&sm.dP[s][e], p.x, p.y);
         gbf_st2(&sm.L1[s][e], l1a, l1b);
         gbf_st2(&sm.L2[s][e], l2a, l2b);
         if (q == 0) s_own = sv;
+        if (TAB && q == 0) m_own = md;
       }
     }
   };
@@ -1650,12 +1671,14 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
   for (int q = 0; q < RS && k0 + q < k1; q++) issue_rows(k0 + q, q);
   float dPma = 0.f, L1ma = 0.f, L2ma = 0.f, dPmb = 0.f, L1mb = 0.f, L2mb = 0.f;
   if (any) {
-    const unsigned c = (unsigned)(ia + j * nx) + (unsigned)(k0 - 1) * pln;
-    const float2 p = gbf_ld2(G.dP + c), sv = gbf_ld2(G.S + c), kv = gbf_ld2(G.K + c);
+    const unsigned c = (unsigned)(ia + j * px) + (unsigned)(k0 - 1) * pln;
+    const float2 p = gbf_ld2(G.dP + c), sv = gbf_ld2(G.S + c);
+    int2 md = make_int2(0, 0);
+    const float2 kv = pair_K(!TAB ? gbf_ld2(G.K + c) : has_media ? gbf_ld2(reinterpret_cast<const float*>(G.media) + c) : p, md);
     dPma = p.x;
     dPmb = p.y;
-    split_props(C, 0, kv.x, p.x, sv.x, j, L1ma, L2ma);
-    split_props(C, 0, kv.y, p.y, sv.y, j, L1mb, L2mb);
+    split_props(C, md.x, kv.x, p.x, sv.x, j, L1ma, L2ma);
+    split_props(C, md.y, kv.y, p.y, sv.y, j, L1mb, L2mb);
   }
   {
     const bool ok = wait_bit(0);
@@ -1685,6 +1708,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
   int u = 0;  // (k - k0) % 3: plane buffer, halo stage and rows stage of plane k
   for (int k = k0; k < k1; k++) {
     const float2 s0 = s_own;  // plane k's, before the build of plane k + 1 replaces it
+    const int mds[2] = {TAB ? m_own.x : 0, TAB ? m_own.y : 0};
     const int t_cur = u, t_next = u == 2 ? 0 : u + 1, t_rows = u;
     {
       const int sn = t_next;
@@ -1712,7 +1736,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       const float2 bu = gbf_ld2(P2 + hc - BX), bd = gbf_ld2(P2 + hc + BX);
       const float2 dp = gbf_ld2(sm.dP[t_next] + hc), ap = gbf_ld2(sm.L1[t_next] + hc),
                    bp = gbf_ld2(sm.L2[t_next] + hc);
-      const float2 ph = gbf_ld2(&raw.phi[t_rows][mi]);
+      const float2 ph = TAB ? make_float2(split_of(C.m, mds[0]), split_of(C.m, mds[1])) : gbf_ld2(&raw.phi[t_rows][mi]);
       MT M1a, M1b, M2a, M2b;
       WidePair<MR>::load(reinterpret_cast<const double*>(&raw.m1[t_rows][mi]), M1a, M1b);
       WidePair<MR>::load(reinterpret_cast<const double*>(&raw.m2[t_rows][mi]), M2a, M2b);
@@ -1736,7 +1760,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       const MT m1s[2] = {M1a, M1b}, m2s[2] = {M2a, M2b};
       const bool cnt[2] = {act_a, act_b};
       GbfCellOut<MR> o[2];
-      split_cells<MR, 2, CFL, PATCH>(C, in, m1s, m2s, R01, R02, rw, 0, rowf, j, k, true, G.mass_partials != nullptr,
+      split_cells<MR, 2, CFL, PATCH>(C, in, m1s, m2s, R01, R02, rw, mds, rowf, j, k, !TAB, G.mass_partials != nullptr,
                                      cnt, acc, o, G.patch_in, ia);
       // The x faces i = 0 and i = nx - 1 (rows and planes interior) take the
       // boundary rules' values here: the new S of the x-neighbour and its dP
@@ -1745,11 +1769,15 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       // the face pass skips them (gbf_boundary_count_no_xfaces, gbf_face_row).
       const GbfCellOut<MR> oa = act_a ? o[0] : GbfCellOut<MR>{hsides ? 0.f : o[1].dPn, o[1].Sn, M1a, M2a};
       const GbfCellOut<MR> ob = act_b ? o[1] : GbfCellOut<MR>{hsides ? 0.f : o[0].dPn, o[0].Sn, M1b, M2b};
-      const unsigned c = (unsigned)(ia + j * nx) + (unsigned)k * pln;  // even: nx and ia are
+      const unsigned c = (unsigned)(ia + j * px) + (unsigned)k * pln;  // even: px and ia are
       gbf_st2(G.dPn + c, oa.dPn, ob.dPn);
       gbf_st2(G.Sn + c, oa.Sn, ob.Sn);
       WidePair<MR>::store(mass_at<MR>(G.M1, c), oa.M1n, ob.M1n);
       WidePair<MR>::store(mass_at<MR>(G.M2, c), oa.M2n, ob.M2n);
+      if (odd_face) {
+        G.dPn[c + 2] = hsides ? 0.f : ob.dPn;
+        G.Sn[c + 2] = ob.Sn;
+      }
       fza1 = o[0].fz1; fza2 = o[0].fz2;
       fzb1 = o[1].fz1; fzb2 = o[1].fz2;
     }
@@ -1768,7 +1796,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
 __device__ __forceinline__ double split_patch_inflow(const GbfSplitConsts& C, const GbfPatchConsts& P,
                                                      const GbfSplitGrid& G, unsigned c, int md, int mdb, float dPb,
                                                      float dPc, float Sc, double phi) {
-  const unsigned b = c - (unsigned)C.nx;
+  const unsigned b = c - (unsigned)C.px;
   const double Ppc = C.H_d + (double)dPc;                   // P - P_atm at the cell (j = 1)
   const double rho2c = C.ro02_d * (1.0 + C.beta2_d * Ppc);  // the centre cell's density
   const double pot = ((double)dPb - (double)dPc) - C.H_d + rho2c * P.gh2;  // h2 times the potential
@@ -1794,8 +1822,8 @@ __device__ __forceinline__ void gbf_split_patch_cell(const GbfSplitConsts& C, co
                                                      const GbfSplitGrid& G, int t) {
   const int i = P.i0 + t % P.n, k = P.k0 + t / P.n;
   if (i < 1 || i > C.nx - 2 || k < 1 || k > C.nz - 2 || C.ny < 3) return;
-  const unsigned c = (unsigned)(i + C.nx) + (unsigned)k * (unsigned)C.nx * (unsigned)C.ny;  // j = 1
-  const unsigned b = c - (unsigned)C.nx;                                                     // the patch cell
+  const unsigned c = (unsigned)(i + C.px) + (unsigned)k * (unsigned)C.px * (unsigned)C.ny;  // j = 1
+  const unsigned b = c - (unsigned)C.px;                                                     // the patch cell
   const int md = G.media ? G.media[c] : 0, mdb = G.media ? G.media[b] : 0;
   const double phi = G.phi ? (double)G.phi[c] : C.m_d[md];
   G.patch_in[t] = gbf_df_from_double(split_patch_inflow(C, P, G, c, md, mdb, G.dP[b], G.dP[c], G.S[c], phi));
