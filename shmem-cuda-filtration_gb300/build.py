@@ -18,10 +18,11 @@ INCLUDE = PKG.parent / "include"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", str(INCLUDE), "-I", str(CSRC)]
 # Per-file extra flags. The one-kernel-per-function path rounds every
-# multiply and add separately like the CPU reference; so does the host field
+# multiply and add separately like the CPU reference (its host code too, which
+# forms its constants); so does the host field
 # generator (the same fields on x86 and Arm, and porosity bit-identical to
 # the device generator).
-EXTRA = {"gbf_eager.cu": ["-fmad=false"], "gbf_fields.cpp": ["-Xcompiler", "-ffp-contract=off"]}
+EXTRA = {"gbf_eager.cu": ["-fmad=false", "-Xcompiler", "-ffp-contract=off"], "gbf_fields.cpp": ["-Xcompiler", "-ffp-contract=off"]}
 SOURCES = ["gbf_host.cpp", "gbf_fields.cpp", "gbf_tma.cpp", "gbf_checkpoint.cpp", "gbf_plots.cpp", "gbf_defines.cpp", "gbf_fields_gpu.cu", "gbf_eager.cu", "gbf_f64.cu", "gbf_split.cu", "gbf_split_fields.cu", "gbf_split_fields_narrow.cu",
            "gbf_split_table.cu", "gbf_split_table_narrow.cu", "gbf_domain.cu", "gbf_dropin.cu",
            "gbf_ensemble.cu"]
