@@ -318,7 +318,7 @@ int gbf_domain_step(gbf_domain* d, int nsteps) {
 int gbf_domain_launches_per_step(gbf_domain* d) {
   if (!d) return 0;
   if (d->precision != GBF_PREC_F64) return gbf_split_launches_per_step(d);
-  return 3 + ((d->out_flags & GBF_OUT_MASS) ? 1 : 0);
+  return 3;
 }
 
 int gbf_domain_sync(gbf_domain* d) {

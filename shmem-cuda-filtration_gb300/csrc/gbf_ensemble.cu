@@ -8,8 +8,9 @@
 // memory. Plain FP64: the two passes of gbf_f64_pair.cuh (or, for models of
 // fewer than 7 Newton iterations, gbf_f64_cell.cuh) over packed chunk lists of
 // all members' cells. Then one face pass over all members'
-// boundary cells and one per-member phase-mass reduction. A step is a CUDA
-// graph (counter reset, step, faces, masses), captured once per buffer parity.
+// boundary cells, which also sums each member's phase masses and resets the
+// tile counter. A step is a CUDA graph (step, faces), captured once per buffer
+// parity.
 //
 // Tuning: the tile shape (one of the six compiled shapes of the enum below)
 // and the k-range per CTA ("fusion depth": planes marched per tile pass) per
@@ -69,8 +70,10 @@ const bool kShapePairs[kShapes] = {false, false, false, true, true, true};
 constexpr int kWideTX = 48, kWideTY = 10;
 bool mixed_wide_tail(int nx) { return nx >= 48 && nx % 32 > 0 && nx % 32 <= 16; }
 // Chunks of 4096 cells: with 16384, seven million cells are 440 blocks, less
-// than one wave of the FP64 passes (363 us against 226 for the flux pass).
-constexpr int kChunkCells = 4096, kBoundaryChunk = 4096, kThreads = 256;
+// than one wave of the FP64 passes (363 us against 226 for the flux pass). The
+// face passes of one boundary cell a thread take 512 each: 30 us with 4096
+// (FP64, four members of 1.7M cells), 12 us with 512.
+constexpr int kChunkCells = 4096, kBoundaryChunk = 512, kThreads = 256;
 
 // ------------------------------------------------------------ split kernels
 
@@ -278,8 +281,38 @@ __global__ void __launch_bounds__(256, gbf_pair_ctas(MR)) k_ens_split_step_x2m(
   }
 }
 
+// What the face pass does beside the faces, in blocks of its own after the
+// first `faces` ones: per member, the phase masses of this step from the
+// step kernel's partials, summed in a fixed order into hist[step][member][2]
+// (hist NULL: none; step from *count, which the last of them advances); and
+// block 0 zeroes the step kernel's tile counter for the next step.
+struct EnsTail {
+  unsigned faces;
+  const double* partials;
+  double* hist;
+  unsigned *count, *done;
+  int nmem, cap;
+  unsigned* tile_counter;
+};
+__device__ __forceinline__ bool ens_tail(const EnsMember* mem, const EnsTail& t) {
+  if (t.tile_counter && blockIdx.x == 0 && threadIdx.x == 0) *t.tile_counter = 0u;
+  if (blockIdx.x < t.faces) return false;
+  const unsigned r = blockIdx.x - t.faces, step = *t.count;
+  const EnsMember& me = mem[r];
+  __shared__ double skip[2];
+  const GbfMassTail tail = {t.partials + 2 * (size_t)me.part_begin, me.part_end - me.part_begin,
+                            step < (unsigned)t.cap ? t.hist + 2 * ((size_t)step * t.nmem + r) : skip, me.k1v};
+  gbf_mass_tail(tail);
+  if (threadIdx.x == 0 && atomicAdd(t.done, 1u) == (unsigned)t.nmem - 1u) {  // every block has read *count
+    *t.done = 0u;
+    *t.count = step + 1u;
+  }
+  return true;
+}
+
 __global__ void __launch_bounds__(kThreads) k_ens_split_boundary(const EnsMember* __restrict__ mem,
-                                                                 const EnsChunk* __restrict__ chunks, int cur) {
+                                                                 const EnsChunk* __restrict__ chunks, int cur, const EnsTail tail) {
+  if (ens_tail(mem, tail)) return;
   const EnsChunk ch = chunks[blockIdx.x];
   const EnsMember* me = mem + ch.member;
   const gbf_model& m = me->m;
@@ -301,7 +334,8 @@ __global__ void __launch_bounds__(kThreads) k_ens_split_boundary(const EnsMember
 // The face pass after the x-pair tiles: each block takes kThreads / 32 row
 // segments of one member (gbf_split_face_segment), one per warp.
 __global__ void __launch_bounds__(kThreads) k_ens_split_faces(const EnsMember* __restrict__ mem,
-                                                              const EnsChunk* __restrict__ chunks, int cur) {
+                                                              const EnsChunk* __restrict__ chunks, int cur, const EnsTail tail) {
+  if (ens_tail(mem, tail)) return;
   const EnsChunk ch = chunks[blockIdx.x];
   const unsigned w = ch.begin + (threadIdx.x >> 5);
   if (w >= ch.end) return;
@@ -366,7 +400,8 @@ __global__ void __launch_bounds__(kThreads) k_ens_f64_flux_newton(const EnsMembe
 }
 
 __global__ void __launch_bounds__(kThreads) k_ens_f64_boundary(const EnsMember* __restrict__ mem,
-                                                               const EnsChunk* __restrict__ chunks, int cur) {
+                                                               const EnsChunk* __restrict__ chunks, int cur, const EnsTail tail) {
+  if (ens_tail(mem, tail)) return;
   const EnsChunk ch = chunks[blockIdx.x];
   const EnsMember& me = mem[ch.member];
   const GbfGeo g = gbf_geo(me.m);
@@ -411,32 +446,6 @@ __global__ void k_ens_pair_rows(const EnsMember* __restrict__ mem) {
   GbfPairRow* rows = const_cast<GbfPairRow*>(me.pw.rows);
   for (int j = threadIdx.x; j < me.m.ny; j += blockDim.x) rows[j] = gbf_pair_row(me.m, j);
 }
-
-// Per-member phase masses of this step: one block per member sums its
-// partials in a fixed order into hist[step][member][2] (step from *count).
-__global__ void k_ens_mass_tail(const EnsMember* __restrict__ mem, const double* partials, double* hist,
-                                unsigned* count, int nmem, int cap) {
-  __shared__ double red[2][256];
-  const EnsMember& me = mem[blockIdx.x];
-  double a = 0., b = 0.;
-  for (int q = me.part_begin + threadIdx.x; q < me.part_end; q += blockDim.x) {
-    a += partials[2 * q];
-    b += partials[2 * q + 1];
-  }
-  red[0][threadIdx.x] = a;
-  red[1][threadIdx.x] = b;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) { red[0][threadIdx.x] += red[0][threadIdx.x + o]; red[1][threadIdx.x] += red[1][threadIdx.x + o]; }
-    __syncthreads();
-  }
-  const unsigned step = *count;
-  if (threadIdx.x == 0 && step < (unsigned)cap) {
-    hist[2 * ((size_t)step * nmem + blockIdx.x)] = red[0][0] + me.k1v;
-    hist[2 * ((size_t)step * nmem + blockIdx.x) + 1] = red[1][0];
-  }
-}
-__global__ void k_ens_count(unsigned* count) { atomicAdd(count, 1u); }
 
 // The step's pre-pass for split members under a Dirichlet patch
 // (gbf_split_patch_cell), one block per member of [r0, r0 + gridDim.x).
@@ -547,7 +556,7 @@ struct gbf_ensemble {
   GbfTmaSet* d_maps = nullptr;  // per-member TMA plane maps of the current tile shape (NULL: plain loads)
   int nparts = 0;
   double* d_partials = nullptr;
-  unsigned *d_counter = nullptr, *d_status = nullptr, *d_mass_count = nullptr;
+  unsigned *d_counter = nullptr, *d_status = nullptr, *d_mass_count = nullptr, *d_tail_done = nullptr;
   double* d_mass_hist = nullptr;
   float* d_cfl_hist = nullptr;  // [mass_cap][n][2] (GBF_OUT_CFL)
   int mass_cap = 0;
@@ -793,9 +802,8 @@ int launch_split_step_t(gbf_ensemble* e, double* partials, cudaStream_t st, cons
   GBF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TX * TY, 0));
   const int blocks = std::max(1, std::min(tr.nt, per_sm * gbf_num_sms()));
   e->persistent_blocks = blocks;
-  kern<<<blocks, TX * TY, 0, st>>>(e->d_mem, e->d_tiles + tr.t0, tr.order, tr.nt, tr.cur, tr.counter,
-                                    partials ? partials + 2 * (size_t)tr.t0 : nullptr, e->d_status, e->d_maps,
-                                    ens_cfl(e));
+  GBF_CUDA(gbf_launch(false, kern, (unsigned)blocks, TX * TY, 0, st, e->d_mem, e->d_tiles + tr.t0, tr.order, tr.nt, tr.cur,
+                      tr.counter, partials ? partials + 2 * (size_t)tr.t0 : nullptr, e->d_status, e->d_maps, ens_cfl(e)));
   return GBF_OK;
 }
 
@@ -810,9 +818,9 @@ int launch_split_step_x2(gbf_ensemble* e, double* partials, cudaStream_t st, con
   GBF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TXC / 2 * TY, bytes));
   const int blocks = std::max(1, std::min(tr.nt, std::max(1, per_sm) * gbf_num_sms()));
   e->persistent_blocks = blocks;
-  kern<<<blocks, TXC / 2 * TY, bytes, st>>>(e->d_mem, e->d_tiles + tr.t0, tr.order, tr.nt, tr.cur, tr.counter,
-                                             partials ? partials + 2 * (size_t)tr.t0 : nullptr, e->d_status,
-                                             e->d_maps, ens_cfl(e));
+  GBF_CUDA(gbf_launch(false, kern, (unsigned)blocks, TXC / 2 * TY, (size_t)bytes, st, e->d_mem, e->d_tiles + tr.t0, tr.order,
+                      tr.nt, tr.cur, tr.counter, partials ? partials + 2 * (size_t)tr.t0 : nullptr, e->d_status,
+                      e->d_maps, ens_cfl(e)));
   return GBF_OK;
 }
 
@@ -826,9 +834,9 @@ int launch_split_step_x2m(gbf_ensemble* e, double* partials, cudaStream_t st, co
   GBF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, bytes));
   const int blocks = std::max(1, std::min(tr.nt, std::max(1, per_sm) * gbf_num_sms()));
   e->persistent_blocks = blocks;
-  kern<<<blocks, 256, bytes, st>>>(e->d_mem, e->d_tiles + tr.t0, tr.order, tr.nt, tr.cur, tr.counter,
-                                   partials ? partials + 2 * (size_t)tr.t0 : nullptr, e->d_status, e->d_maps,
-                                   ens_cfl(e));
+  GBF_CUDA(gbf_launch(false, kern, (unsigned)blocks, 256, (size_t)bytes, st, e->d_mem, e->d_tiles + tr.t0, tr.order, tr.nt,
+                      tr.cur, tr.counter, partials ? partials + 2 * (size_t)tr.t0 : nullptr, e->d_status, e->d_maps,
+                      ens_cfl(e)));
   return GBF_OK;
 }
 
@@ -861,51 +869,51 @@ int launch_split_step(gbf_ensemble* e, double* partials, cudaStream_t st, const 
 
 // Enqueue one step on `st` (also used under stream capture).
 // The FP64 passes over chunks [p0, p0 + np) of the cells and [f0, f0 + nf) of the interior cells.
-void enqueue_f64(gbf_ensemble* e, int p0, int np, int f0, int nf, int cur, double* partials, cudaStream_t st,
-                 GbfTimer* tm) {
+int enqueue_f64(gbf_ensemble* e, int p0, int np, int f0, int nf, int cur, double* partials, cudaStream_t st,
+                GbfTimer* tm) {
   cudaEvent_t ev = gbf_timer_begin(tm, st);
-  if (e->pair) k_ens_pair_props<<<(unsigned)np, kThreads, 0, st>>>(e->d_mem, e->d_props + p0, cur);
-  else k_ens_f64_props<<<(unsigned)np, kThreads, 0, st>>>(e->d_mem, e->d_props + p0, cur);
+  GBF_CUDA(gbf_launch(false, e->pair ? k_ens_pair_props : k_ens_f64_props, (unsigned)np, kThreads, 0, st, e->d_mem,
+                      e->d_props + p0, cur));
   gbf_timer_end(tm, GBF_K_ENS_PROPS, ev, st);
   ev = gbf_timer_begin(tm, st);
-  if (!e->pair) k_ens_f64_flux_newton<<<(unsigned)nf, kThreads, 0, st>>>(e->d_mem, e->d_flux + f0, cur, partials, e->d_status);
-  else if (partials) k_ens_pair_step<true><<<(unsigned)nf, kThreads, 0, st>>>(e->d_mem, e->d_flux + f0, cur, partials, e->d_status);
-  else k_ens_pair_step<false><<<(unsigned)nf, kThreads, 0, st>>>(e->d_mem, e->d_flux + f0, cur, nullptr, e->d_status);
+  GBF_CUDA(gbf_launch(false, !e->pair ? k_ens_f64_flux_newton : partials ? k_ens_pair_step<true> : k_ens_pair_step<false>,
+                      (unsigned)nf, kThreads, 0, st, e->d_mem, e->d_flux + f0, cur, partials, e->d_status));
   gbf_timer_end(tm, GBF_K_ENS_FLUX_NEWTON, ev, st);
+  return GBF_OK;
+}
+// The face pass over chunks [b0, b0 + nb); mass: with the whole ensemble's phase masses.
+int enqueue_faces(gbf_ensemble* e, int b0, int nb, int cur, bool mass, unsigned* tile_counter, cudaStream_t st) {
+  const EnsTail tail = {(unsigned)nb, e->d_partials, mass ? e->d_mass_hist : nullptr, e->d_mass_count, e->d_tail_done,
+                        e->n, e->mass_cap, tile_counter};
+  auto kern = e->precision == GBF_PREC_F64 ? k_ens_f64_boundary : kShapePairs[e->shape] ? k_ens_split_faces : k_ens_split_boundary;
+  GBF_CUDA(gbf_launch(false, kern, (unsigned)(nb + (mass ? e->n : 0)), kThreads, 0, st, e->d_mem, e->d_bnd + b0, cur, tail));
+  return GBF_OK;
 }
 
+// Enqueue one step on `st` (also used under stream capture). The tile counter
+// is zero before: from the creation, or by the last step's face pass.
 int enqueue_step(gbf_ensemble* e, cudaStream_t st) {
-  const bool mass = (e->out_flags & GBF_OUT_MASS) && e->d_mass_hist;
+  const bool mass = (e->out_flags & GBF_OUT_MASS) && e->d_mass_hist, split = e->precision != GBF_PREC_F64;
   double* partials = mass ? e->d_partials : nullptr;
   GbfTimer* tm = &e->timer;
   cudaEvent_t ev;
-  if (e->precision != GBF_PREC_F64) {
-    GBF_CUDA(cudaMemsetAsync(e->d_counter, 0, sizeof(unsigned), st));
+  if (split) {
     ev = gbf_timer_begin(tm, st);
-    if (e->any_patch) k_ens_split_patch<<<e->n, 64, 0, st>>>(e->d_mem, 0, e->cur);  // timed with the step
+    if (e->any_patch)  // timed with the step
+      GBF_CUDA(gbf_launch(false, k_ens_split_patch, (unsigned)e->n, 64, 0, st, e->d_mem, 0, e->cur));
     if (int s = launch_split_step(e, partials, st, {0, (int)e->tiles.size(), e->cur, e->d_counter, e->d_order}))
       return s;
     gbf_timer_end(tm, GBF_K_ENS_STEP, ev, st);
-    ev = gbf_timer_begin(tm, st);
-    if (kShapePairs[e->shape])
-      k_ens_split_faces<<<(unsigned)e->bnd.size(), kThreads, 0, st>>>(e->d_mem, e->d_bnd, e->cur);
-    else
-      k_ens_split_boundary<<<(unsigned)e->bnd.size(), kThreads, 0, st>>>(e->d_mem, e->d_bnd, e->cur);
-    gbf_timer_end(tm, GBF_K_ENS_BOUNDARY, ev, st);
-  } else {
-    enqueue_f64(e, 0, (int)e->props.size(), 0, (int)e->flux.size(), e->cur, partials, st, tm);
-    ev = gbf_timer_begin(tm, st);
-    k_ens_f64_boundary<<<(unsigned)e->bnd.size(), kThreads, 0, st>>>(e->d_mem, e->d_bnd, e->cur);
-    gbf_timer_end(tm, GBF_K_ENS_BOUNDARY, ev, st);
+  } else if (int s = enqueue_f64(e, 0, (int)e->props.size(), 0, (int)e->flux.size(), e->cur, partials, st, tm)) {
+    return s;
   }
-  if (mass) {
-    ev = gbf_timer_begin(tm, st);
-    k_ens_mass_tail<<<e->n, 256, 0, st>>>(e->d_mem, e->d_partials, e->d_mass_hist, e->d_mass_count, e->n, e->mass_cap);
-    k_ens_count<<<1, 1, 0, st>>>(e->d_mass_count);
-    gbf_timer_end(tm, GBF_K_MASS_TAIL, ev, st);
+  ev = gbf_timer_begin(tm, st);
+  if (int s = enqueue_faces(e, 0, (int)e->bnd.size(), e->cur, mass, split ? e->d_counter : nullptr, st)) {
+    if (split) cudaMemsetAsync(e->d_counter, 0, sizeof(unsigned), st);
+    return s;
   }
-  cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? GBF_OK : gbf_cuda_check(err, "gbf_ensemble step");
+  gbf_timer_end(tm, GBF_K_ENS_BOUNDARY, ev, st);
+  return GBF_OK;
 }
 
 int capture_graph(gbf_ensemble* e, int parity) {
@@ -944,18 +952,12 @@ int enqueue_group_step(gbf_ensemble* e, int r0, int r1, int cur, unsigned* count
   const auto &a = e->starts[r0], &b = e->starts[r1];
   if (e->precision != GBF_PREC_F64) {
     GBF_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), st));
-    if (e->any_patch) k_ens_split_patch<<<r1 - r0, 64, 0, st>>>(e->d_mem, r0, cur);
+    if (e->any_patch) GBF_CUDA(gbf_launch(false, k_ens_split_patch, (unsigned)(r1 - r0), 64, 0, st, e->d_mem, r0, cur));
     if (int s = launch_split_step(e, nullptr, st, {a.tiles, b.tiles - a.tiles, cur, counter, nullptr})) return s;
-    if (kShapePairs[e->shape])
-      k_ens_split_faces<<<(unsigned)(b.bnd - a.bnd), kThreads, 0, st>>>(e->d_mem, e->d_bnd + a.bnd, cur);
-    else
-      k_ens_split_boundary<<<(unsigned)(b.bnd - a.bnd), kThreads, 0, st>>>(e->d_mem, e->d_bnd + a.bnd, cur);
-  } else {
-    enqueue_f64(e, a.props, b.props - a.props, a.flux, b.flux - a.flux, cur, nullptr, st, nullptr);
-    k_ens_f64_boundary<<<(unsigned)(b.bnd - a.bnd), kThreads, 0, st>>>(e->d_mem, e->d_bnd + a.bnd, cur);
+  } else if (int s = enqueue_f64(e, a.props, b.props - a.props, a.flux, b.flux - a.flux, cur, nullptr, st, nullptr)) {
+    return s;
   }
-  cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? GBF_OK : gbf_cuda_check(err, "gbf_ensemble group step");
+  return enqueue_faces(e, a.bnd, b.bnd - a.bnd, cur, false, nullptr, st);
 }
 
 // Member groups of the host-resident pipeline: contiguous ranges, at least
@@ -1081,9 +1083,12 @@ int gbf_ensemble_create(int n, const gbf_model* models, const gbf_cells* host_ce
   if (!s) s |= ens_alloc(e, (void**)&e->d_counter, sizeof(unsigned));
   if (!s) s |= ens_alloc(e, (void**)&e->d_status, sizeof(unsigned));
   if (!s) s |= ens_alloc(e, (void**)&e->d_mass_count, sizeof(unsigned));
+  if (!s) s |= ens_alloc(e, (void**)&e->d_tail_done, sizeof(unsigned));
   if (!s) {
+    cudaMemset(e->d_counter, 0, sizeof(unsigned));
     cudaMemset(e->d_status, 0, sizeof(unsigned));
     cudaMemset(e->d_mass_count, 0, sizeof(unsigned));
+    cudaMemset(e->d_tail_done, 0, sizeof(unsigned));
     s = build_lists(e);
   }
   if (!s && e->precision != GBF_PREC_F64) {  // the members' row-constant tables, once
@@ -1387,8 +1392,7 @@ int gbf_ensemble_kernel_times(gbf_ensemble* e, double* ms, int* launches, int nk
 
 int gbf_ensemble_launches_per_step(gbf_ensemble* e) {
   if (!e) return 0;
-  const int mass = (e->out_flags & GBF_OUT_MASS) ? 2 : 0;
-  return (e->precision == GBF_PREC_F64 ? 3 : 2 + (e->any_patch ? 1 : 0)) + mass;
+  return e->precision == GBF_PREC_F64 ? 3 : 2 + (e->any_patch ? 1 : 0);
 }
 
 int gbf_ensemble_set_tuning(gbf_ensemble* e, int shape, int edge, int kchunk) {

@@ -34,6 +34,7 @@ constexpr int kThreads = 256;
 
 __global__ void __launch_bounds__(kThreads) k_f64_props(const gbf_model m, const GbfDerived d, const gbf_cells cells,
                                                         const GbfF64Step s, const int flags) {
+  gbf_pdl_begin();
   const GbfGeo g = gbf_geo(m);
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < g.n; c += (size_t)gridDim.x * blockDim.x)
     gbf_f64_props_cell(m, d, cells, s, flags, g, c);
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(kThreads) k_f64_props(const gbf_model m, const
 
 __global__ void __launch_bounds__(kThreads) k_f64_flux_newton(const gbf_model m, const GbfDerived d,
                                                               const gbf_cells cells, const GbfF64Step s) {
+  gbf_pdl_begin();
   const GbfGeo g = gbf_geo(m);
   const size_t ix = (size_t)g.nx - 2, iy = (size_t)g.ny - 2;
   const size_t nint = ix * iy * (size_t)(g.nz - 2);
@@ -57,13 +59,15 @@ __global__ void __launch_bounds__(kThreads) k_f64_flux_newton(const gbf_model m,
 template <bool DROPIN>
 __global__ void __launch_bounds__(kThreads) k_pair_props(const GbfPairConsts C, const gbf_cells cells,
                                                          const GbfF64Step s, const GbfPairWork w) {
+  gbf_pdl_begin();
   for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < C.n; c += gridDim.x * blockDim.x)
     gbf_pair_props_cell<DROPIN>(C, cells, s, w, c);
 }
 
-template <bool MASS>
-__global__ void __launch_bounds__(kThreads, 4) k_pair_step(const GbfPairConsts C, const gbf_cells cells,
-                                                        const GbfF64Step s, const GbfPairWork w, double V) {
+template <bool MASS, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_pair_step(const GbfPairConsts C, const gbf_cells cells,
+                                                          const GbfF64Step s, const GbfPairWork w, double V) {
+  gbf_pdl_begin();
   GbfPairMass acc;
   unsigned bad = 0;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < C.nint; t += gridDim.x * blockDim.x) {
@@ -72,7 +76,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_pair_step(const GbfPairConsts C
     gbf_pair_step_cell<MASS>(C, cells, s, w, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc, bad);
   }
   if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
-  if (MASS) gbf_block_sum2<kThreads>(acc.m1 - pf_to_double(acc.r1), acc.m2, V, s.mass_partials + 2 * blockIdx.x);
+  if (MASS) gbf_block_sum2<NT>(acc.m1 - pf_to_double(acc.r1), acc.m2, V, s.mass_partials + 2 * blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kThreads) k_density(double ro0, double beta, double Patm, const double* P,
@@ -85,33 +89,33 @@ __global__ void k_pair_rows(const gbf_model m, GbfPairRow* rows) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m.ny; j += gridDim.x * blockDim.x) rows[j] = gbf_pair_row(m, j);
 }
 
-__global__ void __launch_bounds__(kThreads) k_f64_boundary(const gbf_model m, const GbfF64Step s) {
+__global__ void __launch_bounds__(kThreads) k_f64_boundary(const gbf_model m, const GbfF64Step s, const GbfMassTail tail) {
+  gbf_pdl_begin();
+  unsigned blocks = gridDim.x;
+  if (tail.out && blockIdx.x == --blocks) {
+    gbf_mass_tail(tail);
+    return;
+  }
   const GbfGeo g = gbf_geo(m);
   const size_t nb = gbf_boundary_count(g);
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb; t += (size_t)gridDim.x * blockDim.x)
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb; t += (size_t)blocks * blockDim.x)
     gbf_f64_boundary_cell(m, s, g, t);
 }
 
 }  // namespace
 
-// Sum per-block partial pairs [2q, 2q+1] in a fixed order (one block of 256).
-__global__ void gbf_k_mass_tail(const double* partials, int nblocks, double* out) {
-  __shared__ double red[2][256];
-  double a = 0., b = 0.;
-  for (int q = threadIdx.x; q < nblocks; q += blockDim.x) { a += partials[2 * q]; b += partials[2 * q + 1]; }
-  red[0][threadIdx.x] = a;
-  red[1][threadIdx.x] = b;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) { red[0][threadIdx.x] += red[0][threadIdx.x + o]; red[1][threadIdx.x] += red[1][threadIdx.x + o]; }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { out[0] = red[0][0]; out[1] = red[1][0]; }
-}
+namespace {
+// Block size of the pair step's passes over n cells: 64 where 256 would leave
+// less than a few blocks an SM. Time of a step with 256, 128, 64, 32 threads:
+// 40^3 17.3, 15.9, 15.1, 14.8 us; 64^3 25.5, 23.8, 23.4, 26.4 us.
+unsigned pair_threads(size_t n) { return n < (size_t)gbf_num_sms() * 2048 ? 64u : (unsigned)kThreads; }
+}  // namespace
 
+// Blocks of the flux pass: one wave (its per-block mass partials).
 unsigned gbf_f64_flux_grid(const gbf_model& m) {
-  size_t nint = (size_t)(m.nx - 2) * (m.ny - 2) * (m.nz - 2);
-  return gbf_grid_for(nint, kThreads, 4);
+  const size_t nint = (size_t)(m.nx - 2) * (m.ny - 2) * (m.nz - 2);
+  const unsigned t = gbf_pair_applies(m) ? pair_threads(gbf_geo(m).n) : (unsigned)kThreads;
+  return gbf_grid_for(nint, (int)t, 1024 / (int)t);
 }
 
 GbfPairConsts gbf_pair_consts(const gbf_model& m) {
@@ -196,36 +200,42 @@ int gbf_f64_launch_step(const gbf_model& m, const GbfDerived& d, const gbf_cells
   const GbfGeo g = gbf_geo(m);
   const unsigned fg = gbf_f64_flux_grid(m);
   const bool mass = s.mass_partials && mass_out;
+  cudaError_t err = cudaSuccess;
+  // programmatic launches up to 4M cells (256^3: 613 us a step without, 619 with)
+  const bool pdl = g.n < (4u << 20);
+  unsigned threads = kThreads;
+  auto go = [&](auto kern, unsigned blocks, auto... args) {
+    if (err == cudaSuccess) err = gbf_launch(pdl, kern, blocks, threads, 0, st, args...);
+  };
   cudaEvent_t e = gbf_timer_begin(tm, st);
   if (pair) {
-    const unsigned pg = gbf_grid_for(g.n, kThreads, 8);
-    if (pair->P_from) k_pair_props<true><<<pg, kThreads, 0, st>>>(*pc, cells, s, *pair);
-    else k_pair_props<false><<<pg, kThreads, 0, st>>>(*pc, cells, s, *pair);
+    threads = pair_threads(g.n);
+    const unsigned pg = gbf_grid_for(g.n, (int)threads, 2048 / (int)threads);
+    go(pair->P_from ? k_pair_props<true> : k_pair_props<false>, pg, *pc, cells, s, *pair);
     if (props_flags) {  // the outputs P2, Xi, u of the state the step starts from
       GbfF64Step o = s;
       o.L1 = nullptr;
-      k_f64_props<<<gbf_grid_for(g.n, kThreads, 4), kThreads, 0, st>>>(m, d, cells, o, props_flags);
+      threads = kThreads;
+      go(k_f64_props, gbf_grid_for(g.n, kThreads, 4), m, d, cells, o, props_flags);
     }
   } else {
-    k_f64_props<<<gbf_grid_for(g.n, kThreads, 4), kThreads, 0, st>>>(m, d, cells, s, props_flags);
+    go(k_f64_props, gbf_grid_for(g.n, kThreads, 4), m, d, cells, s, props_flags);
   }
   gbf_timer_end(tm, GBF_K_PROPS, e, st);
   e = gbf_timer_begin(tm, st);
   if (pair) {
-    if (mass) k_pair_step<true><<<fg, kThreads, 0, st>>>(*pc, cells, s, *pair, d.V);
-    else k_pair_step<false><<<fg, kThreads, 0, st>>>(*pc, cells, s, *pair, d.V);
+    threads = pair_threads(g.n);
+    go(threads == 64 ? (mass ? k_pair_step<true, 64> : k_pair_step<false, 64>)
+                     : (mass ? k_pair_step<true, kThreads> : k_pair_step<false, kThreads>),
+       fg, *pc, cells, s, *pair, d.V);
+    threads = kThreads;
   } else {
-    k_f64_flux_newton<<<fg, kThreads, 0, st>>>(m, d, cells, s);
+    go(k_f64_flux_newton, fg, m, d, cells, s);
   }
   gbf_timer_end(tm, GBF_K_FLUX_NEWTON, e, st);
   e = gbf_timer_begin(tm, st);
-  k_f64_boundary<<<gbf_grid_for(gbf_boundary_count(g), kThreads, 4), kThreads, 0, st>>>(m, s);
+  const GbfMassTail tail = {s.mass_partials, (int)fg, mass ? mass_out : nullptr, 0.0};
+  go(k_f64_boundary, gbf_grid_for(gbf_boundary_count(g), kThreads, 4) + (mass ? 1 : 0), m, s, tail);
   gbf_timer_end(tm, GBF_K_BOUNDARY, e, st);
-  if (mass) {
-    e = gbf_timer_begin(tm, st);
-    gbf_k_mass_tail<<<1, 256, 0, st>>>(s.mass_partials, (int)fg, mass_out);
-    gbf_timer_end(tm, GBF_K_MASS_TAIL, e, st);
-  }
-  cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? GBF_OK : gbf_cuda_check(err, "gbf_f64_launch_step");
 }

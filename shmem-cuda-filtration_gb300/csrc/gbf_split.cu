@@ -118,6 +118,7 @@ int tiles_y(const GbfSplitConsts& C) { return (C.ny - 2 + kSplitTY - 1) / kSplit
 template <int MR, bool CFL, bool PATCH>
 __global__ void __launch_bounds__(kSplitThreads, 4) k_split_step(const GbfSplitConsts C, const GbfSplitGrid G,
                                                               const int kchunk, const int kc0) {
+  gbf_pdl_begin();
   __shared__ GbfSplitPlane pl[2];
   const int ntx = (C.nx - 2 + kSplitTX - 1) / kSplitTX, nty = (C.ny - 2 + kSplitTY - 1) / kSplitTY;
   const int b = blockIdx.x;
@@ -134,9 +135,15 @@ __global__ void __launch_bounds__(kSplitThreads, 4) k_split_step(const GbfSplitC
 // Boundary cells [0, nb) of gbf_boundary_cell's enumeration (all, or all but
 // the x faces that the x-pair tile writes).
 __global__ void __launch_bounds__(kThreads) k_split_boundary(const gbf_model m, int px, const GbfSplitGrid G, float H,
-                                                             size_t nb, int k_lo, int k_hi) {
+                                                             size_t nb, int k_lo, int k_hi, const GbfMassTail tail) {
+  gbf_pdl_begin();
+  unsigned blocks = gridDim.x;
+  if (tail.out && blockIdx.x == --blocks) {
+    gbf_mass_tail(tail);
+    return;
+  }
   const GbfGeo g = gbf_geo(m, px);
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb; t += (size_t)gridDim.x * blockDim.x) {
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb; t += (size_t)blocks * blockDim.x) {
     int i, j, k;
     gbf_boundary_cell(g, t, i, j, k);
     if (k < k_lo || k >= k_hi) continue;  // planes [k_lo, k_hi) only (a slab of the host pipeline)
@@ -172,20 +179,6 @@ __global__ void k_defect_k1_sum(const double* rows, int nrows, double V, double*
     for (int q = 0; q < nrows; q++) a += rows[q];
     *out = a * V;
   }
-}
-
-__global__ void k_split_mass_tail(const double* partials, int nblocks, double* out, double k1v) {
-  __shared__ double red[2][256];
-  double a = 0., b = 0.;
-  for (int q = threadIdx.x; q < nblocks; q += blockDim.x) { a += partials[2 * q]; b += partials[2 * q + 1]; }
-  red[0][threadIdx.x] = a;
-  red[1][threadIdx.x] = b;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) { red[0][threadIdx.x] += red[0][threadIdx.x + o]; red[1][threadIdx.x] += red[1][threadIdx.x + o]; }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { out[0] = red[0][0] + k1v; out[1] = red[1][0]; }
 }
 
 // The state conversions of cells [c0, c1): each block kConvCells consecutive
@@ -326,6 +319,7 @@ namespace {
 // The Dirichlet patch's pre-pass, one thread per patch cell (gbf_split_patch_cell).
 __global__ void __launch_bounds__(kThreads) k_split_patch(const GbfSplitConsts C, const GbfPatchConsts P,
                                                           const GbfSplitGrid G) {
+  gbf_pdl_begin();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < P.n * P.n; t += gridDim.x * blockDim.x)
     gbf_split_patch_cell(C, P, G, t);
 }
@@ -334,8 +328,8 @@ __global__ void __launch_bounds__(kThreads) k_split_patch(const GbfSplitConsts C
 template <int MR, bool PATCH>
 int launch_plain(const GbfSplitConsts& C, const GbfSplitGrid& G, cudaStream_t st, int kchunk, int kc0, int nkc) {
   const unsigned blocks = (unsigned)(tiles_x(C) * tiles_y(C) * nkc);
-  if (G.cfl_out) k_split_step<MR, true, PATCH><<<blocks, kSplitThreads, 0, st>>>(C, G, kchunk, kc0);
-  else k_split_step<MR, false, PATCH><<<blocks, kSplitThreads, 0, st>>>(C, G, kchunk, kc0);
+  GBF_CUDA(gbf_launch(true, G.cfl_out ? k_split_step<MR, true, PATCH> : k_split_step<MR, false, PATCH>, blocks, kSplitThreads, 0,
+                      st, C, G, kchunk, kc0));
   return GBF_OK;
 }
 
@@ -372,7 +366,7 @@ int gbf_split_launch_domain(const gbf_model& m, const GbfSplitConsts& C, const G
   cudaEvent_t e = gbf_timer_begin(tm, st);
   if (G.patch_in) {  // the Dirichlet patch's FP64 inflow, timed with the step kernel
     const GbfPatchConsts P = gbf_patch_consts(m);
-    k_split_patch<<<gbf_grid_for((size_t)P.n * P.n, kThreads), kThreads, 0, st>>>(C, P, G);
+    GBF_CUDA(gbf_launch(true, k_split_patch, gbf_grid_for((size_t)P.n * P.n, kThreads), kThreads, 0, st, C, P, G));
   }
   // TMA staging (maps): the x-pair tile; else the plain-load tile
   if (int s = launch_chunks(C, G, mr, shape, maps, buf, st, kchunk, 0, nkc)) return s;
@@ -381,13 +375,11 @@ int gbf_split_launch_domain(const gbf_model& m, const GbfSplitConsts& C, const G
   // one cell per thread (row segments, as the ensembles' face pass walks
   // them, measured 8.6 -> 10.4 us on 256^3: too few warps for a latency-bound pass)
   const size_t nb = maps ? gbf_boundary_count_no_xfaces(gbf_geo(m)) : gbf_boundary_count(gbf_geo(m));
-  k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, st>>>(m, C.px, G, C.H, nb, 0, C.nz);
+  const bool mass = G.mass_partials && mass_out;
+  const GbfMassTail tail = {G.mass_partials, (int)blocks, mass ? mass_out : nullptr, gbf_is_defect(mr) ? k1v : 0.0};
+  GBF_CUDA(gbf_launch(true, k_split_boundary, gbf_grid_for(nb, kThreads, 4) + (mass ? 1 : 0), kThreads, 0, st, m, C.px, G, C.H, nb,
+                      0, C.nz, tail));
   gbf_timer_end(tm, GBF_K_SPLIT_BOUNDARY, e, st);
-  if (G.mass_partials && mass_out) {
-    e = gbf_timer_begin(tm, st);
-    k_split_mass_tail<<<1, 256, 0, st>>>(G.mass_partials, (int)blocks, mass_out, gbf_is_defect(mr) ? k1v : 0.0);
-    gbf_timer_end(tm, GBF_K_MASS_TAIL, e, st);
-  }
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? GBF_OK : gbf_cuda_check(err, "gbf_split_launch_domain");
 }
@@ -727,7 +719,12 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
       GbfSplitGrid Gr = G;
       if (Gr.mass_partials) Gr.mass_partials += 2 * (size_t)tiles * r;
       if (int s = launch_chunks(C, Gr, mr, shape, maps, 0, cs, kp, r, 1)) return s;
-      k_split_boundary<<<gbf_grid_for(nb, kThreads, 4), kThreads, 0, cs>>>(m, C.px, G, C.H, nb, pa(r), pb(r));
+      // the last slab's pass also sums the masses of all (every slab's tiles precede it on the stream)
+      const bool sum = mass_out && q == ns;
+      const GbfMassTail tail = {G.mass_partials, (int)(tiles * ns), sum ? mass_out : nullptr,
+                                gbf_is_defect(mr) ? d->defect_k1v : 0.0};
+      GBF_CUDA(gbf_launch(true, k_split_boundary, gbf_grid_for(nb, kThreads, 4) + (sum ? 1 : 0), kThreads, 0, cs, m, C.px, G, C.H,
+                          nb, pa(r), pb(r), tail));
       if (int e = gbf_split_state_to_f64(m, d->px, d->split_rows, d->Pf[1], d->Sf[1], stP, stS, c0, c1, cs)) return e;
       GBF_CUDA(cudaGetLastError());
       GBF_CUDA(cudaEventRecord(d->pipe_ev[2 + ns + r], cs));
@@ -737,9 +734,6 @@ int split_advance_host(gbf_domain* d, const double* P_in, const double* S_in, do
       GBF_CUDA(cudaMemcpyAsync(S_out + c0, stS + c0, b, cudaMemcpyDefault, d->pipe_out));
     }
   }
-  if (mass_out)
-    k_split_mass_tail<<<1, 256, 0, cs>>>(G.mass_partials, (int)(tiles * ns), mass_out,
-                                         gbf_is_defect(mr) ? d->defect_k1v : 0.0);
   GBF_CUDA(cudaGetLastError());
   GBF_CUDA(cudaEventRecord(d->pipe_ev[1], d->pipe_out));
   GBF_CUDA(cudaStreamWaitEvent(cs, d->pipe_ev[1], 0));
@@ -762,7 +756,7 @@ int gbf_split_advance_host(gbf_domain* d, const double* P_in, const double* S_in
 }
 
 int gbf_split_launches_per_step(gbf_domain* d) {
-  return 2 + ((d->out_flags & GBF_OUT_MASS) ? 1 : 0) + (d->split_patch ? 1 : 0);
+  return 2 + (d->split_patch ? 1 : 0);
 }
 
 // ----------------------------------------------------------- diagnostics

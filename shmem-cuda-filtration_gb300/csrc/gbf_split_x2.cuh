@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(TX / 2 * TY, gbf_pair_ctas(MR)) k_split_step_x
   const int k0 = 1 + kc * kchunk;
   const int k1 = min(k0 + kchunk, C.nz - 1);
   if (threadIdx.x == 0) gbf_pair_bars_init(cta.bars);
+  gbf_pdl_begin();
   __syncthreads();
   unsigned phases = 0;
   GbfSplitAcc<MR> acc;
@@ -55,7 +56,8 @@ int launch_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, const GbfTmaSet* m
   const unsigned blocks = (unsigned)(tiles_x2<TX>(C) * tiles_y2<TY>(C) * nkc);
   const int bytes = (int)sizeof(GbfPairCta<TX, TY, MR>);
   GBF_CUDA(cudaFuncSetAttribute(k_split_step_x2<MR, TX, TY, CFL, PATCH, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  k_split_step_x2<MR, TX, TY, CFL, PATCH, TAB><<<blocks, TX / 2 * TY, bytes, st>>>(C, G, kchunk, kc0, maps, buf);
+  GBF_CUDA(gbf_launch(true, k_split_step_x2<MR, TX, TY, CFL, PATCH, TAB>, blocks, TX / 2 * TY, (size_t)bytes, st, C, G, kchunk, kc0,
+                      maps, buf));
   return GBF_OK;
 }
 
