@@ -987,6 +987,120 @@ __device__ __forceinline__ void split_cells(const GbfSplitConsts& C, const GbfCe
   }
 }
 
+// split_cells for cells that hold no DNAPL, have none around them and get
+// none (S = 0 and M2 = 0; L2 = 0 at the cell and its six neighbours; no
+// source): every DNAPL flux, r2, the Newton's dS and P_k's derivative times S
+// are zero, S_e = 1 and P_k = P_d, and the second Newton step is not needed.
+// What is left, the water equation, is the same operations on the same
+// numbers, so dP, S, M1, the masses and CFL numbers keep the bits of split_cells (a
+// zero's sign aside); M2 stays as it is and the DNAPL sums get nothing. A
+// water equation that overflows makes S non-finite, as there.
+template <int MR, int N, bool CFL>
+__device__ __forceinline__ void split_cells_dry(const GbfSplitConsts& C, const GbfCellIn (&in)[N],
+                                                const typename MassRep<MR>::T (&M1)[N], typename WideOf<MR>::T R01,
+                                                const GbfDefectRow& rw, const int (&md)[N], unsigned rowf, int j,
+                                                bool phi_field, bool mass, const bool (&count)[N],
+                                                GbfSplitAcc<MR>& acc, GbfCellOut<MR> (&o)[N]) {
+  using W = WideOf<MR>;
+  using L = Lanes<N>;
+  using F = typename L::F;
+  constexpr bool DEF = gbf_is_defect(MR);
+  const bool noflow = rowf & 1u;
+  auto sp = [](float x) { return L::splat(x); };
+  auto mt = [&](const float (&t)[2]) { return L::make([&](int n) { return split_of(t, md[n]); }); };
+  auto upw = [](F x, F Lm, F Lp) {
+    return L::make([&](int n) { return L::get(x, n) >= 0.f ? L::get(Lm, n) : L::get(Lp, n); });
+  };
+  const F dPc = L::make([&](int n) { return in[n].dPc; });
+  const F L1c = L::make([&](int n) { return in[n].L1c; });
+  float ax1[N], ax2[N], dx1[N];
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    ax1[n] = split_face(__fsub_rn(in[n].dPxm, in[n].dPc), in[n].L1xm, in[n].L1c);
+    ax2[n] = split_face(__fsub_rn(in[n].dPc, in[n].dPxp), in[n].L1c, in[n].L1xp);
+    dx1[n] = __fsub_rn(ax1[n], ax2[n]);
+  }
+  const F Pp = vfma(sp((float)j), sp(C.H), dPc);
+  const F yb1 = vsub(L::make([&](int n) { return in[n].dPym; }), dPc);
+  const F yb2 = vsub(dPc, L::make([&](int n) { return in[n].dPyp; }));
+  const F z2 = vsub(dPc, L::make([&](int n) { return in[n].dPp; }));
+  const F y11 = vfma(sp(C.gh1), Pp, yb1), y21 = noflow ? sp(0.f) : vfma(sp(C.gh1), Pp, yb2);
+  const F ay2 = vmul(y21, upw(y21, L1c, L::make([&](int n) { return in[n].L1yp; })));
+  const F az2 = vmul_exact(z2, upw(z2, L1c, L::make([&](int n) { return in[n].L1p; })));
+  const F az1 = L::make([&](int n) { return in[n].fz1; });
+  const F dy1 = vfma(y11, upw(y11, L::make([&](int n) { return in[n].L1ym; }), L1c), vneg(ay2));
+  const F f = vfma(vsub(az1, az2), sp(C.wz), vfma(dy1, sp(C.wy), vmul(L::make([&](int n) { return dx1[n]; }), sp(C.wx))));
+  const F nrphi = L::make([&](int n) { return split_rcp(-in[n].phi); });
+  const F dm1 = vmul_exact(f, nrphi);
+  if (CFL) {
+#pragma unroll
+    for (int n = 0; n < N; n++)
+      if (count[n]) {
+        const float ay1 = split_face(L::get(y11, n), in[n].L1ym, in[n].L1c);
+        const float ay2n = split_face(L::get(y21, n), in[n].L1c, in[n].L1yp);
+        const float c1 = fmaxf(fmaxf(__fmul_rn(fmaxf(fabsf(ax1[n]), fabsf(ax2[n])), C.wx),
+                                     __fmul_rn(fmaxf(fabsf(ay1), fabsf(ay2n)), C.wy)),
+                               __fmul_rn(fmaxf(fabsf(L::get(az1, n)), fabsf(L::get(az2, n))), C.wz));
+        acc.cfl1 = fmaxf(acc.cfl1, __fmul_rn(__fmul_rn(c1, -L::get(nrphi, n)), C.cfl1));
+      }
+  }
+  F r1;
+  if constexpr (DEF)
+    r1 = vfma(vneg(f), nrphi, vsub(vfma(sp(C.ro01b1), dPc, sp(rw.e1)), L::make([&](int n) { return defect_f(M1[n]); })));
+  else
+    r1 = L::make([&](int n) {
+      return __fmaf_rn(-L::get(f, n), L::get(nrphi, n),
+                       __fadd_rn(__fmul_rn(C.ro01b1, L::get(Pp, n)), W::rho_1mS_minus(R01, M1[n], 0.f)));
+    });
+  const F J22 = vmul(sp(C.ro02), vfma(sp(C.beta2), vadd(mt(C.P_d), Pp), sp(1.f)));
+  const F det = vmul(sp(C.ro01b1), J22);
+  const F ninv = L::make([&](int n) { return split_rcp(-L::get(det, n)); });
+  F dPn = vfma(ninv, vmul(J22, r1), dPc);
+  if constexpr (MR == kMassDefectDF) {  // the residual-correction step
+    F s, e;  // T1' = D1 + dm1 as a pair
+    {
+      const F d = L::make([&](int n) { return M1[n].hi; });
+      s = vadd(d, dm1);
+      const F bb = vsub(s, d);
+      e = vadd(vsub(d, vsub(s, bb)), vsub(dm1, bb));
+    }
+    const F T1l = vadd(e, L::make([&](int n) { return M1[n].lo; }));
+    const F a1 = vmul_exact(sp(C.ro01b1), dPn);
+    const F a1e = vfma(sp(C.ro01b1_lo), dPn, vfma(sp(C.ro01b1), dPn, vneg(a1)));
+    const F q1 = vadd(vsub(a1, s), vsub(vadd(sp(rw.e1), a1e), T1l));
+    dPn = vfma(ninv, vmul(J22, q1), dPn);
+  }
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    const float P = L::get(dPn, n), d = L::get(dm1, n);
+    o[n].dPn = P;
+    o[n].Sn = __fmaf_rn(P, 0.f, 0.f);  // 0, or NaN
+    o[n].fz1 = L::get(az2, n);
+    o[n].fz2 = 0.f;
+    if (count[n] && !isfinite(P)) acc.bad = 1;
+    if constexpr (DEF) o[n].M1n = defect_add(M1[n], d);
+    else o[n].M1n = W::add_f(M1[n], d);
+  }
+  if (mass) {
+#pragma unroll
+    for (int n = 0; n < N; n++)
+      if (count[n]) {
+        const float ph = phi_field ? in[n].phi : md[n] ? C.m_df[1].x : C.m_df[0].x;
+        const float pl = phi_field ? 0.f : md[n] ? C.m_df[1].y : C.m_df[0].y;
+        if constexpr (MR == kMassDefect) {
+          acc.b1 = __fmaf_rn(ph, o[n].M1n, acc.b1);
+        } else if constexpr (MR == kMassDefectDF) {
+          acc.b1 = Wide<true>::acc_phi(acc.b1, ph, o[n].M1n);
+          if (!phi_field) acc.b1.lo = __fmaf_rn(pl, o[n].M1n.hi, acc.b1.lo);
+        } else if (phi_field) {
+          acc.m1 = W::acc_phi(acc.m1, in[n].phi, o[n].M1n);
+        } else {
+          acc.m1 = W::add(acc.m1, W::mul(W::c(md[n] ? C.m_d[1] : C.m_d[0], md[n] ? C.m_df[1] : C.m_df[0]), o[n].M1n));
+        }
+      }
+  }
+}
+
 // One CTA: interior cells [i0, i0+TX) x [j0, j0+TY) of planes [k0, k1); i0,
 // j0, k0 >= 1. `pl` points to two planes of shared memory.
 //
@@ -1455,6 +1569,7 @@ struct GbfPairSmem {
   Ring ring;
   float dP[kTmaStages][Ring::NP];
   float L1[kTmaStages][Ring::NP], L2[kTmaStages][Ring::NP];
+  int wet[kTmaStages];  // the last plane of each buffer with DNAPL (of another tile before: taken as wet, no harm)
 };
 // The mbarriers of the two rings (halo planes, interior rows), apart from the
 // ring data: a CTA that runs tiles of two shapes keeps one set of barriers,
@@ -1497,6 +1612,10 @@ template <int MR>
 __device__ __forceinline__ double* mass_at(double* p, size_t c) {
   return reinterpret_cast<double*>(reinterpret_cast<MassElem<MR>*>(p) + c);
 }
+// The bits of a value's parts, for "all of these are zero" ((bits << 1) == 0: the signs aside).
+__device__ __forceinline__ unsigned fbits(float a) { return __float_as_uint(a); }
+__device__ __forceinline__ unsigned fbits(float2 a) { return __float_as_uint(a.x) | __float_as_uint(a.y); }
+__device__ __forceinline__ unsigned fbits(GbfDF a) { return __float_as_uint(a.hi) | __float_as_uint(a.lo); }
 template <int MR> struct WidePair;
 template <> struct WidePair<kMassF64> {  // FP64 masses: two doubles
   static __device__ __forceinline__ void load(const double* p, double& a, double& b) {
@@ -1533,7 +1652,13 @@ template <> struct WidePair<kMassDefect> {  // FP32 defects: two floats
 // The x-pair z-marching tile: cells x0 .. x0 + TXC - 1 (interior ones only)
 // of rows j0 .. j0 + TY - 1, planes k0 .. k1 - 1. Same staging protocol,
 // bounded waits and give-up as split_tile<..., TMA = true>; each cell is
-// updated by split_cell, so results equal the other tiles' bit for bit. The
+// updated by split_cells or, warp by warp, split_cells_dry, so results equal the
+// other tiles' bit for bit. A dry warp leaves M2 unwritten and issues about half
+// of the instructions (in the pair defect form): 256^3 with DNAPL in a fifth of
+// the cells 199 -> 171 us a step, 512x512x256 744 -> 596; in the defect form
+// 256^3 156 -> 135. Where every cell has DNAPL the look costs 199 -> 208 us (defect
+// form 156 -> 157). Flags of a whole tile's plane, built with it, and a look at
+// every fourth plane only were slower (175 and 209, 179 and 213 us). The
 // CTA has NTB >= TXC / 2 * TY threads; the ones beyond the tile take part in
 // the barriers only. TAB: a grid of the media table instead of K and porosity
 // fields; the halo box that holds K holds the cells' media indices (as they
@@ -1644,7 +1769,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
     md = has_media ? make_int2(__float_as_int(kv.x), __float_as_int(kv.y)) : make_int2(0, 0);
     return make_float2(split_of(C.K, md.x), split_of(C.K, md.y));
   };
-  auto build = [&](int s) {  // plane buffer s from halo stage s
+  auto build = [&](int s, int k) {  // plane buffer s (plane k) from halo stage s
 #pragma unroll
     for (int q = 0; q < SLOTS; q++) {
       // slot 0: the own pair of every thread in the tile; the first later
@@ -1682,7 +1807,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
   }
   {
     const bool ok = wait_bit(0);
-    if (ok) build(0);
+    if (ok) build(0, k0);
     if (__syncthreads_or(!ok)) {
       give_up();
       return false;
@@ -1705,6 +1830,8 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
     acc.c1 = rw.c1;
     acc.c2 = rw.c2;
   }
+  // the tile has cells of the rate source's or the patch's row and columns
+  const bool src_cols = j0 == 1 && x0 < C.ri0 + C.rn && x0 + TXC > C.ri0;
   int u = 0;  // (k - k0) % 3: plane buffer, halo stage and rows stage of plane k
   for (int k = k0; k < k1; k++) {
     const float2 s0 = s_own;  // plane k's, before the build of plane k + 1 replaces it
@@ -1714,7 +1841,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       const int sn = t_next;
       bool ok = wait_bit(sn);
       ok = ok && wait_bit(8 + t_rows);
-      if (ok) build(sn);
+      if (ok) build(sn, k + 1);
       if (__syncthreads_or(!ok)) {
         give_up();
         return false;
@@ -1724,62 +1851,82 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       if (k + 1 + kTmaStages <= k1) issue(k + 1 + kTmaStages, sn);
       if (k > k0 && k + 2 < k1) issue_rows(k + 2, sn == 2 ? 0 : sn + 1);
     }
-    if (any) {
+    // Warps whose cells hold no DNAPL and have none around or coming take
+    // split_cells_dry: L2 zero at the cells and their neighbours (fz2: the
+    // plane below), S and M2 zero, no source in the tile's plane.
+    const float* P2 = sm.L2[t_cur];
+    const int e = in_tile ? hc : BX + 4;
+    const float2 b0 = gbf_ld2(P2 + e), bl = gbf_ld2(P2 + e - 2), br = gbf_ld2(P2 + e + 2);
+    const float2 bu = gbf_ld2(P2 + e - BX), bd = gbf_ld2(P2 + e + BX), bp = gbf_ld2(sm.L2[t_next] + e);
+    MT M2a, M2b;
+    WidePair<MR>::load(reinterpret_cast<const double*>(&raw.m2[t_rows][in_tile ? mi : 0]), M2a, M2b);
+    unsigned wet = fbits(b0) | fbits(bl.y) | fbits(br.x) | fbits(bu) | fbits(bd) | fbits(bp) | fbits(s0) | fbits(fza2) |
+                   fbits(fzb2) | fbits(M2a) | fbits(M2b);
+    if (src_cols && (unsigned)(k - C.rk0) < (unsigned)C.rn) wet = ~0u;
+    const bool dry = !__any_sync(0xffffffffu, any && (wet << 1) != 0u);
+    auto update = [&](bool dry_cells) {
       const float* Pd = sm.dP[t_cur];
       const float* P1 = sm.L1[t_cur];
-      const float* P2 = sm.L2[t_cur];
       const float2 d0 = gbf_ld2(Pd + hc), dl = gbf_ld2(Pd + hc - 2), dr = gbf_ld2(Pd + hc + 2);
       const float2 du = gbf_ld2(Pd + hc - BX), dd = gbf_ld2(Pd + hc + BX);
       const float2 a0 = gbf_ld2(P1 + hc), al = gbf_ld2(P1 + hc - 2), ar = gbf_ld2(P1 + hc + 2);
       const float2 au = gbf_ld2(P1 + hc - BX), ad = gbf_ld2(P1 + hc + BX);
-      const float2 b0 = gbf_ld2(P2 + hc), bl = gbf_ld2(P2 + hc - 2), br = gbf_ld2(P2 + hc + 2);
-      const float2 bu = gbf_ld2(P2 + hc - BX), bd = gbf_ld2(P2 + hc + BX);
-      const float2 dp = gbf_ld2(sm.dP[t_next] + hc), ap = gbf_ld2(sm.L1[t_next] + hc),
-                   bp = gbf_ld2(sm.L2[t_next] + hc);
+      const float2 dp = gbf_ld2(sm.dP[t_next] + hc), ap = gbf_ld2(sm.L1[t_next] + hc);
       const float2 ph = TAB ? make_float2(split_of(C.m, mds[0]), split_of(C.m, mds[1])) : gbf_ld2(&raw.phi[t_rows][mi]);
-      MT M1a, M1b, M2a, M2b;
+      MT M1a, M1b;
       WidePair<MR>::load(reinterpret_cast<const double*>(&raw.m1[t_rows][mi]), M1a, M1b);
-      WidePair<MR>::load(reinterpret_cast<const double*>(&raw.m2[t_rows][mi]), M2a, M2b);
       GbfCellIn in[2];
       // cell a
-      in[0].dPc = d0.x; in[0].S0 = s0.x; in[0].L1c = a0.x; in[0].L2c = b0.x;
+      in[0].dPc = d0.x; in[0].S0 = s0.x; in[0].L1c = a0.x;
       in[0].dPxm = dl.y; in[0].dPxp = d0.y; in[0].dPym = du.x; in[0].dPyp = dd.x;
       in[0].L1xm = al.y; in[0].L1xp = a0.y; in[0].L1ym = au.x; in[0].L1yp = ad.x;
-      in[0].L2xm = bl.y; in[0].L2xp = b0.y; in[0].L2ym = bu.x; in[0].L2yp = bd.x;
       in[0].fz1 = fza1; in[0].fz2 = fza2;
-      in[0].dPp = dp.x; in[0].L1p = ap.x; in[0].L2p = bp.x;
+      in[0].dPp = dp.x; in[0].L1p = ap.x;
       in[0].phi = ph.x;
       // cell b
-      in[1].dPc = d0.y; in[1].S0 = s0.y; in[1].L1c = a0.y; in[1].L2c = b0.y;
+      in[1].dPc = d0.y; in[1].S0 = s0.y; in[1].L1c = a0.y;
       in[1].dPxm = d0.x; in[1].dPxp = dr.x; in[1].dPym = du.y; in[1].dPyp = dd.y;
       in[1].L1xm = a0.x; in[1].L1xp = ar.x; in[1].L1ym = au.y; in[1].L1yp = ad.y;
-      in[1].L2xm = b0.x; in[1].L2xp = br.x; in[1].L2ym = bu.y; in[1].L2yp = bd.y;
       in[1].fz1 = fzb1; in[1].fz2 = fzb2;
-      in[1].dPp = dp.y; in[1].L1p = ap.y; in[1].L2p = bp.y;
+      in[1].dPp = dp.y; in[1].L1p = ap.y;
       in[1].phi = ph.y;
-      const MT m1s[2] = {M1a, M1b}, m2s[2] = {M2a, M2b};
+      const MT m1s[2] = {M1a, M1b};
       const bool cnt[2] = {act_a, act_b};
       GbfCellOut<MR> o[2];
-      split_cells<MR, 2, CFL, PATCH>(C, in, m1s, m2s, R01, R02, rw, mds, rowf, j, k, !TAB, G.mass_partials != nullptr,
-                                     cnt, acc, o, G.patch_in, ia);
+      if (dry_cells) {
+        split_cells_dry<MR, 2, CFL>(C, in, m1s, R01, rw, mds, rowf, j, !TAB, G.mass_partials != nullptr, cnt, acc, o);
+      } else {
+        in[0].L2c = b0.x; in[0].L2p = bp.x;
+        in[0].L2xm = bl.y; in[0].L2xp = b0.y; in[0].L2ym = bu.x; in[0].L2yp = bd.x;
+        in[1].L2c = b0.y; in[1].L2p = bp.y;
+        in[1].L2xm = b0.x; in[1].L2xp = br.x; in[1].L2ym = bu.y; in[1].L2yp = bd.y;
+        const MT m2s[2] = {M2a, M2b};
+        split_cells<MR, 2, CFL, PATCH>(C, in, m1s, m2s, R01, R02, rw, mds, rowf, j, k, !TAB, G.mass_partials != nullptr,
+                                       cnt, acc, o, G.patch_in, ia);
+        const unsigned c = (unsigned)(ia + j * px) + (unsigned)k * pln;
+        WidePair<MR>::store(mass_at<MR>(G.M2, c), act_a ? o[0].M2n : M2a, act_b ? o[1].M2n : M2b);
+      }
       // The x faces i = 0 and i = nx - 1 (rows and planes interior) take the
       // boundary rules' values here: the new S of the x-neighbour and its dP
       // (cpu.cpp:327-331, 366-372), or the hydrostatic side value dP = 0 with
       // GBF_BC_HYDROSTATIC_SIDES; no other boundary rule reads these cells, so
       // the face pass skips them (gbf_boundary_count_no_xfaces, gbf_face_row).
-      const GbfCellOut<MR> oa = act_a ? o[0] : GbfCellOut<MR>{hsides ? 0.f : o[1].dPn, o[1].Sn, M1a, M2a};
-      const GbfCellOut<MR> ob = act_b ? o[1] : GbfCellOut<MR>{hsides ? 0.f : o[0].dPn, o[0].Sn, M1b, M2b};
+      const GbfCellOut<MR> oa = act_a ? o[0] : GbfCellOut<MR>{hsides ? 0.f : o[1].dPn, o[1].Sn, M1a};
+      const GbfCellOut<MR> ob = act_b ? o[1] : GbfCellOut<MR>{hsides ? 0.f : o[0].dPn, o[0].Sn, M1b};
       const unsigned c = (unsigned)(ia + j * px) + (unsigned)k * pln;  // even: px and ia are
       gbf_st2(G.dPn + c, oa.dPn, ob.dPn);
       gbf_st2(G.Sn + c, oa.Sn, ob.Sn);
       WidePair<MR>::store(mass_at<MR>(G.M1, c), oa.M1n, ob.M1n);
-      WidePair<MR>::store(mass_at<MR>(G.M2, c), oa.M2n, ob.M2n);
       if (odd_face) {
         G.dPn[c + 2] = hsides ? 0.f : ob.dPn;
         G.Sn[c + 2] = ob.Sn;
       }
       fza1 = o[0].fz1; fza2 = o[0].fz2;
       fzb1 = o[1].fz1; fzb2 = o[1].fz2;
+    };
+    if (any) {
+      if (dry) update(true);
+      else update(false);
     }
     u = t_next;
   }
