@@ -176,23 +176,3 @@ __device__ __forceinline__ void gbf_f64_boundary_cell(const gbf_model& m, const 
   s.Sn[c] = gbf_sweep_S<double>(m, g, s.Sn, s.S, i, j, k);
   s.Pn[c] = gbf_sweep_P<double>(m, g, s.Pn, s.P, i, j, k, ro1_top);
 }
-
-// Sum of warp values of the block into out[0..1] (thread 0), fixed order.
-template <int NT>
-__device__ __forceinline__ void gbf_block_sum2(double a, double b, double V, double* out) {
-  __shared__ double red[2][NT / 32];
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    b += __shfl_down_sync(0xffffffffu, b, o);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { red[0][w] = a; red[1][w] = b; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double x = 0., y = 0.;
-    for (int q = 0; q < NT / 32; q++) { x += red[0][q]; y += red[1][q]; }
-    out[0] = x * V;
-    out[1] = y * V;
-  }
-  __syncthreads();
-}

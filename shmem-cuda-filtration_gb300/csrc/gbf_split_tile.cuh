@@ -1507,29 +1507,12 @@ __device__ __forceinline__ void split_block_cfl(float c1, float c2, float* out) 
   __syncthreads();  // red is reused by the next tile of a persistent CTA
 }
 
-// Deterministic block reduction of the threads' phase masses (FP64).
-template <int NT>
-__device__ __forceinline__ void split_block_mass_d(double a, double b, double V, double* out2) {
-  __shared__ double red[2][NT / 32];
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    b += __shfl_down_sync(0xffffffffu, b, o);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { red[0][w] = a; red[1][w] = b; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double x = 0., y = 0.;
-    for (int q = 0; q < NT / 32; q++) { x += red[0][q]; y += red[1][q]; }
-    out2[0] = x * V;
-    out2[1] = y * V;
-  }
-}
+// The threads' phase masses, summed over the block (FP64).
 template <int MR, int NT = kSplitThreads>
 __device__ __forceinline__ void split_block_mass(const GbfSplitAcc<MR>& acc, double V, double* out2) {
   double a, b;
   acc.masses(a, b);
-  split_block_mass_d<NT>(a, b, V, out2);
+  gbf_block_sum2<NT>(a, b, V, out2);
 }
 
 // ------------------------------------------------ x-pair tile (TMA only)
