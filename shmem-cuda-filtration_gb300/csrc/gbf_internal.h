@@ -237,7 +237,8 @@ void gbf_timer_free(GbfTimer* t);
 // 1 us) shrinks. Every kernel launched with pdl calls it before its first
 // access to global memory. The ensembles' steps are launched without: as edges
 // of their CUDA graphs the programmatic launches cost more than the gaps (a
-// step of two FP64 members 187 us plain, 245 us with them).
+// step of two FP64 members 187 us plain, 245 us with them); so are a caller's
+// captures of a domain's stream.
 #ifdef __CUDACC__
 __device__ __forceinline__ void gbf_pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;");
@@ -246,6 +247,8 @@ __device__ __forceinline__ void gbf_pdl_begin() {
 template <class... P, class... A>
 cudaError_t gbf_launch(bool pdl, void (*kern)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
                        A&&... args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (pdl && (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) pdl = false;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
