@@ -7,17 +7,20 @@
 // (gbf_f64_pair.cuh) and touches the FP64 pipe for five additions a cell:
 //   pass 1 (k_pair_props, every cell): pressure against the row's hydrostatic
 //     value, mobility x density of both phases, capillary pressure, as pairs
-//     (32 bytes a cell written);
+//     (32 bytes a cell written, 24 without DNAPL);
 //   pass 2 (k_pair_step, interior cells): upwinded face fluxes with gravity
 //     (cpu.cpp:218-291) and the 2x2 Newton (cpu.cpp:293-320) in increments,
 //     the next FP64 state (ping-pong), phase-mass partial sums on request.
 // Two passes, not one tile: a cell's properties cost half of its fluxes and
 // Newton, so they are not computed again for halos, and the 64 bytes a cell
 // that this moves beside the state are hidden behind the arithmetic. Both are
-// bound by instruction issue (pass 1 with the FP64 pipe 61% busy); 256^3,
-// heterogeneous, a quarter of the cells with DNAPL: pass 1 223 us, pass 2 440
-// us (2.3 and 2.6 TB/s of their 52 and 68 bytes a cell), where the FP64
-// passes took 2460 and 6270. Pass 2 takes 64 registers for four blocks an SM:
+// bound by instruction issue, with the FP64 pipe about half busy; 256^3,
+// heterogeneous, a fifth of the cells with DNAPL: pass 1 204 us (223 with the
+// DNAPL mobility formed and P_k stored in every cell), pass 2 445 us (2.2 and
+// 2.4 TB/s of 44 and 62 bytes a cell), where the FP64 passes took 2460 and
+// 6270. Pass 1 keeps to 32 registers for eight blocks an SM: at 40 it takes 226
+// us, and on small grids fewer blocks of the next kernel fit beside it (40
+// steps of 40^3 778 -> 881 us). Pass 2 takes 64 registers for four blocks an SM:
 // at three (80 registers) its latencies show, 808 us; at five and six it spills
 // (627, 764).
 //   face pass (k_f64_boundary): the reference's sweep-ordered boundary
@@ -57,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) k_f64_flux_newton(const gbf_model m,
 }
 
 template <bool DROPIN>
-__global__ void __launch_bounds__(kThreads) k_pair_props(const GbfPairConsts C, const gbf_cells cells,
+__global__ void __launch_bounds__(kThreads, 8) k_pair_props(const GbfPairConsts C, const gbf_cells cells,
                                                          const GbfF64Step s, const GbfPairWork w) {
   gbf_pdl_begin();
   for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < C.n; c += gridDim.x * blockDim.x)

@@ -75,7 +75,7 @@ int gbf_pair_fill_rows(const gbf_model& m, GbfPairRow* rows, cudaStream_t st);
 
 // Arrays of a pair step beside GbfF64Step's P, S, Pn, Sn.
 struct GbfPairWork {
-  float2 *D, *L1, *L2, *Pk;  // P - P_hs(j), mobility x density of both phases, capillary pressure
+  float2 *D, *L1, *L2, *Pk;  // P - P_hs(j), mobility x density of both phases, capillary pressure (where S is not 0)
   const GbfPairRow* rows;
   // drop-in (NULL: none): the caller's (P, S) that pass 1 reads and copies to
   // s.P, s.S; it also writes the density arrays s.ro1, s.ro2
@@ -130,11 +130,13 @@ __device__ __forceinline__ void gbf_pair_props_cell(const GbfPairConsts& C, cons
   const GbfPairRow R = w.rows[j];
   const GbfPf D = pf_from_double(__dsub_rn(P, R.phs));
   const GbfPf Pp = pf_add(R.pp, D);
-  GbfPf kr1 = {1.f, 0.f}, kr2 = {0.f, 0.f}, pk = C.pd[md];
-  if (!gbf_is_zero(S)) {  // S = 0: the fully water-saturated values
+  const float K = cells.K ? __ldg(cells.K + c) : 0.f;
+  auto over_mu = [&](const GbfPf& rmu) { return cells.K ? pf_mulf(rmu, K) : pf_mul(rmu, C.K[md]); };  // K / mu
+  GbfPf l1 = over_mu(C.c1), l2 = {0.f, 0.f};
+  if (!gbf_is_zero(S)) {  // S = 0: kr1 = 1, kr2 = 0, and P_k = P_d is not stored
     const double om = __dmul_rn(S, C.inv_d[md]);
     const GbfPf omp = pf_from_double(om);
-    GbfPf w2;
+    GbfPf kr1, w2, pk = C.pd[md];
     if (pair_om_ok(omp.h)) {
       const double l = gbf_ln1m(om, omp.h);
       const GbfPf lp = pf_from_double(l);
@@ -146,23 +148,13 @@ __device__ __forceinline__ void gbf_pair_props_cell(const GbfPairConsts& C, cons
       w2 = pf_from_double(1.0 - pair_pow_general(om, C.E2[md]));
       pk = pf_mul(pk, pf_from_double(pair_pow_general(om, C.E3[md])));
     }
-    kr2 = pf_mul(pf_mul(omp, omp), w2);
-  }
-  const GbfPf rho1 = pf_add(C.ro1, pf_mul_raw(C.k1, Pp));
-  const GbfPf rho2 = pf_add(C.ro2, pf_mul_raw(C.k2, Pp));
-  GbfPf q1, q2;
-  if (cells.K) {
-    const float K = __ldg(cells.K + c);
-    q1 = pf_mulf(C.c1, K);
-    q2 = pf_mulf(C.c2, K);
-  } else {
-    q1 = pf_mul(C.c1, C.K[md]);
-    q2 = pf_mul(C.c2, C.K[md]);
+    l1 = pf_mul(l1, kr1);
+    l2 = pf_mul(pf_mul(over_mu(C.c2), pf_mul(pf_mul(omp, omp), w2)), pf_add(C.ro2, pf_mul_raw(C.k2, Pp)));
+    pf_st(w.Pk + c, pk);
   }
   pf_st(w.D + c, D);
-  pf_st(w.L1 + c, pf_mul(pf_mul(q1, kr1), rho1));
-  pf_st(w.L2 + c, pf_mul(pf_mul(q2, kr2), rho2));
-  pf_st(w.Pk + c, pk);
+  pf_st(w.L1 + c, pf_mul(l1, pf_add(C.ro1, pf_mul_raw(C.k1, Pp))));
+  pf_st(w.L2 + c, l2);
 }
 
 // a - b, normalised
@@ -336,7 +328,7 @@ __device__ __forceinline__ void gbf_pair_step_cell(const GbfPairConsts& C, const
     double rest = 0.;  // what the pair r2 leaves of the source
     if (src) r2 = pf_sub(r2, pair_source(C.dtsrc_d, cells.phi ? gbf_f2d(phif) : C.phi_d[md], rest));
     GbfPf ds;
-    pair_newton(C, md, Pp, pf_from_double(Sd), pf_ld(w.Pk + c), r1, r2, dp, ds);
+    pair_newton(C, md, Pp, pf_from_double(Sd), gbf_is_zero(Sd) ? C.pd[md] : pf_ld(w.Pk + c), r1, r2, dp, ds);
     const double dsd = pf_to_double(ds);
     Sn = __dadd_rn(Sd, dsd);
     if (src) Sn = pair_add_rest(Sd, dsd, rest, C.rro2_d);
