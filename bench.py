@@ -359,19 +359,21 @@ class DropinRunner:
 # Algorithmic bytes per interior (or every) cell of each kernel: the
 # compulsory DRAM traffic of its inputs and outputs.
 ALGO_BYTES = {
-    "f64_props": (60.0, "all"),             # read P, S, K (20); write L1, L2, ro1, ro2, lnSe (40)
-    "ensemble_f64_props": (60.0, "all"),
-    "f64_flux_newton": (76.0, "interior"),  # read P, S, L1, L2, ro1, ro2, lnSe (56), phi (4); write P, S (16)
-    "ensemble_f64_flux_newton": (76.0, "interior"),
-    "split_step": (56.0, "interior"),       # read dP, S, K, phi (16), M1, M2 (16); write dP, S (8), M1, M2 (16)
+    "f64_props": (52.0, "all"),             # read P, S, K (20); write P - P_hs, L1, L2, P_k as FP32 pairs (32)
+    "ensemble_f64_props": (52.0, "all"),
+    "f64_flux_newton": (60.0, "interior"),  # read P, S, P - P_hs, L1, L2 (40), phi (4); write P, S (16); 8 more with DNAPL
+    "ensemble_f64_flux_newton": (60.0, "interior"),
+    # read dP, S, K, phi (16), M1, M2 (16); write dP, S (8), M1, M2 (16). Cells without DNAPL leave M2
+    # unwritten: 8 bytes fewer (4 in the defect form)
+    "split_step": (56.0, "interior"),
     "ensemble_step": (56.0, "interior"),
 }
 # The defect form holds M1, M2 in 4 bytes: read 16 + 8, write 8 + 8.
 ALGO_BYTES_DEFECT = {"split_step": (40.0, "interior"), "ensemble_step": (40.0, "interior")}
-# The drop-in's media-table grid reads an int media index instead of K, phi (props: P, S, media;
-# flux/Newton: no phi read).
+# The drop-in's media-table grid reads an int media index instead of K, phi (props: P, S, media, and the
+# copy of the caller's state and its densities written; flux/Newton: media in place of phi).
 # Split mode: read dP, S (8), media (4), M1, M2 (16); write dP, S (8), M1, M2 (16).
-ALGO_BYTES_DROPIN = {"f64_props": (60.0, "all"), "f64_flux_newton": (72.0, "interior"),
+ALGO_BYTES_DROPIN = {"f64_props": (84.0, "all"), "f64_flux_newton": (60.0, "interior"),
                      "split_step": (52.0, "interior")}
 
 
@@ -544,15 +546,14 @@ def run_ours(args, rank, world):
             "frac": achieved / hbm, "peak_source": peak_kind, "traffic": traffic,
             "algorithmic_bytes_per_launch": algo, "bytes_per_cell": bpc, "ms_per_launch": per_launch_s * 1e3,
             "kernel_times_ms": {k: {"total_ms": v[0], "launches": v[1]} for k, v in ktimes.items()},
-            "binding_resource": ("FP64 pipe (ncu: 85% of FP64-pipe cycles active in the flux/Newton pass; "
-                                 "GB300 DFMA 1.2 TFLOP/s)") if f64 else
-                                ("instruction issue and the per-plane block barrier (ncu: 66-80% issue "
-                                 "active; DRAM traffic 1.12-1.16x the algorithmic bytes on config 4, halo "
-                                 "rows re-read)"),
+            "binding_resource": ("instruction issue, and beside it the FP64 pipe (ncu: 72% issue active, "
+                                 "46% of FP64-pipe cycles active in the flux/Newton pass)") if f64 else
+                                ("instruction issue and the per-plane block barrier (algorithmic bytes are those of "
+                                 "a cell with DNAPL; others leave the DNAPL mass, 8 or 4 bytes, unwritten)"),
             "ms_per_step_with_kernel_events": ms_k / args.steps}
-    if f64:  # the FP64 kernels' own roof: the FP64 pipe, from the ncu capture of this pass
-        roof["fp64_pipe"] = {"frac": 0.853, "metric": "sm__pipe_fp64_cycles_active",
-                             "source": "profiles/f64_flux_newton_config1.md (flux/Newton pass, 192^3)"}
+    if f64:  # the FP64 pipe beside it, from the ncu capture of this pass
+        roof["fp64_pipe"] = {"frac": 0.464, "metric": "sm__pipe_fp64_cycles_active",
+                             "source": "profiles/f64_pair_step_config1.md (flux/Newton pass, 192^3)"}
 
     # e2e through the public API with pinned host buffers: H2D state, one step, D2H P and S,
     # every step timed on its own (the host link is shared with other jobs on the host)
@@ -619,10 +620,10 @@ def run_ours(args, rank, world):
            "data": "synthetic (seeded fields with the configuration's shapes and statistics)",
            "config": W.config(),
            "details": {"dt_used_range": [min(m.model.dt for m in members), max(m.model.dt for m in members)],
-                       "newton": ("converge-and-exit (tol 1e-11, at most the reference's 7)" if p == "dropin" else
+                       "newton": ("increments on FP32 pairs, to round-off" if p == "dropin" else
                                   "increment Newton, a second iteration where nonlinear, one residual-correction "
                                   "step" if p == "dropinsplit" else
-                                  "FP64: converge-and-exit (tol 1e-11, max 7); split: increment Newton, a second "
+                                  "FP64: increments on FP32 pairs, to round-off; split: increment Newton, a second "
                                   "iteration where nonlinear, and (split) one residual-correction step"),
                        "tuning": tuning, "graphs": ensemble, "rank_cells": cells,
                        "plane_staging": ("none (FP64)" if p in ("f64", "dropin") else
