@@ -64,9 +64,13 @@ __device__ __forceinline__ GbfPf pf_mulf(GbfPf a, float b) {
   return pf_fast(p.h, p.l);
 }
 __device__ __forceinline__ float pf_rcp(float x) {  // about 1 ulp (PTX rcp.approx)
+#ifdef __CUDACC__
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+#else
+  return 1.f / x;  // the tests' build for the CPU
+#endif
 }
 // a / b
 __device__ __forceinline__ GbfPf pf_div(GbfPf a, GbfPf b) {
@@ -194,11 +198,42 @@ struct GbfPfTables {
   double ex[1 << kPfExpBits];    // 2^(i / 256)
   float2 exp_pf[1 << kPfExpBits];  // the same as a pair
 };
-constexpr double pf_cx_ln(double c) {  // 2 atanh((c - 1) / (c + 1))
-  const double z = (c - 1.0) / (c + 1.0), z2 = z * z;
-  double s = 0.0;
-  for (int k = 41; k >= 1; k -= 2) s = s * z2 + 1.0 / k;
-  return 2.0 * z * s;
+// Sums of two FP64 numbers, for entries rounded once: error-free product by
+// Dekker's splitting, products of two of them to about 2^-104.
+struct GbfDd {
+  double h, l;
+};
+constexpr GbfDd dd_fast(double a, double b) {
+  const double s = a + b;
+  return {s, b - (s - a)};
+}
+constexpr double dd_top(double a) {
+  const double t = 134217729.0 * a;
+  return t - (t - a);
+}
+constexpr GbfDd dd_prod(double a, double b) {
+  const double p = a * b, ah = dd_top(a), al = a - ah, bh = dd_top(b), bl = b - bh;
+  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr GbfDd dd_mul(GbfDd a, GbfDd b) {
+  const GbfDd p = dd_prod(a.h, b.h);
+  return dd_fast(p.h, p.l + (a.h * b.l + a.l * b.h));
+}
+constexpr GbfDd dd_div(double a, double b) {
+  const double q = a / b;
+  const GbfDd p = dd_prod(q, b);
+  return dd_fast(q, ((a - p.h) - p.l) / b);
+}
+// 2 atanh(z), z = (c - 1) / (c + 1), |z| < 0.19: 2 z (1 + z^2 (1/3 + z^2 t)), t
+// in plain FP64 (z^4 < 2^-9). c in 11 bits.
+constexpr double pf_cx_ln(double c) {
+  const GbfDd z = dd_div(c - 1.0, c + 1.0), z2 = dd_mul(z, z);
+  double t = 0.0;
+  for (int k = 41; k >= 5; k -= 2) t = t * z2.h + 1.0 / k;
+  const GbfDd third = dd_div(1.0, 3.0), zt = dd_mul(z2, GbfDd{t, 0.0});
+  const GbfDd u = dd_mul(z2, dd_fast(third.h, third.l + zt.h + zt.l));
+  const GbfDd s = dd_mul(z, dd_fast(1.0, u.h + u.l));
+  return 2.0 * s.h;
 }
 constexpr double pf_cx_exp(double x) {
   double s = 1.0;
@@ -227,7 +262,7 @@ constexpr GbfPfTables pf_make_tables() {
 }
 static __device__ const GbfPfTables g_pf_tab = pf_make_tables();
 
-// x^2 and x^3 / n of a pair x, with the higher terms x^4 (a + b x + ..) in FP32 left to the caller.
+// x^2 and x^3 f of a pair x.
 struct GbfPfPowers {
   float p, pe;  // x^2
   float c, ce;  // x^3 f
@@ -242,8 +277,10 @@ __device__ __forceinline__ GbfPfPowers pf_powers(GbfPf x, GbfPf f) {
   return w;
 }
 
-// ln(1 - om) for 1 - om in (2^-12, 1.37); omf: om in FP32. Error below 2^-52
-// of the larger of ln and ulp(om) / (1 - om). 1 - om = 2^k m, m in [0.6875, 1.375).
+// ln(1 - om) for 1 - om in (2^-12, 1.37); omf: om in FP32. Error below 2^-51 of
+// ln (the entry, r and two sums rounded, the entry up to 1.5 ln; 2^-50.7 for om in
+// (-2^-9, 0), where r is twice as long), in the mean 2^-53.7. 1 - om = 2^k m, m in
+// [0.6875, 1.375).
 template <bool LOW>
 __device__ __forceinline__ double pf_ln1m_k(double om, unsigned tmp) {
   const GbfLnEntry* t = &g_pf_tab.ln[(int)(tmp >> (23 - kPfLnBits)) & ((1 << kPfLnBits) - 1)];
@@ -257,10 +294,11 @@ __device__ __forceinline__ double pf_ln1m_k(double om, unsigned tmp) {
   }
   const double r = __fma_rn(-gbf_f2d(ic.x), om, gbf_f2d(ic.y));  // m / c - 1: nothing cancels as om -> 0
   const GbfPf x = pf_from_double(r);
-  const GbfPfPowers w = pf_powers(x, GbfPf{0.333333343f, -9.93410776e-9f});
-  const float q = __fmul_rn(__fmul_rn(w.p, w.p), __fmaf_rn(x.h, __fmaf_rn(x.h, -0.166666672f, 0.2f), -0.25f));
+  // x^3 (1/3 - x/4 + x^2/5 - x^3/6), the terms beyond 1/3 in the pair's low part
+  const GbfPfPowers w = pf_powers(x, GbfPf{0.333333343f, __fmaf_rn(x.h, __fmaf_rn(x.h, __fmaf_rn(x.h, -0.166666672f, 0.2f), -0.25f),
+                                                                   -9.93410776e-9f)});
   const GbfPf s = pf_fast(__fmul_rn(-0.5f, w.p), w.c);
-  const double corr = pf_to_double(GbfPf{s.h, __fadd_rn(s.l, __fadd_rn(__fmaf_rn(-0.5f, w.pe, w.ce), q))});
+  const double corr = pf_to_double(GbfPf{s.h, __fadd_rn(s.l, __fmaf_rn(-0.5f, w.pe, w.ce))});
   return __dadd_rn(__dadd_rn(lnc, r), corr);
 }
 static __device__ __noinline__ double pf_ln1m_low(double om, unsigned tmp) { return pf_ln1m_k<true>(om, tmp); }
@@ -269,7 +307,7 @@ __device__ __forceinline__ double gbf_ln1m(double om, float omf) {
   return tmp >> 23 ? pf_ln1m_low(om, tmp) : pf_ln1m_k<false>(om, tmp);
 }
 
-// The reduced exponential of 2^u, |u| < 100: 2^u = 2^(n / 256) (1 + e), |e| < 2^-9.5.
+// The reduced exponential of 2^u, |u| < 1000 (2^u a normal number): 2^u = 2^(n / 256) (1 + e), |e| < 2^-9.5.
 struct GbfPfExp {
   GbfPf e;
   int n;
@@ -298,7 +336,8 @@ __device__ __forceinline__ double pf_exp2_scale(int n) {
   const double T = __ldg(&g_pf_tab.ex[n & 255]);
   return __hiloint2double(__double2hiint(T) + (n >> 8) * (1 << 20), __double2loint(T));
 }
-// 2^u and 1 - 2^u in FP64; 2^u as a pair (about 2^-46).
+// 2^u and 1 - 2^u in FP64; 2^u as a pair: 2^-46 and its argument's rounding, |u|
+// 2^-48 (-100 < u < 127: P_k's u is above -0.33 / lambda and below 11 / lambda <= 88).
 __device__ __forceinline__ double gbf_exp2(double u, float uf) {
   const GbfPfExp x = pf_exp2_reduce(u, uf);
   const double T = pf_exp2_scale(x.n);
