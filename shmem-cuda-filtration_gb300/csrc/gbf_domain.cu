@@ -9,28 +9,6 @@
 #include "gbf_f64_pair.cuh"
 #include "gbf_split.h"
 
-GbfDerived gbf_derive(const gbf_model& m) {
-  GbfDerived d;
-  for (int md = 0; md < 2; md++) {
-    const double lam = m.lambda[md], swr = m.S_wr[md];
-    d.inv_1mswr[md] = 1.0 / (1.0 - swr);
-    d.e1[md] = (2. + 3. * lam) / lam;
-    d.e2[md] = (2. + lam) / lam;
-    d.m_inv_lam[md] = -1. / lam;
-    d.inv_lam_1mswr[md] = 1.0 / (lam * (1.0 - swr));
-  }
-  d.neg_inv_mu1 = -1.0 / m.mu1;
-  d.neg_inv_mu2 = -1.0 / m.mu2;
-  d.inv_h1 = 1.0 / m.h1;
-  d.inv_h2 = 1.0 / m.h2;
-  d.inv_h3 = 1.0 / m.h3;
-  d.V = m.h1 * m.h2 * m.h3;
-  d.src = (m.source_mode == GBF_SOURCE_RATE && m.rate_cells > 0)
-              ? m.rate / (double)(m.rate_cells * m.rate_cells) / d.V
-              : 0.0;
-  return d;
-}
-
 int gbf_domain_alloc(gbf_domain* d, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
   if (e != cudaSuccess) {
@@ -43,21 +21,22 @@ int gbf_domain_alloc(gbf_domain* d, void** p, size_t bytes) {
 
 namespace {
 
-int alloc_f64_work(gbf_domain* d) {
+// The work arrays of the model's FP64 step, pair or plain (a drop-in's model
+// can change from one to the other: it then keeps both).
+int prepare_f64_work(gbf_domain* d) {
   const size_t n = gbf_geo(d->m).n, b = n * sizeof(double);
   int s = GBF_OK;
-  if (gbf_pair_applies(d->m)) {
-    s |= gbf_domain_alloc(d, (void**)&d->pair_work, 4 * n * sizeof(float2));
-    s |= gbf_domain_alloc(d, (void**)&d->pair_rows, sizeof(GbfPairRow) * (size_t)d->m.ny);
+  d->pair = gbf_pair_applies(d->m);
+  if (d->pair) {
+    if (!d->pair_work) s |= gbf_domain_alloc(d, (void**)&d->pair_work, 4 * n * sizeof(float2));
+    if (!s && !d->pair_rows) s |= gbf_domain_alloc(d, (void**)&d->pair_rows, sizeof(GbfPairRow) * (size_t)d->m.ny);
     if (!s) s |= gbf_pair_fill_rows(d->m, d->pair_rows, d->stream);
     d->pair_consts.reset(new GbfPairConsts(gbf_pair_consts(d->m)));
     return s ? GBF_ERR_NOMEM : GBF_OK;
   }
-  s |= gbf_domain_alloc(d, (void**)&d->L1, b);
-  s |= gbf_domain_alloc(d, (void**)&d->L2, b);
-  s |= gbf_domain_alloc(d, (void**)&d->ro1, b);
-  s |= gbf_domain_alloc(d, (void**)&d->ro2, b);
-  s |= gbf_domain_alloc(d, (void**)&d->lnSe, b);
+  double** w[] = {&d->L1, &d->L2, &d->ro1, &d->ro2, &d->lnSe};
+  for (double** p : w)
+    if (!*p && !s) s |= gbf_domain_alloc(d, (void**)p, b);
   return s ? GBF_ERR_NOMEM : GBF_OK;
 }
 
@@ -88,10 +67,12 @@ void free_all(gbf_domain* d) {
 // step starts from is first copied to buffer 1, where it stays for the lazily
 // materialised derived arrays (gbf_dropin_materialize).
 int f64_step(gbf_domain* d, int props_flags) {
+  if (d->pair ? !d->pair_rows : !d->lnSe)  // a change of the model that ended without memory
+    if (int s = prepare_f64_work(d)) return s;
   const int nxt = d->cur ^ 1;
   GbfF64Step s = {};
   GbfPairWork pw = {};
-  if (d->pair_work) {
+  if (d->pair) {
     const size_t n = gbf_geo(d->m).n;
     pw.D = d->pair_work;
     pw.L1 = pw.D + n;
@@ -100,7 +81,7 @@ int f64_step(gbf_domain* d, int props_flags) {
     pw.rows = d->pair_rows;
   }
   if (d->borrowed) {
-    if (d->pair_work) {  // pass 1 reads the caller's arrays and leaves the copy
+    if (d->pair) {  // pass 1 reads the caller's arrays and leaves the copy
       pw.P_from = d->P[0];
       pw.S_from = d->S[0];
     } else {
@@ -136,7 +117,7 @@ int f64_step(gbf_domain* d, int props_flags) {
     s.ro1 = d->caller.ro1;
     s.ro2 = d->caller.ro2;
   }
-  int st = gbf_f64_launch_step(d->m, d->d, d->cells, s, d->pair_consts.get(), d->pair_work ? &pw : nullptr, props_flags,
+  int st = gbf_f64_launch_step(d->m, d->d, d->cells, s, d->pair_consts.get(), d->pair ? &pw : nullptr, props_flags,
                                mass_out, d->stream, &d->timer);
   if (st) return st;
   if (d->borrowed)
@@ -194,7 +175,7 @@ int gbf_domain_create(const gbf_model* m, const gbf_cells* host_cells, int preci
       s |= gbf_domain_alloc(d, (void**)&d->P[b], n * sizeof(double));
       s |= gbf_domain_alloc(d, (void**)&d->S[b], n * sizeof(double));
     }
-    if (!s) s = alloc_f64_work(d);
+    if (!s) s = prepare_f64_work(d);
   }
   if (!s && precision != GBF_PREC_F64) s = gbf_split_alloc(d);
   if (s) {
@@ -446,7 +427,7 @@ int gbf_domain_download(gbf_domain* d, int field, double* host) {
   const size_t n = gbf_geo(d->m).n, b = n * sizeof(double);
   if (d->precision != GBF_PREC_F64) return gbf_split_download(d, field, host);
   const double* src = nullptr;
-  if (d->pair_work && (field == GBF_FIELD_RO1 || field == GBF_FIELD_RO2)) {
+  if (d->pair && (field == GBF_FIELD_RO1 || field == GBF_FIELD_RO2)) {
     // the densities of the state the last step started from (the other buffer)
     double* tmp = nullptr;
     GBF_CUDA(cudaMallocAsync((void**)&tmp, b, d->stream));
@@ -525,7 +506,7 @@ int gbf_domain_attach_dropin(const gbf_model* m, gbf_arrays caller, gbf_cells ce
   d->S[0] = caller.S2;
   if (!s) s |= gbf_domain_alloc(d, (void**)&d->P[1], n * sizeof(double));
   if (!s) s |= gbf_domain_alloc(d, (void**)&d->S[1], n * sizeof(double));
-  if (!s) s = precision == GBF_PREC_F64 ? alloc_f64_work(d) : gbf_split_alloc(d);
+  if (!s) s = precision == GBF_PREC_F64 ? prepare_f64_work(d) : gbf_split_alloc(d);
   if (!s) s = gbf_domain_alloc(d, (void**)&d->bscratch, gbf_boundary_scratch_doubles(m) * sizeof(double));
   if (s) {
     free_all(d);
@@ -621,11 +602,9 @@ int gbf_dropin_defer(gbf_domain* d, const gbf_model& m, int stage) {
     if (int s = gbf_dropin_writeback(d)) return s;
     d->m = m;
     d->d = gbf_derive(m);
-    if (d->pair_work) {  // fused mode: its constants and row table
-      *d->pair_consts = gbf_pair_consts(m);
-      if (int s = gbf_pair_fill_rows(m, d->pair_rows, d->stream)) return s;
-    }
-    if (d->precision != GBF_PREC_F64) {  // split mode: its row constants, and the state formed anew
+    if (d->precision == GBF_PREC_F64) {  // fused mode: the step's form, its constants and row table
+      if (int s = prepare_f64_work(d)) return s;
+    } else {  // split mode: its row constants, and the state formed anew
       if (int s = gbf_split_fill_rows(d->m, d->split_rows, d->stream)) return s;
       d->split_stale = true;
       if (gbf_is_defect(gbf_mass_rep(d->precision)))

@@ -19,7 +19,27 @@ struct GbfDerived {
   double src;  // rate-mode source per unit volume [kg/(m^3 s)], 0 otherwise
   double V;    // cell volume
 };
-GbfDerived gbf_derive(const gbf_model& m);
+inline GbfDerived gbf_derive(const gbf_model& m) {
+  GbfDerived d;
+  for (int md = 0; md < 2; md++) {
+    const double lam = m.lambda[md], swr = m.S_wr[md];
+    d.inv_1mswr[md] = 1.0 / (1.0 - swr);
+    d.e1[md] = (2. + 3. * lam) / lam;
+    d.e2[md] = (2. + lam) / lam;
+    d.m_inv_lam[md] = -1. / lam;
+    d.inv_lam_1mswr[md] = 1.0 / (lam * (1.0 - swr));
+  }
+  d.neg_inv_mu1 = -1.0 / m.mu1;
+  d.neg_inv_mu2 = -1.0 / m.mu2;
+  d.inv_h1 = 1.0 / m.h1;
+  d.inv_h2 = 1.0 / m.h2;
+  d.inv_h3 = 1.0 / m.h3;
+  d.V = m.h1 * m.h2 * m.h3;
+  d.src = (m.source_mode == GBF_SOURCE_RATE && m.rate_cells > 0)
+              ? m.rate / (double)(m.rate_cells * m.rate_cells) / d.V
+              : 0.0;
+  return d;
+}
 
 // Props-pass output flags.
 enum { GBF_PF_WRITE_XI_P2 = 1, GBF_PF_WRITE_U = 2 };
@@ -65,7 +85,8 @@ struct gbf_domain {
   double *P[2] = {nullptr, nullptr}, *S[2] = {nullptr, nullptr};
   int cur = 0;
   double *L1 = nullptr, *L2 = nullptr, *ro1 = nullptr, *ro2 = nullptr, *lnSe = nullptr;  // plain FP64 passes
-  // the pair step (gbf_f64_pair.cuh): constants, work arrays, row table
+  // the pair step (gbf_f64_pair.cuh), where the model is one for it: constants, work arrays, row table
+  bool pair = false;
   std::unique_ptr<GbfPairConsts> pair_consts;
   float2* pair_work = nullptr;  // D, L1, L2, P_k: n each
   struct GbfPairRow* pair_rows = nullptr;

@@ -427,17 +427,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_ens_pair_step(const EnsMember* 
   __shared__ EnsMember me;
   const EnsChunk ch = chunks[blockIdx.x];
   ens_copy_member(me, mem + ch.member);
-  const GbfF64Step s = ens_f64_step(me, cur);
-  const GbfPairConsts& C = me.pc64;
+  GbfF64Step s = ens_f64_step(me, cur);
+  s.status = status;
   GbfPairMass acc;
-  unsigned bad = 0;
-  for (unsigned t = ch.begin + threadIdx.x; t < ch.end; t += blockDim.x) {
-    const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
-    const unsigned i = 1u + t - r * C.dix.d, j = 1u + r - q * C.diy.d, k = 1u + q;
-    gbf_pair_step_cell<MASS>(C, me.cells, s, me.pw, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc,
-                             bad);
-  }
-  if (bad) atomicOr(status, GBF_DEV_NONFINITE);
+  gbf_pair_step_cells<MASS>(me.pc64, me.m, me.d, me.cells, s, me.pw, ch.begin + threadIdx.x, blockDim.x, ch.end, acc);
   if (MASS) gbf_block_sum2<kThreads>(acc.m1 - pf_to_double(acc.r1), acc.m2, me.d.V, partials + 2 * blockIdx.x);
 }
 

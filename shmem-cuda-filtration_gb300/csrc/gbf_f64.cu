@@ -68,18 +68,16 @@ __global__ void __launch_bounds__(kThreads, 8) k_pair_props(const GbfPairConsts 
 }
 
 template <bool MASS, int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_pair_step(const GbfPairConsts C, const gbf_cells cells,
-                                                          const GbfF64Step s, const GbfPairWork w, double V) {
+__global__ void __launch_bounds__(NT, 1024 / NT) k_pair_step(const __grid_constant__ GbfPairConsts C,
+                                                          const __grid_constant__ gbf_model m,
+                                                          const __grid_constant__ GbfDerived d,
+                                                          const __grid_constant__ gbf_cells cells,
+                                                          const __grid_constant__ GbfF64Step s,
+                                                          const __grid_constant__ GbfPairWork w) {
   gbf_pdl_begin();
   GbfPairMass acc;
-  unsigned bad = 0;
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < C.nint; t += gridDim.x * blockDim.x) {
-    const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
-    const unsigned i = 1u + t - r * C.dix.d, j = 1u + r - q * C.diy.d, k = 1u + q;
-    gbf_pair_step_cell<MASS>(C, cells, s, w, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc, bad);
-  }
-  if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
-  if (MASS) gbf_block_sum2<NT>(acc.m1 - pf_to_double(acc.r1), acc.m2, V, s.mass_partials + 2 * blockIdx.x);
+  gbf_pair_step_cells<MASS>(C, m, d, cells, s, w, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, C.nint, acc);
+  if (MASS) gbf_block_sum2<NT>(acc.m1 - pf_to_double(acc.r1), acc.m2, d.V, s.mass_partials + 2 * blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kThreads) k_density(double ro0, double beta, double Patm, const double* P,
@@ -119,68 +117,6 @@ unsigned gbf_f64_flux_grid(const gbf_model& m) {
   const size_t nint = (size_t)(m.nx - 2) * (m.ny - 2) * (m.nz - 2);
   const unsigned t = gbf_pair_applies(m) ? pair_threads(gbf_geo(m).n) : (unsigned)kThreads;
   return gbf_grid_for(nint, (int)t, 1024 / (int)t);
-}
-
-GbfPairConsts gbf_pair_consts(const gbf_model& m) {
-  GbfPairConsts C = {};
-  const GbfDerived d = gbf_derive(m);
-  C.nx = m.nx; C.ny = m.ny; C.nz = m.nz;
-  C.noflow = m.bc_mode == GBF_BC_HYDROSTATIC_SIDES;
-  C.pl = (unsigned)m.nx * (unsigned)m.ny;
-  C.n = C.pl * (unsigned)m.nz;
-  C.nint = (unsigned)(m.nx - 2) * (unsigned)(m.ny - 2) * (unsigned)(m.nz - 2);
-  C.dnx = gbf_fast_div((unsigned)m.nx);
-  C.dny = gbf_fast_div((unsigned)m.ny);
-  C.dix = gbf_fast_div((unsigned)m.nx - 2);
-  C.diy = gbf_fast_div((unsigned)m.ny - 2);
-  if (d.src != 0.) {
-    C.rn = m.rate_cells;
-    C.ri0 = m.nx / 2 - m.rate_cells / 2;
-    C.rk0 = m.nz / 2 - m.rate_cells / 2;
-  }
-  C.max_iter = m.newton_iterations;
-  C.Patm = (float)fabs(m.P_atm);
-  // 2^e that brings the water mobility x density of media 0 to about 1
-  int e = 0;
-  const double L = m.K[0] * m.ro01 / m.mu1;
-  if (L > 0. && isfinite(L)) frexp(L, &e);
-  e = e < -60 ? -60 : e > 60 ? 60 : e;
-  const double sc = ldexp(1.0, -e), log2e = 1.4426950408889634074;
-  C.k1 = pf_const(m.ro01 * m.beta1);
-  C.k2 = pf_const(m.ro02 * m.beta2);
-  C.rk1 = pf_const(1.0 / (m.ro01 * m.beta1));
-  C.ro1 = pf_const(m.ro01);
-  C.ro2 = pf_const(m.ro02);
-  C.g1 = pf_const(m.g * m.h2 * m.ro01 * m.beta1);
-  C.g2 = pf_const(m.g * m.h2 * m.ro02 * m.beta2);
-  C.ghd = pf_const(m.g * m.h2 * (m.ro02 - m.ro01));
-  C.wx = pf_const(m.dt / (m.h1 * m.h1) / sc);
-  C.wy = pf_const(m.dt * m.kv / (m.h2 * m.h2) / sc);
-  C.wz = pf_const(m.dt / (m.h3 * m.h3) / sc);
-  C.c1 = pf_const(sc / m.mu1);
-  C.c2 = pf_const(sc / m.mu2);
-  C.dtsrc_d = m.dt * d.src;
-  C.rro2_d = 1.0 / m.ro02;
-  for (int md = 0; md < 2; md++) {
-    C.K[md] = pf_const(m.K[md]);
-    C.phi_d[md] = m.m[md];
-    C.phip[md] = pf_const(m.m[md]);
-    C.rphi[md] = pf_const(1.0 / m.m[md]);
-    C.inv[md] = pf_const(d.inv_1mswr[md]);
-    C.inv_d[md] = d.inv_1mswr[md];
-    C.E1[md] = d.e1[md] * log2e;
-    C.E2[md] = d.e2[md] * log2e;
-    C.E3[md] = d.m_inv_lam[md] * log2e;
-    C.E1f[md] = (float)C.E1[md];
-    C.E2f[md] = (float)C.E2[md];
-    C.E3p[md] = pf_const(C.E3[md]);
-    C.pd[md] = pf_const(m.P_d[md]);
-    C.ilam[md] = pf_const(d.inv_lam_1mswr[md]);
-    for (int n = 1; n <= 4; n++) C.taylor[md][n - 1] = (float)((1.0 / m.lambda[md] + n) / (n + 1));
-  }
-  C.ro1_d = m.ro01; C.ro2_d = m.ro02; C.beta1_d = m.beta1; C.beta2_d = m.beta2; C.Patm_d = m.P_atm;
-  C.k1_d = m.ro01 * m.beta1; C.k2_d = m.ro02 * m.beta2;
-  return C;
 }
 
 int gbf_density_launch(const gbf_model& m, int phase, const double* P, double* out, cudaStream_t st) {
@@ -230,7 +166,7 @@ int gbf_f64_launch_step(const gbf_model& m, const GbfDerived& d, const gbf_cells
     threads = pair_threads(g.n);
     go(threads == 64 ? (mass ? k_pair_step<true, 64> : k_pair_step<false, 64>)
                      : (mass ? k_pair_step<true, kThreads> : k_pair_step<false, kThreads>),
-       fg, *pc, cells, s, *pair, d.V);
+       fg, *pc, m, d, cells, s, *pair);
     threads = kThreads;
   } else {
     go(k_f64_flux_newton, fg, m, d, cells, s);

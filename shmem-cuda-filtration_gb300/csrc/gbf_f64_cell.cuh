@@ -8,28 +8,40 @@
 
 __device__ __forceinline__ int gbf_media_at(const gbf_cells& c, size_t idx) { return c.media ? c.media[idx] : 0; }
 
-// Pass 1 at cell c (every cell): Brooks-Corey kr from one log and two exp
-// (cpu.cpp:57-74), densities, L = Xi ro, ln S_e; optionally the reference's
-// P2/Xi arrays and a2's velocities (cpu.cpp:77-160).
-__device__ __forceinline__ void gbf_f64_props_cell(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells,
-                                                   const GbfF64Step& s, int flags, const GbfGeo& g, size_t c) {
+// Mobilities and densities of a cell with saturation S2 and pressure P1:
+// Brooks-Corey kr from one log and two exp (cpu.cpp:57-74).
+struct GbfF64Props {
+  double Xi1, Xi2, ro1, ro2, lnSe;
+};
+__device__ __forceinline__ GbfF64Props gbf_f64_props(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells,
+                                                     double P1, double S2, size_t c) {
   const int md = gbf_media_at(cells, c);
   const double K = cells.K ? (double)cells.K[c] : m.K[md];
-  const double S2 = s.S[c], P1 = s.P[c];
   const double S_e = (1. - S2 - m.S_wr[md]) / (1. - m.S_wr[md]);  // a division: exactly 1 at S = 0, where kr2 is 0
-  const double l = log(S_e);
-  const double k1 = exp(d.e1[md] * l);
-  const double k2 = (1. - S_e) * (1. - S_e) * (1. - exp(d.e2[md] * l));
-  const double Xi1 = K * k1 * d.neg_inv_mu1;
-  const double Xi2 = K * k2 * d.neg_inv_mu2;
-  const double ro1 = m.ro01 * (1. + m.beta1 * (P1 - m.P_atm));
-  const double ro2 = m.ro02 * (1. + m.beta2 * (P1 - m.P_atm));  // P2 = P1 (P_k = 0, cpu.cpp:63)
+  GbfF64Props q;
+  q.lnSe = log(S_e);
+  const double k1 = exp(d.e1[md] * q.lnSe);
+  const double k2 = (1. - S_e) * (1. - S_e) * (1. - exp(d.e2[md] * q.lnSe));
+  q.Xi1 = K * k1 * d.neg_inv_mu1;
+  q.Xi2 = K * k2 * d.neg_inv_mu2;
+  q.ro1 = m.ro01 * (1. + m.beta1 * (P1 - m.P_atm));
+  q.ro2 = m.ro02 * (1. + m.beta2 * (P1 - m.P_atm));  // P2 = P1 (P_k = 0, cpu.cpp:63)
+  return q;
+}
+
+// Pass 1 at cell c (every cell): densities, L = Xi ro, ln S_e; optionally the
+// reference's P2/Xi arrays and a2's velocities (cpu.cpp:77-160).
+__device__ __forceinline__ void gbf_f64_props_cell(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells,
+                                                   const GbfF64Step& s, int flags, const GbfGeo& g, size_t c) {
+  const double P1 = s.P[c];
+  const GbfF64Props q = gbf_f64_props(m, d, cells, P1, s.S[c], c);
+  const double Xi1 = q.Xi1, Xi2 = q.Xi2, ro1 = q.ro1, ro2 = q.ro2;
   if (s.L1) {  // NULL: only the outputs below (beside the pair step)
     s.L1[c] = Xi1 * ro1;
     s.L2[c] = Xi2 * ro2;
     s.ro1[c] = ro1;
     s.ro2[c] = ro2;
-    s.lnSe[c] = l;
+    s.lnSe[c] = q.lnSe;
   }
   if (flags & GBF_PF_WRITE_XI_P2) {
     s.Xi1[c] = Xi1;
@@ -111,39 +123,44 @@ __device__ __forceinline__ void gbf_f64_newton(const gbf_model& m, const GbfDeri
   }
 }
 
-// Pass 2 at interior cell (i, j, k): face fluxes with gravity and the mass
-// update (cpu.cpp:218-291), then the Newton step; writes the next state.
-// Adds phi * A to the mass sums and flags non-finite results.
-__device__ __forceinline__ void gbf_f64_flux_newton_cell(const gbf_model& m, const GbfDerived& d,
-                                                         const gbf_cells& cells, const GbfF64Step& s,
-                                                         const GbfGeo& g, int i, int j, int k, double& msum1,
-                                                         double& msum2, unsigned& bad) {
+// Face potentials of a cell (P2 = P1 in the flux step), and a phase's flux
+// divergence: L of the cell and its neighbours (own, x -, +, y -, +, z -, +),
+// rg = rho g.
+struct GbfF64Faces {
+  double x1, x2, y1, y2, z1, z2;  // without gravity
+};
+__device__ __forceinline__ GbfF64Faces gbf_f64_faces(const GbfDerived& d, const double* P, size_t c, size_t nx, size_t pl) {
+  const double Pc = P[c];
+  return {(P[c - 1] - Pc) * d.inv_h1,  (Pc - P[c + 1]) * d.inv_h1,  (P[c - nx] - Pc) * d.inv_h2,
+          (Pc - P[c + nx]) * d.inv_h2, (P[c - pl] - Pc) * d.inv_h3, (Pc - P[c + pl]) * d.inv_h3};
+}
+__device__ __forceinline__ double gbf_f64_divergence(const gbf_model& m, const GbfDerived& d, const GbfF64Faces& f,
+                                                     double rg, bool noflow_bottom, const double (&L)[7]) {
+  const double y1 = f.y1 + rg, y2 = noflow_bottom ? 0. : f.y2 + rg;
+  return gbf_donor(f.x1, f.x2, L[0], L[1], L[2]) * d.inv_h1 +
+         m.kv * gbf_donor(y1, y2, L[0], L[3], L[4]) * d.inv_h2 +
+         gbf_donor(f.z1, f.z2, L[0], L[5], L[6]) * d.inv_h3;
+}
+// What pass 2 takes of pass 1.
+struct GbfF64Stencil {
+  double L1[7], L2[7], ro1, ro2, lnSe;
+};
+// Interior cell (i, j, k): face fluxes with gravity and the mass update
+// (cpu.cpp:218-291), then the Newton step; writes the next state. Adds phi * A
+// to the mass sums and flags non-finite results.
+__device__ __forceinline__ void gbf_f64_cell_update(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells,
+                                                    const GbfF64Step& s, const GbfGeo& g, int i, int j, int k,
+                                                    const GbfF64Stencil& q, double& msum1, double& msum2,
+                                                    unsigned& bad) {
   const size_t c = gbf_idx(g, i, j, k), nx = g.nx, pl = g.pl;
   const bool noflow_bottom = (m.bc_mode == GBF_BC_HYDROSTATIC_SIDES) && (j == g.ny - 2);
   const int md = gbf_media_at(cells, c);
   const double phi = cells.phi ? (double)cells.phi[c] : m.m[md];
-  const double* P = s.P;
-  const double Pc = P[c];
-  // face potentials (P2 = P1 in the flux step)
-  const double x1 = (P[c - 1] - Pc) * d.inv_h1, x2 = (Pc - P[c + 1]) * d.inv_h1;
-  const double yb1 = (P[c - nx] - Pc) * d.inv_h2, yb2 = (Pc - P[c + nx]) * d.inv_h2;
-  const double z1 = (P[c - pl] - Pc) * d.inv_h3, z2 = (Pc - P[c + pl]) * d.inv_h3;
-  const double ro1 = s.ro1[c], ro2 = s.ro2[c];
-  const double rg1 = ro1 * m.g, rg2 = ro2 * m.g;
-  const double y1_1 = yb1 + rg1, y1_2 = yb1 + rg2;
-  const double y2_1 = noflow_bottom ? 0. : yb2 + rg1;
-  const double y2_2 = noflow_bottom ? 0. : yb2 + rg2;
-  const double* L1 = s.L1;
-  const double* L2 = s.L2;
-  const double L1c = L1[c], L2c = L2[c];
-  const double f = gbf_donor(x1, x2, L1c, L1[c - 1], L1[c + 1]) * d.inv_h1 +
-                   m.kv * gbf_donor(y1_1, y2_1, L1c, L1[c - nx], L1[c + nx]) * d.inv_h2 +
-                   gbf_donor(z1, z2, L1c, L1[c - pl], L1[c + pl]) * d.inv_h3;
-  const double gsum = gbf_donor(x1, x2, L2c, L2[c - 1], L2[c + 1]) * d.inv_h1 +
-                      m.kv * gbf_donor(y1_2, y2_2, L2c, L2[c - nx], L2[c + nx]) * d.inv_h2 +
-                      gbf_donor(z1, z2, L2c, L2[c - pl], L2[c + pl]) * d.inv_h3;
+  const GbfF64Faces faces = gbf_f64_faces(d, s.P, c, nx, pl);
+  const double f = gbf_f64_divergence(m, d, faces, q.ro1 * m.g, noflow_bottom, q.L1);
+  const double gsum = gbf_f64_divergence(m, d, faces, q.ro2 * m.g, noflow_bottom, q.L2);
   const double S2 = s.S[c];
-  const double roS1 = ro1 * (1. - S2), roS2 = ro2 * S2;
+  const double roS1 = q.ro1 * (1. - S2), roS2 = q.ro2 * S2;
   const double dtphi = m.dt / phi;
   const double A1 = roS1 - dtphi * f;
   double A2 = roS2 - dtphi * gsum;
@@ -156,11 +173,24 @@ __device__ __forceinline__ void gbf_f64_flux_newton_cell(const gbf_model& m, con
   }
   msum1 += phi * A1;
   msum2 += phi * A2;
-  double Pn = Pc, Sn = S2;
-  gbf_f64_newton(m, d, md, s.lnSe[c], A1, A2, Pn, Sn);
+  double Pn = s.P[c], Sn = S2;
+  gbf_f64_newton(m, d, md, q.lnSe, A1, A2, Pn, Sn);
   if (!isfinite(Pn) || !isfinite(Sn)) bad = 1;
   s.Pn[c] = Pn;
   s.Sn[c] = Sn;
+}
+
+// Pass 2 at interior cell (i, j, k).
+__device__ __forceinline__ void gbf_f64_flux_newton_cell(const gbf_model& m, const GbfDerived& d,
+                                                         const gbf_cells& cells, const GbfF64Step& s,
+                                                         const GbfGeo& g, int i, int j, int k, double& msum1,
+                                                         double& msum2, unsigned& bad) {
+  const size_t c = gbf_idx(g, i, j, k), nx = g.nx, pl = g.pl;
+  const double *L1 = s.L1, *L2 = s.L2;
+  const GbfF64Stencil q = {{L1[c], L1[c - 1], L1[c + 1], L1[c - nx], L1[c + nx], L1[c - pl], L1[c + pl]},
+                           {L2[c], L2[c - 1], L2[c + 1], L2[c - nx], L2[c + nx], L2[c - pl], L2[c + pl]},
+                           s.ro1[c], s.ro2[c], s.lnSe[c]};
+  gbf_f64_cell_update(m, d, cells, s, g, i, j, k, q, msum1, msum2, bad);
 }
 
 // Face pass at boundary cell number t (gbf_boundary_cell order).

@@ -13,13 +13,22 @@
 //     gravity and the hydrostatic gradient cancel before any rounding;
 //   * 1 - S_e = S / (1 - S_wr) and ln S_e = ln(1 - .) are taken without
 //     forming S_e, so kr2 keeps its relative accuracy as S -> 0.
-// An increment is then accurate to about 2^-45 of itself, and P + dP, S + dS
+// An increment is then accurate to about 2^-46 of itself, and P + dP, S + dS
 // are rounded once in FP64. The arithmetic that forms masses of 1000 kg/m^3 in
-// FP64 and recovers P through rho0 beta from their rounding (1e-13) loses more:
-// the error against 64-bit increments is 1e-12 of P there and 1e-16 here.
+// FP64 and recovers P through rho0 beta from their rounding loses about
+// 2^-53 / beta1 of P: with beta1 = 1e-9 and P near hydrostatic the error against
+// 64-bit increments is 8e-13 of P there and 4e-17 here. Cells that pairs do not
+// hold are refused, and taken again in FP64 (pair_cell_again):
+//   * S_e below 2^-11, capillary pressure above a limit (`ratio` in
+//     pair_newton), and a Newton that 7 iterations do not end. The limit keeps P_k
+//     and its slope in FP32's range and the Newton's convergence quadratic: near
+//     residual water the reference's 7 iterations stop before they converge, and
+//     what they leave is the result.
+// S below about 1e-13 has no mobility in pairs (om^3 is below FP32's range; in
+// FP64 it would move 1e-26 of itself a step).
 #pragma once
 
-#include "gbf_domain.h"
+#include "gbf_f64_cell.cuh"
 #include "gbf_pair.cuh"
 
 // A row's constants: P_hs(j), P_hs(j) - P_atm as a pair, and what rounding
@@ -51,7 +60,6 @@ struct GbfPairConsts {
   unsigned pl, n, nint;
   GbfFastDiv dnx, dny, dix, diy;
   int ri0, rk0, rn;  // rate source cells (rn = 0: none)
-  int max_iter;
   float Patm;
   GbfPf k1, k2, rk1;     // rho01 beta1, rho02 beta2, 1 / (rho01 beta1)
   GbfPf ro1, ro2;        // rho01, rho02
@@ -59,17 +67,89 @@ struct GbfPairConsts {
   GbfPf wx, wy, wz;      // dt / h1^2, dt kv / h2^2, dt / h3^2 (over the scale)
   GbfPf c1, c2;          // 1 / mu (times the scale)
   GbfPf K[2], phip[2], rphi[2], inv[2], E3p[2], pd[2], ilam[2];
-  double phi_d[2], inv_d[2], E1[2], E2[2], E3[2];  // 1 / (1 - S_wr); Brooks-Corey exponents over ln 2
+  double phi_d[2], inv_d[2], E1[2], E2[2];  // 1 / (1 - S_wr); Brooks-Corey exponents over ln 2
   float E1f[2], E2f[2];
   float taylor[2][4];    // (1 / lambda + n) / (n + 1), n = 1..4
   double ro1_d, ro2_d, beta1_d, beta2_d, Patm_d, k1_d, k2_d;  // the densities' constants
   double dtsrc_d, rro2_d;  // dt x the rate source per volume, 1 / rho02
 };
-GbfPairConsts gbf_pair_consts(const gbf_model& m);
-// The pair step solves the Newton's equations to round-off. The reference's 7
-// iterations (and more) do too; a model that asks for fewer stops before, and
-// keeps the plain FP64 passes (gbf_f64_cell.cuh).
-inline bool gbf_pair_applies(const gbf_model& m) { return m.newton_iterations >= 7; }
+inline GbfPairConsts gbf_pair_consts(const gbf_model& m) {
+  GbfPairConsts C = {};
+  const GbfDerived d = gbf_derive(m);
+  C.nx = m.nx; C.ny = m.ny; C.nz = m.nz;
+  C.noflow = m.bc_mode == GBF_BC_HYDROSTATIC_SIDES;
+  C.pl = (unsigned)m.nx * (unsigned)m.ny;
+  C.n = C.pl * (unsigned)m.nz;
+  C.nint = (unsigned)(m.nx - 2) * (unsigned)(m.ny - 2) * (unsigned)(m.nz - 2);
+  C.dnx = gbf_fast_div((unsigned)m.nx);
+  C.dny = gbf_fast_div((unsigned)m.ny);
+  C.dix = gbf_fast_div((unsigned)m.nx - 2);
+  C.diy = gbf_fast_div((unsigned)m.ny - 2);
+  if (d.src != 0.) {
+    C.rn = m.rate_cells;
+    C.ri0 = m.nx / 2 - m.rate_cells / 2;
+    C.rk0 = m.nz / 2 - m.rate_cells / 2;
+  }
+  C.Patm = (float)fabs(m.P_atm);
+  // 2^e that brings the water mobility x density of media 0 to about 1
+  int e = 0;
+  const double L = m.K[0] * m.ro01 / m.mu1;
+  if (L > 0. && isfinite(L)) frexp(L, &e);
+  e = e < -60 ? -60 : e > 60 ? 60 : e;
+  const double sc = ldexp(1.0, -e), log2e = 1.4426950408889634074;
+  C.k1 = pf_const(m.ro01 * m.beta1);
+  C.k2 = pf_const(m.ro02 * m.beta2);
+  C.rk1 = pf_const(1.0 / (m.ro01 * m.beta1));
+  C.ro1 = pf_const(m.ro01);
+  C.ro2 = pf_const(m.ro02);
+  C.g1 = pf_const(m.g * m.h2 * m.ro01 * m.beta1);
+  C.g2 = pf_const(m.g * m.h2 * m.ro02 * m.beta2);
+  C.ghd = pf_const(m.g * m.h2 * (m.ro02 - m.ro01));
+  C.wx = pf_const(m.dt / (m.h1 * m.h1) / sc);
+  C.wy = pf_const(m.dt * m.kv / (m.h2 * m.h2) / sc);
+  C.wz = pf_const(m.dt / (m.h3 * m.h3) / sc);
+  C.c1 = pf_const(sc / m.mu1);
+  C.c2 = pf_const(sc / m.mu2);
+  C.dtsrc_d = m.dt * d.src;
+  C.rro2_d = 1.0 / m.ro02;
+  for (int md = 0; md < 2; md++) {
+    C.K[md] = pf_const(m.K[md]);
+    C.phi_d[md] = m.m[md];
+    C.phip[md] = pf_const(m.m[md]);
+    C.rphi[md] = pf_const(1.0 / m.m[md]);
+    C.inv[md] = pf_const(d.inv_1mswr[md]);
+    C.inv_d[md] = d.inv_1mswr[md];
+    C.E1[md] = d.e1[md] * log2e;
+    C.E2[md] = d.e2[md] * log2e;
+    C.E1f[md] = (float)C.E1[md];
+    C.E2f[md] = (float)C.E2[md];
+    C.E3p[md] = pf_const(d.m_inv_lam[md] * log2e);
+    C.pd[md] = pf_const(m.P_d[md]);
+    C.ilam[md] = pf_const(d.inv_lam_1mswr[md]);
+    for (int n = 1; n <= 4; n++) C.taylor[md][n - 1] = (float)((1.0 / m.lambda[md] + n) / (n + 1));
+  }
+  C.ro1_d = m.ro01; C.ro2_d = m.ro02; C.beta1_d = m.beta1; C.beta2_d = m.beta2; C.Patm_d = m.P_atm;
+  C.k1_d = m.ro01 * m.beta1; C.k2_d = m.ro02 * m.beta2;
+  return C;
+}
+// Models of the pair step. It solves the Newton's equations to round-off, as
+// the reference's 7 iterations (and more) do; a model that asks for fewer stops
+// before, and keeps the plain FP64 passes (gbf_f64_cell.cuh). So does one whose
+// constants, or the exponents of 2 that S_e >= 2^-11 gives (11 / lambda in P_k),
+// are too near the ends of FP32's range for products of two or three of them
+// and the low parts of their pairs.
+inline bool gbf_pair_applies(const gbf_model& m) {
+  auto fits = [](double x) { return fabs(x) >= 0x1p-40 && fabs(x) <= 0x1p40; };
+  const GbfDerived d = gbf_derive(m);
+  bool ok = m.newton_iterations >= 7 && fits(m.ro01) && fits(m.ro02) && fits(m.ro01 * m.beta1) && m.beta1 > 0. &&
+            fits(1. / m.beta1) && (m.beta2 == 0. || fits(m.ro02 * m.beta2)) && (m.g == 0. || fits(m.g * m.h2)) &&
+            fits(m.dt / (m.h1 * m.h1) / m.mu1) && fits(m.dt * m.kv / (m.h2 * m.h2) / m.mu1) &&
+            fits(m.dt / (m.h3 * m.h3) / m.mu1) && fits(m.mu1) && fits(m.mu2) && fabs(m.P_atm) <= 0x1p40;
+  for (int md = 0; md < 2; md++)
+    ok = ok && m.lambda[md] >= 0.125 && m.lambda[md] <= 1024. && d.inv_1mswr[md] <= 0x1p10 && fits(m.m[md]) &&
+         m.P_d[md] <= 0x1p40 && m.K[md] >= 0. && m.K[md] <= 0x1p40;
+  return ok;
+}
 // Fill rows[0, ny) for the model (stream-ordered on st).
 int gbf_pair_fill_rows(const gbf_model& m, GbfPairRow* rows, cudaStream_t st);
 
@@ -90,18 +170,19 @@ __device__ __forceinline__ void pf_st(float2* p, GbfPf a) { *p = make_float2(a.h
 
 // Brooks-Corey functions of om = 1 - S_e = S / (1 - S_wr): kr1 = S_e^e1, w =
 // 1 - S_e^e2 (kr2 = om^2 w) and P_k / P_d = S_e^(-1/lambda). Beyond the
-// tables' range (S_e <= 2^-11, S far below 0, NaN) they come from CUDA's
-// functions, with the FP64 passes' limits (S_e = 0: kr1 = 0, P_k infinite;
-// S_e < 0: NaN).
+// tables' range (S_e <= 2^-11, S far below 0, NaN) the mobilities come from
+// CUDA's functions, with the FP64 passes' limits (S_e = 0: kr1 = 0; S_e < 0:
+// NaN), and P_k is infinite, which sends the cell itself to pair_cell_f64.
 __device__ __forceinline__ bool pair_om_ok(float om) { return om < 0.9995f && om > -0.25f; }
 static __device__ __noinline__ double pair_pow_general(double om, double E) {
   return exp2(E * log(1.0 - om));
 }
+__device__ __forceinline__ GbfPf pair_pk_none() { return {__uint_as_float(0x7f800000u), 0.f}; }
 // P_k(S) (rare: the Newton's changes of S beyond its expansion's range).
 static __device__ __noinline__ GbfPf pair_pk(const GbfPairConsts& C, int md, GbfPf S) {
   const double om = __dmul_rn(pf_to_double(S), C.inv_d[md]);
   const float omf = pf_from_double(om).h;
-  if (!pair_om_ok(omf)) return pf_mul(C.pd[md], pf_from_double(pair_pow_general(om, C.E3[md])));
+  if (!pair_om_ok(omf)) return pair_pk_none();
   return pf_mul(C.pd[md], pf_exp2(pf_mul(pf_from_double(gbf_ln1m(om, omf)), C.E3p[md])));
 }
 
@@ -146,7 +227,7 @@ __device__ __forceinline__ void gbf_pair_props_cell(const GbfPairConsts& C, cons
     } else {
       kr1 = pf_from_double(pair_pow_general(om, C.E1[md]));
       w2 = pf_from_double(1.0 - pair_pow_general(om, C.E2[md]));
-      pk = pf_mul(pk, pf_from_double(pair_pow_general(om, C.E3[md])));
+      pk = pair_pk_none();
     }
     l1 = pf_mul(l1, kr1);
     l2 = pf_mul(pf_mul(over_mu(C.c2), pf_mul(pf_mul(omp, omp), w2)), pf_add(C.ro2, pf_mul_raw(C.k2, Pp)));
@@ -211,8 +292,11 @@ static __device__ __noinline__ void pair_mass_arrays(const GbfPairConsts& C, con
 //   r2 + k2 (dp + P_k(S + ds) - P_k(S)) (S + ds) + rho2 ds = 0, rho2 at P + P_k(S),
 // r2 with the k2 P_k S that the targets leave out (cpu.cpp:63 vs :306).
 // The Jacobian and its inverse are FP32, the residual pairs: a step leaves
-// 2^-21 of itself, so two or three reach round-off.
-__device__ __forceinline__ void pair_newton(const GbfPairConsts& C, int md, GbfPf Pp, GbfPf S, GbfPf Pk, GbfPf r1,
+// 2^-21 of itself, so two or three reach round-off, and it ends there whatever
+// newton_tol is (an end at newton_tol = 1e-11 errs by 1.7e-16 of P where this
+// one errs by 8e-17). False: it did not, or the cell is none for pairs (see the
+// top of this file).
+__device__ __forceinline__ bool pair_newton(const GbfPairConsts& C, int md, GbfPf Pp, GbfPf S, GbfPf Pk, GbfPf r1,
                                             GbfPf r2, GbfPf& dp, GbfPf& ds) {
   const GbfPf rho1 = pf_add(C.ro1, pf_mul_raw(C.k1, Pp));
   const GbfPf rho2 = pf_add(C.ro2, pf_mul_raw(C.k2, pf_add(Pp, Pk)));
@@ -220,30 +304,32 @@ __device__ __forceinline__ void pair_newton(const GbfPairConsts& C, int md, GbfP
   const GbfPf Se = pf_sub(GbfPf{1.f, 0.f}, pf_mul(S, C.inv[md]));
   r2 = pf_add(r2, pf_mul(pf_mul(C.k2, Pk), S));
   const GbfPf slope = pf_div(pf_mul(Pk, C.ilam[md]), Se);  // dP_k/dS
-  const float rSe = pf_rcp(Se.h);
+  const float rSe = __fmul_rn(C.inv[md].h, pf_rcp(Se.h));  // relative change of S_e per change of S
   float J11 = __fmul_rn(C.k1.h, omS.h), mJ12 = rho1.h, J21 = __fmul_rn(C.k2.h, S.h);
-  const float share = __fmul_rn(J21, slope.h);
+  const float share = __fmul_rn(J21, slope.h), rrho2 = pf_rcp(rho2.h);
   float J22 = __fadd_rn(rho2.h, share);
   float inv = pf_rcp(__fmaf_rn(J11, J22, __fmul_rn(mJ12, J21)));
-  const float ratio = fabsf(__fmul_rn(share, pf_rcp(rho2.h)));  // the capillary term's part of J22
+  const float ratio = fabsf(__fmul_rn(share, rrho2));  // the capillary term's part of J22
+  // what the pairs' 2^-46 of P_k leave of S is below 2^-54 with ratio <= 2^-8
+  if (!(ratio <= 3.90625e-3f)) return false;
+  const float rb = fmaxf(__fmul_rn(C.k1.h, pf_rcp(rho1.h)), fabsf(__fmul_rn(C.k2.h, rrho2)));  // of the densities, per change of P
   GbfPf G1 = r1, G2 = r2;
-  for (int it = 0;; it++) {
+  for (int it = 0; it < 7; it++) {
     const float ep = -__fmul_rn(inv, __fmaf_rn(J22, G1.h, __fmul_rn(mJ12, G2.h)));
     const float es = -__fmul_rn(inv, __fmaf_rn(J11, G2.h, -__fmul_rn(J21, G1.h)));
     dp = it ? pf_addf(dp, ep) : GbfPf{ep, 0.f};
     ds = it ? pf_addf(ds, es) : GbfPf{es, 0.f};
-    const float x = __fmul_rn(__fmul_rn(ds.h, C.inv[md].h), rSe);  // relative change of S_e
-    if (it > 0) {
-      // what the step leaves: the Jacobian's error (2^-21) or its change over the increments,
-      // of the step; small enough once below 2^-54 of S and of P
-      const float q = fmaxf(4.77e-7f, it > 1 ? 0.f : __fmul_rn(8.f, fabsf(x)));
-      const float lim_s = __fmul_rn(5.55e-17f, fabsf(__fadd_rn(S.h, ds.h)));
-      const float lim_p = __fmul_rn(5.55e-17f, __fadd_rn(fabsf(Pp.h), C.Patm));
-      const bool done =
-          (__fmul_rn(q, fabsf(es)) <= lim_s || fabsf(es) <= __fmul_rn(2.8e-14f, fabsf(ds.h))) &&
-          (__fmul_rn(q, fabsf(ep)) <= lim_p || fabsf(ep) <= __fmul_rn(2.8e-14f, fabsf(dp.h)));
-      if (done || it + 1 >= C.max_iter || !(fabsf(ep) < 3e38f && fabsf(es) < 3e38f)) break;
-    }
+    const float x = __fmul_rn(ds.h, rSe);  // relative change of S_e
+    if (!(fabsf(x) <= 0.5f)) return false;
+    // what the step leaves: the Jacobian's error (2^-21) or its change since the point it was formed
+    // at, of the step; small enough once below 2^-54 of S and of P
+    const float chg = it > 1 ? __fmaf_rn(fabsf(ep), rb, fabsf(__fmul_rn(es, rSe))) : __fmaf_rn(fabsf(dp.h), rb, fabsf(x));
+    const float q = fmaxf(4.77e-7f, __fmul_rn(8.f, chg));
+    const float Pa = __fadd_rn(fabsf(Pp.h), C.Patm);
+    const float lim_s = __fmul_rn(5.55e-17f, fabsf(__fadd_rn(S.h, ds.h))), lim_p = __fmul_rn(5.55e-17f, Pa);
+    if ((__fmul_rn(q, fabsf(es)) <= lim_s || fabsf(es) <= __fmul_rn(2.8e-14f, fabsf(ds.h))) &&
+        (__fmul_rn(q, fabsf(ep)) <= lim_p || fabsf(ep) <= __fmul_rn(2.8e-14f, fabsf(dp.h))))
+      return true;
     // residual at the new point
     const GbfPf omn = pf_sub(omS, ds), Sn = pf_add(S, ds);
     GbfPf dPk;
@@ -270,12 +356,56 @@ __device__ __forceinline__ void pair_newton(const GbfPairConsts& C, int md, GbfP
       inv = pf_rcp(__fmaf_rn(J11, J22, __fmul_rn(mJ12, J21)));
     }
   }
+  return false;
 }
+
+// The plain FP64 step of one cell (gbf_f64_cell.cuh), its stencil's mobilities
+// formed here since no pass keeps them in FP64. Returns its part of the masses.
+static __device__ __noinline__ double2 pair_cell_f64(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells,
+                                                     const GbfF64Step& s, int i, int j, int k) {
+#ifdef GBF_COUNT_FP64_CELL
+  GBF_COUNT_FP64_CELL;  // the tests' build for the CPU
+#endif
+  const GbfGeo g = gbf_geo(m);
+  const size_t c = gbf_idx(g, i, j, k);
+  GbfF64Stencil q;
+  double S[7], P[7];
+  auto at = [&](int t) {
+    const size_t st = t < 3 ? 1 : t < 5 ? (size_t)g.nx : g.pl;
+    return t == 0 ? c : (t & 1) ? c - st : c + st;
+  };
+#pragma unroll
+  for (int t = 0; t < 7; t++) {
+    S[t] = s.S[at(t)];
+    P[t] = s.P[at(t)];
+  }
+#pragma unroll 1
+  for (int t = 0; t < 7; t++) {
+    const GbfF64Props p = gbf_f64_props(m, d, cells, P[t], S[t], at(t));
+    q.L1[t] = p.Xi1 * p.ro1;
+    q.L2[t] = p.Xi2 * p.ro2;
+    if (t == 0) {
+      q.ro1 = p.ro1;
+      q.ro2 = p.ro2;
+      q.lnSe = p.lnSe;
+    }
+  }
+  double m1 = 0., m2 = 0.;
+  unsigned bad = 0;
+  gbf_f64_cell_update(m, d, cells, s, g, i, j, k, q, m1, m2, bad);
+  if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
+  return make_double2(m1, m2);
+}
+// What stands in S of the next state at a cell that the pairs refused until it
+// is taken again: a NaN of its own.
+constexpr int kPairRefused = 0x7ffaf64c;
+__device__ __forceinline__ double pair_refused() { return __hiloint2double(kPairRefused, 0); }
 
 // Pass 2 at interior cell (i, j, k) = c: fluxes, Newton, next state (the
 // water-only form where no DNAPL is in the cell or flows through its faces).
+// False, and a mark left in S: not a cell for pairs (see the top of this file).
 template <bool MASS>
-__device__ __forceinline__ void gbf_pair_step_cell(const GbfPairConsts& C, const gbf_cells& cells,
+__device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const gbf_cells& cells,
                                                    const GbfF64Step& s, const GbfPairWork& w, int i, int j, int k,
                                                    unsigned c, GbfPairMass& acc, unsigned& bad) {
   const unsigned nx = (unsigned)C.nx, pl = C.pl;
@@ -315,8 +445,8 @@ __device__ __forceinline__ void gbf_pair_step_cell(const GbfPairConsts& C, const
   const GbfPf Lzm = pf_ld(w.L2 + c - pl), Lzp = pf_ld(w.L2 + c + pl);
   const bool dnapl = !gbf_is_zero(Sd) || src || Lc.h != 0.f || Lxm.h != 0.f || Lxp.h != 0.f || Lyu.h != 0.f ||
                      Lyd.h != 0.f || Lzm.h != 0.f || Lzp.h != 0.f;
-  if (MASS) acc.r1 = pf_add(acc.r1, cells.phi ? pf_mulf(r1, phif) : pf_mul(r1, C.phip[md]));
   double Sn;
+  bool ok;
   GbfPf dp, r2 = zero;
   if (dnapl) {
     const GbfPf G = pf_add(pf_mul(C.g2, Pp), C.ghd);
@@ -328,11 +458,11 @@ __device__ __forceinline__ void gbf_pair_step_cell(const GbfPairConsts& C, const
     double rest = 0.;  // what the pair r2 leaves of the source
     if (src) r2 = pf_sub(r2, pair_source(C.dtsrc_d, cells.phi ? gbf_f2d(phif) : C.phi_d[md], rest));
     GbfPf ds;
-    pair_newton(C, md, Pp, pf_from_double(Sd), gbf_is_zero(Sd) ? C.pd[md] : pf_ld(w.Pk + c), r1, r2, dp, ds);
+    ok = pair_newton(C, md, Pp, pf_from_double(Sd), gbf_is_zero(Sd) ? C.pd[md] : pf_ld(w.Pk + c), r1, r2, dp, ds);
     const double dsd = pf_to_double(ds);
     Sn = __dadd_rn(Sd, dsd);
     if (src) Sn = pair_add_rest(Sd, dsd, rest, C.rro2_d);
-    if (MASS) {
+    if (MASS && ok) {
       const double phi = cells.phi ? gbf_f2d(phif) : C.phi_d[md];
       const double pa = __dsub_rn(Pd, C.Patm_d), q1 = __fma_rn(C.k1_d, pa, C.ro1_d);
       acc.m1 = __fma_rn(phi, __fma_rn(-q1, Sd, q1), acc.m1);
@@ -341,14 +471,57 @@ __device__ __forceinline__ void gbf_pair_step_cell(const GbfPairConsts& C, const
   } else {
     dp = pf_neg(pf_mul(r1, C.rk1));  // rho01 beta1 dP = -r1
     Sn = Sd;
-    if (MASS) {
+    ok = true;
+    if (MASS && ok) {
       const double phi = cells.phi ? gbf_f2d(phif) : C.phi_d[md];
       acc.m1 = __fma_rn(phi, __fma_rn(C.k1_d, __dsub_rn(Pd, C.Patm_d), C.ro1_d), acc.m1);
     }
   }
+  if (!ok) {
+    s.Sn[c] = pair_refused();
+    return false;
+  }
+  if (MASS) acc.r1 = pf_add(acc.r1, cells.phi ? pf_mulf(r1, phif) : pf_mul(r1, C.phip[md]));
   if (s.roS1) pair_mass_arrays(C, s, c, Pd, Sd, r1, r2);
   const double Pn = __dadd_rn(Pd, pf_to_double(dp));
   if (!gbf_is_finite(Pn) || !gbf_is_finite(Sn)) bad = 1;
   s.Pn[c] = Pn;
   s.Sn[c] = Sn;
+  return true;
+}
+
+// A cell, if gbf_pair_step_cell refused it; its part of the masses.
+static __device__ __noinline__ double2 pair_cell_again(const GbfPairConsts& C, const gbf_model& m, const GbfDerived& d,
+                                                       const gbf_cells& cells, const GbfF64Step& s, unsigned t) {
+  const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
+  const int i = (int)(1u + t - r * C.dix.d), j = (int)(1u + r - q * C.diy.d), k = (int)(1u + q);
+  const unsigned c = (unsigned)i + (unsigned)j * (unsigned)C.nx + (unsigned)k * C.pl;
+  if (__double2hiint(s.Sn[c]) != kPairRefused) return make_double2(0., 0.);
+  return pair_cell_f64(m, d, cells, s, i, j, k);
+}
+// Pass 2 at interior cells t0, t0 + stride, .. below t1, summed into acc. The
+// cells that the pairs refuse are taken after the others: calls among the pair
+// arithmetic cost it registers (256^3, none refused: pass 2 488 us with them there,
+// 466 after the others).
+template <bool MASS>
+__device__ __forceinline__ void gbf_pair_step_cells(const GbfPairConsts& C, const gbf_model& m, const GbfDerived& d,
+                                                    const gbf_cells& cells, const GbfF64Step& s, const GbfPairWork& w,
+                                                    unsigned t0, unsigned stride, unsigned t1, GbfPairMass& acc) {
+  unsigned bad = 0, first = t1, last = 0;  // of the refused cells
+  for (unsigned t = t0; t < t1; t += stride) {
+    const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
+    const unsigned i = 1u + t - r * C.dix.d, j = 1u + r - q * C.diy.d, k = 1u + q;
+    if (!gbf_pair_step_cell<MASS>(C, cells, s, w, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc, bad)) {
+      first = min(first, t);
+      last = t;
+    }
+  }
+  if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
+  for (unsigned t = first; t < t1 && t <= last; t += stride) {
+    const double2 phiA = pair_cell_again(C, m, d, cells, s, t);
+    if (MASS) {
+      acc.m1 += phiA.x;
+      acc.m2 += phiA.y;
+    }
+  }
 }
