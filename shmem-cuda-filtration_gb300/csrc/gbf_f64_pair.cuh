@@ -23,13 +23,30 @@
 //     pair_newton), and a Newton that 7 iterations do not end. The limit keeps P_k
 //     and its slope in FP32's range and the Newton's convergence quadratic: near
 //     residual water the reference's 7 iterations stop before they converge, and
-//     what they leave is the result.
+//     what they leave is the result;
+//   * a change of a phase's mass above 2^-5 of its density, where 2^-46 of it
+//     would show beside FP64's 2^-53. With the reference's compressibilities and
+//     white noise of 1000 and 10,000 Pa in P the mean errors of S are 1.6e-17 and
+//     1.8e-17, the plain FP64 passes' 2.4e-17 (without the limit 1.8e-17, 1.4e-16);
+//   * P further than 2^-5 P_atm from hydrostatic (2^-5 / beta1 where that is
+//     more) in the cell or next to it. P - P_hs is a multiple of P's last place,
+//     2^-53 to 2^-52 of P: nearer than that it fits the pair's 48 bits, further
+//     away the cell's face potentials are taken from FP64 differences. So are
+//     those at pressures above 32 / beta1, where the water's weight is that of
+//     32 times its density and fluxes of 2^3 of the limit above cancel.
+// What the looks for these cost where no cell is refused: 256^3 640 -> 655 us a
+// step. Where many are (192^3, all wet, us a step; 613 with none): all of them
+// 10,000 Pa off hydrostatic with the reference's compressibilities 1020; noise
+// of 10,000 Pa 20,900; S_e 1e-6 17,800, more than the plain passes' (about 3700),
+// which form each mobility once.
 // S below about 1e-13 has no mobility in pairs (om^3 is below FP32's range; in
 // FP64 it would move 1e-26 of itself a step).
 #pragma once
 
 #include "gbf_f64_cell.cuh"
 #include "gbf_pair.cuh"
+
+constexpr float kPairMost = 0.03125f;  // 2^-5: the largest change of a cell (of its density or saturation) in pairs
 
 // A row's constants: P_hs(j), P_hs(j) - P_atm as a pair, and what rounding
 // leaves of rho01 g h2 minus the rows' differences of P_hs (above, below).
@@ -61,6 +78,10 @@ struct GbfPairConsts {
   GbfFastDiv dnx, dny, dix, diy;
   int ri0, rk0, rn;  // rate source cells (rn = 0: none)
   float Patm;
+  float far;          // limit of |P - P_hs|: 2^-5 of P_atm or 1 / beta1
+  float deep;         // limit of P - P_atm: 32 / beta1
+  float rro1, rro2;   // 1 / rho0
+  double H_d;         // rho01 g h2
   GbfPf k1, k2, rk1;     // rho01 beta1, rho02 beta2, 1 / (rho01 beta1)
   GbfPf ro1, ro2;        // rho01, rho02
   GbfPf g1, g2, ghd;     // g h2 rho01 beta1, g h2 rho02 beta2, g h2 (rho02 - rho01)
@@ -91,6 +112,11 @@ inline GbfPairConsts gbf_pair_consts(const gbf_model& m) {
     C.rk0 = m.nz / 2 - m.rate_cells / 2;
   }
   C.Patm = (float)fabs(m.P_atm);
+  C.far = (float)(0x1p-5 * fmax(fabs(m.P_atm), 1. / m.beta1));
+  C.deep = (float)(32. / m.beta1);
+  C.rro1 = (float)(1. / m.ro01);
+  C.rro2 = (float)(1. / m.ro02);
+  C.H_d = m.ro01 * m.g * m.h2;
   // 2^e that brings the water mobility x density of media 0 to about 1
   int e = 0;
   const double L = m.K[0] * m.ro01 / m.mu1;
@@ -233,7 +259,8 @@ __device__ __forceinline__ void gbf_pair_props_cell(const GbfPairConsts& C, cons
     l2 = pf_mul(pf_mul(over_mu(C.c2), pf_mul(pf_mul(omp, omp), w2)), pf_add(C.ro2, pf_mul_raw(C.k2, Pp)));
     pf_st(w.Pk + c, pk);
   }
-  pf_st(w.D + c, D);
+  // NaN: pass 2 refuses the cells whose potentials use it
+  pf_st(w.D + c, fabsf(D.h) <= C.far && Pp.h <= C.deep ? D : GbfPf{__uint_as_float(0x7fffffffu), 0.f});
   pf_st(w.L1 + c, pf_mul(l1, pf_add(C.ro1, pf_mul_raw(C.k1, Pp))));
   pf_st(w.L2 + c, l2);
 }
@@ -248,8 +275,10 @@ __device__ __forceinline__ GbfPf pair_face(GbfPf x, GbfPf Lm, GbfPf Lp) {
   const bool f = x.h >= 0.f;
   return pf_mul_raw(x, GbfPf{f ? Lm.h : Lp.h, f ? Lm.l : Lp.l});
 }
-// w (out - in)
-__device__ __forceinline__ GbfPf pair_net(GbfPf out, GbfPf in, GbfPf w) {
+// w (out - in); MAG: mag + w times the larger of the two
+template <bool MAG>
+__device__ __forceinline__ GbfPf pair_net(GbfPf out, GbfPf in, GbfPf w, float& mag) {
+  if (MAG) mag = __fmaf_rn(w.h, fmaxf(fabsf(out.h), fabsf(in.h)), mag);
   const GbfPf s = pf_two_sum(out.h, -in.h);
   return pf_mul_raw(GbfPf{s.h, __fadd_rn(s.l, __fsub_rn(out.l, in.l))}, w);
 }
@@ -320,7 +349,7 @@ __device__ __forceinline__ bool pair_newton(const GbfPairConsts& C, int md, GbfP
     dp = it ? pf_addf(dp, ep) : GbfPf{ep, 0.f};
     ds = it ? pf_addf(ds, es) : GbfPf{es, 0.f};
     const float x = __fmul_rn(ds.h, rSe);  // relative change of S_e
-    if (!(fabsf(x) <= 0.5f)) return false;
+    if (!(fabsf(x) <= 0.5f && fabsf(ds.h) <= kPairMost)) return false;
     // what the step leaves: the Jacobian's error (2^-21) or its change since the point it was formed
     // at, of the step; small enough once below 2^-54 of S and of P
     const float chg = it > 1 ? __fmaf_rn(fabsf(ep), rb, fabsf(__fmul_rn(es, rSe))) : __fmaf_rn(fabsf(dp.h), rb, fabsf(x));
@@ -359,7 +388,34 @@ __device__ __forceinline__ bool pair_newton(const GbfPairConsts& C, int md, GbfP
   return false;
 }
 
-// The plain FP64 step of one cell (gbf_f64_cell.cuh), its stencil's mobilities
+// The Newton's equations of pair_newton in FP64. False: not a cell for
+// increments, or no end within 7 iterations.
+__device__ __forceinline__ bool pair_newton_f64(const gbf_model& m, const GbfDerived& d, int md, double P, double S,
+                                                double r1, double r2, double& dp, double& ds) {
+  const double inv = d.inv_1mswr[md], om = S * inv, Se = 1. - om, k1 = m.ro01 * m.beta1, k2 = m.ro02 * m.beta2;
+  if (!(om > -0.25 && om < 0.9995)) return false;
+  const double Pk = m.P_d[md] * exp(d.m_inv_lam[md] * log1p(-om)), pa = P - m.P_atm;
+  const double rho1 = m.ro01 * (1. + m.beta1 * pa), rho2 = m.ro02 * (1. + m.beta2 * (pa + Pk));
+  r2 += k2 * Pk * S;
+  double dPk = 0.;
+  dp = ds = 0.;
+  for (int it = 0; it < 7; it++) {
+    const double Sn = S + ds, slope = (Pk + dPk) * d.inv_lam_1mswr[md] / (Se - ds * inv);
+    if (it == 0 && !(fabs(k2 * S * slope) <= 0x1p-8 * fabs(rho2))) return false;
+    const double G1 = r1 + k1 * dp * (1. - Sn) - rho1 * ds, G2 = r2 + k2 * (dp + dPk) * Sn + rho2 * ds;
+    const double J11 = k1 * (1. - Sn), J12 = -(rho1 + k1 * dp), J21 = k2 * Sn;
+    const double J22 = rho2 + k2 * (dp + dPk + slope * Sn), rdet = 1. / (J11 * J22 - J12 * J21);
+    const double ep = -rdet * (J22 * G1 - J12 * G2), es = -rdet * (J11 * G2 - J21 * G1);
+    dp += ep;
+    ds += es;
+    if (!(fabs(ds * inv) <= 0.5 * fabs(Se))) return false;
+    if (fabs(ep) <= 0x1p-50 * fabs(dp) + 0x1p-56 * fabs(P) && fabs(es) <= 0x1p-50 * fabs(ds) + 0x1p-56 * fabs(S)) return true;
+    dPk = Pk * expm1(d.m_inv_lam[md] * log1p(-ds * inv / Se));
+  }
+  return false;
+}
+
+// The step of one cell in FP64 and in increments, its stencil's mobilities
 // formed here since no pass keeps them in FP64. Returns its part of the masses.
 static __device__ __noinline__ double2 pair_cell_f64(const gbf_model& m, const GbfDerived& d, const gbf_cells& cells,
                                                      const GbfF64Step& s, int i, int j, int k) {
@@ -368,8 +424,7 @@ static __device__ __noinline__ double2 pair_cell_f64(const gbf_model& m, const G
 #endif
   const GbfGeo g = gbf_geo(m);
   const size_t c = gbf_idx(g, i, j, k);
-  GbfF64Stencil q;
-  double S[7], P[7];
+  double S[7], P[7], L1[7], L2[7];
   auto at = [&](int t) {
     const size_t st = t < 3 ? 1 : t < 5 ? (size_t)g.nx : g.pl;
     return t == 0 ? c : (t & 1) ? c - st : c + st;
@@ -379,44 +434,98 @@ static __device__ __noinline__ double2 pair_cell_f64(const gbf_model& m, const G
     S[t] = s.S[at(t)];
     P[t] = s.P[at(t)];
   }
+  const int md = gbf_media_at(cells, c);
+  const double phi = cells.phi ? (double)cells.phi[c] : m.m[md], dtphi = m.dt / phi;
+  const bool src = d.src != 0. && j == 1 && gbf_in_rate_patch(m, i, k);
+  bool dry = !src;
+#pragma unroll
+  for (int t = 0; t < 7; t++) dry = dry && gbf_is_zero(S[t]);
 #pragma unroll 1
   for (int t = 0; t < 7; t++) {
-    const GbfF64Props p = gbf_f64_props(m, d, cells, P[t], S[t], at(t));
-    q.L1[t] = p.Xi1 * p.ro1;
-    q.L2[t] = p.Xi2 * p.ro2;
-    if (t == 0) {
-      q.ro1 = p.ro1;
-      q.ro2 = p.ro2;
-      q.lnSe = p.lnSe;
+    const int mt = gbf_media_at(cells, at(t));
+    const double K = cells.K ? (double)cells.K[at(t)] : m.K[mt], pa = P[t] - m.P_atm;
+    double k1 = 1., k2 = 0.;
+    if (!gbf_is_zero(S[t])) {
+      const double om = S[t] * d.inv_1mswr[mt], l = log1p(-om);
+      k1 = exp(d.e1[mt] * l);
+      k2 = om * om * -expm1(d.e2[mt] * l);
+    }
+    L1[t] = K * k1 * d.neg_inv_mu1 * (m.ro01 * (1. + m.beta1 * pa));
+    L2[t] = K * k2 * d.neg_inv_mu2 * (m.ro02 * (1. + m.beta2 * pa));
+  }
+  const bool noflow_bottom = m.bc_mode == GBF_BC_HYDROSTATIC_SIDES && j == g.ny - 2;
+  const GbfF64Faces faces = gbf_f64_faces(d, s.P, c, g.nx, g.pl);
+  const double ro1 = m.ro01 * (1. + m.beta1 * (P[0] - m.P_atm)), ro2 = m.ro02 * (1. + m.beta2 * (P[0] - m.P_atm));
+  const double r1 = dtphi * gbf_f64_divergence(m, d, faces, ro1 * m.g, noflow_bottom, L1);
+  const double q1 = ro1 * (1. - S[0]), q2 = ro2 * S[0];
+  double r2 = 0., Pn = P[0], Sn = S[0];
+  if (dry) {
+    Pn -= r1 / (m.ro01 * m.beta1);
+  } else {
+    double dp, ds;
+    r2 = dtphi * gbf_f64_divergence(m, d, faces, ro2 * m.g, noflow_bottom, L2);
+    if (src) r2 -= dtphi * d.src;
+    if (pair_newton_f64(m, d, md, P[0], S[0], r1, r2, dp, ds)) {
+      Pn += dp;
+      Sn += ds;
+    } else {
+      gbf_f64_newton(m, d, md, log((1. - S[0] - m.S_wr[md]) / (1. - m.S_wr[md])), q1 - r1, q2 - r2, Pn, Sn);
     }
   }
-  double m1 = 0., m2 = 0.;
-  unsigned bad = 0;
-  gbf_f64_cell_update(m, d, cells, s, g, i, j, k, q, m1, m2, bad);
-  if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
-  return make_double2(m1, m2);
+  if (s.roS1) {
+    s.roS1_old[c] = q1;
+    s.roS2_old[c] = q2;
+    s.roS1[c] = q1 - r1;
+    s.roS2[c] = q2 - r2;
+  }
+  if (!gbf_is_finite(Pn) || !gbf_is_finite(Sn)) atomicOr(s.status, GBF_DEV_NONFINITE);
+  s.Pn[c] = Pn;
+  s.Sn[c] = Sn;
+  return make_double2(phi * (q1 - r1), phi * (q2 - r2));
 }
-// What stands in S of the next state at a cell that the pairs refused until it
-// is taken again: a NaN of its own.
+// (*a - *b) + H as a pair.
+static __device__ __noinline__ GbfPf pair_diff64(const double* a, const double* b, double H) {
+  return pf_from_double(__dadd_rn(__dsub_rn(*a, *b), H));
+}
+
+// What stands in S of the next state at a cell that the pairs refused, for its
+// differences of P - P_hs or for good, until it is taken again: NaNs of its own.
 constexpr int kPairRefused = 0x7ffaf64c;
-__device__ __forceinline__ double pair_refused() { return __hiloint2double(kPairRefused, 0); }
+__device__ __forceinline__ double pair_refused(bool differences) { return __hiloint2double(kPairRefused, differences ? 1 : 0); }
 
 // Pass 2 at interior cell (i, j, k) = c: fluxes, Newton, next state (the
 // water-only form where no DNAPL is in the cell or flows through its faces).
 // False, and a mark left in S: not a cell for pairs (see the top of this file).
-template <bool MASS>
+// FAR: such a cell again, its potentials from FP64 differences (without a mark).
+template <bool MASS, bool FAR>
 __device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const gbf_cells& cells,
                                                    const GbfF64Step& s, const GbfPairWork& w, int i, int j, int k,
                                                    unsigned c, GbfPairMass& acc, unsigned& bad) {
   const unsigned nx = (unsigned)C.nx, pl = C.pl;
   const int md = cells.media ? __ldg(cells.media + c) : 0;
   const GbfPairRow R = w.rows[j];
-  const GbfPf D = pf_ld(w.D + c);
+  const double Pd = s.P[c];
+  const GbfPf D = FAR ? pf_from_double(__dsub_rn(Pd, R.phs)) : pf_ld(w.D + c);
   const GbfPf Pp = pf_add(R.pp, D);  // P - P_atm
   // face potentials times h; gravity g h2 (rho_a - rho01) with the centre cell's density
-  const GbfPf xm = pf_diff(pf_ld(w.D + c - 1), D), xp = pf_diff(D, pf_ld(w.D + c + 1));
-  const GbfPf zm = pf_diff(pf_ld(w.D + c - pl), D), zp = pf_diff(D, pf_ld(w.D + c + pl));
-  const GbfPf yu = pf_addf(pf_diff(pf_ld(w.D + c - nx), D), R.eu), yd = pf_addf(pf_diff(D, pf_ld(w.D + c + nx)), R.ed);
+  GbfPf xm = pf_ld(w.D + c - 1), xp = pf_ld(w.D + c + 1), yu = pf_ld(w.D + c - nx), yd = pf_ld(w.D + c + nx);
+  GbfPf zm = pf_ld(w.D + c - pl), zp = pf_ld(w.D + c + pl);
+  if (FAR) {
+    const double* P = s.P + c;
+    xm = pair_diff64(P - 1, P, 0.);
+    xp = pair_diff64(P, P + 1, 0.);
+    zm = pair_diff64(P - pl, P, 0.);
+    zp = pair_diff64(P, P + pl, 0.);
+    yu = pair_diff64(P - nx, P, C.H_d);
+    yd = pair_diff64(P, P + nx, C.H_d);
+  } else {
+    xm = pf_diff(xm, D);
+    xp = pf_diff(D, xp);
+    zm = pf_diff(zm, D);
+    zp = pf_diff(D, zp);
+    yu = pf_addf(pf_diff(yu, D), R.eu);
+    yd = pf_addf(pf_diff(D, yd), R.ed);
+  }
   const bool noflow = C.noflow && j == C.ny - 2;
   const GbfPf zero = {0.f, 0.f};
   GbfPf rphi;
@@ -429,16 +538,23 @@ __device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const
     rphi = C.rphi[md];
   }
   GbfPf r1;
+  // a phase's net change of density in the cell and 2^-3 of that through its faces (FAR), over rho0; a NaN shows
+  auto change = [&](GbfPf r, float mag, float rro) {
+    return __fmul_rn(FAR ? __fmaf_rn(mag, __fmul_rn(0.125f, rphi.h), fabsf(r.h)) : fabsf(r.h), rro);
+  };
+  float mag = 0.f, most;
   {
     const GbfPf Lc = pf_ld(w.L1 + c), G = pf_mul(C.g1, Pp);
     const GbfPf y1 = pf_add(yu, G), y2 = noflow ? zero : pf_add(yd, G);
     const GbfPf f = pair_sum3(
-        pair_net(pair_face(xp, Lc, pf_ld(w.L1 + c + 1)), pair_face(xm, pf_ld(w.L1 + c - 1), Lc), C.wx),
-        pair_net(pair_face(y2, Lc, pf_ld(w.L1 + c + nx)), pair_face(y1, pf_ld(w.L1 + c - nx), Lc), C.wy),
-        pair_net(pair_face(zp, Lc, pf_ld(w.L1 + c + pl)), pair_face(zm, pf_ld(w.L1 + c - pl), Lc), C.wz));
+        pair_net<FAR>(pair_face(xp, Lc, pf_ld(w.L1 + c + 1)), pair_face(xm, pf_ld(w.L1 + c - 1), Lc), C.wx, mag),
+        pair_net<FAR>(pair_face(y2, Lc, pf_ld(w.L1 + c + nx)), pair_face(y1, pf_ld(w.L1 + c - nx), Lc), C.wy, mag),
+        pair_net<FAR>(pair_face(zp, Lc, pf_ld(w.L1 + c + pl)), pair_face(zm, pf_ld(w.L1 + c - pl), Lc), C.wz, mag));
     r1 = pf_mul(f, rphi);
+    most = change(r1, mag, C.rro1);
+    mag = 0.f;
   }
-  const double Sd = __ldg(s.S + c), Pd = __ldg(s.P + c);
+  const double Sd = __ldg(s.S + c);
   const bool src = C.rn > 0 && j == 1 && (unsigned)(i - C.ri0) < (unsigned)C.rn && (unsigned)(k - C.rk0) < (unsigned)C.rn;
   const GbfPf Lc = pf_ld(w.L2 + c), Lxm = pf_ld(w.L2 + c - 1), Lxp = pf_ld(w.L2 + c + 1);
   const GbfPf Lyu = pf_ld(w.L2 + c - nx), Lyd = pf_ld(w.L2 + c + nx);
@@ -451,14 +567,15 @@ __device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const
   if (dnapl) {
     const GbfPf G = pf_add(pf_mul(C.g2, Pp), C.ghd);
     const GbfPf y1 = pf_add(yu, G), y2 = noflow ? zero : pf_add(yd, G);
-    const GbfPf f = pair_sum3(pair_net(pair_face(xp, Lc, Lxp), pair_face(xm, Lxm, Lc), C.wx),
-                              pair_net(pair_face(y2, Lc, Lyd), pair_face(y1, Lyu, Lc), C.wy),
-                              pair_net(pair_face(zp, Lc, Lzp), pair_face(zm, Lzm, Lc), C.wz));
+    const GbfPf f = pair_sum3(pair_net<FAR>(pair_face(xp, Lc, Lxp), pair_face(xm, Lxm, Lc), C.wx, mag),
+                              pair_net<FAR>(pair_face(y2, Lc, Lyd), pair_face(y1, Lyu, Lc), C.wy, mag),
+                              pair_net<FAR>(pair_face(zp, Lc, Lzp), pair_face(zm, Lzm, Lc), C.wz, mag));
     r2 = pf_mul(f, rphi);
+    ok = most <= kPairMost && change(r2, mag, C.rro2) <= kPairMost;
     double rest = 0.;  // what the pair r2 leaves of the source
     if (src) r2 = pf_sub(r2, pair_source(C.dtsrc_d, cells.phi ? gbf_f2d(phif) : C.phi_d[md], rest));
     GbfPf ds;
-    ok = pair_newton(C, md, Pp, pf_from_double(Sd), gbf_is_zero(Sd) ? C.pd[md] : pf_ld(w.Pk + c), r1, r2, dp, ds);
+    ok = ok && pair_newton(C, md, Pp, pf_from_double(Sd), gbf_is_zero(Sd) ? C.pd[md] : pf_ld(w.Pk + c), r1, r2, dp, ds);
     const double dsd = pf_to_double(ds);
     Sn = __dadd_rn(Sd, dsd);
     if (src) Sn = pair_add_rest(Sd, dsd, rest, C.rro2_d);
@@ -471,14 +588,14 @@ __device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const
   } else {
     dp = pf_neg(pf_mul(r1, C.rk1));  // rho01 beta1 dP = -r1
     Sn = Sd;
-    ok = true;
+    ok = most <= kPairMost;
     if (MASS && ok) {
       const double phi = cells.phi ? gbf_f2d(phif) : C.phi_d[md];
       acc.m1 = __fma_rn(phi, __fma_rn(C.k1_d, __dsub_rn(Pd, C.Patm_d), C.ro1_d), acc.m1);
     }
   }
   if (!ok) {
-    s.Sn[c] = pair_refused();
+    if (!FAR) s.Sn[c] = pair_refused(most != most);
     return false;
   }
   if (MASS) acc.r1 = pf_add(acc.r1, cells.phi ? pf_mulf(r1, phif) : pf_mul(r1, C.phip[md]));
@@ -490,38 +607,98 @@ __device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const
   return true;
 }
 
-// A cell, if gbf_pair_step_cell refused it; its part of the masses.
-static __device__ __noinline__ double2 pair_cell_again(const GbfPairConsts& C, const gbf_model& m, const GbfDerived& d,
-                                                       const gbf_cells& cells, const GbfF64Step& s, unsigned t) {
+// Interior cell number t.
+__device__ __forceinline__ unsigned pair_cell(const GbfPairConsts& C, unsigned t, int& i, int& j, int& k) {
   const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
-  const int i = (int)(1u + t - r * C.dix.d), j = (int)(1u + r - q * C.diy.d), k = (int)(1u + q);
-  const unsigned c = (unsigned)i + (unsigned)j * (unsigned)C.nx + (unsigned)k * C.pl;
-  if (__double2hiint(s.Sn[c]) != kPairRefused) return make_double2(0., 0.);
+  i = (int)(1u + t - r * C.dix.d);
+  j = (int)(1u + r - q * C.diy.d);
+  k = (int)(1u + q);
+  return (unsigned)i + (unsigned)j * (unsigned)C.nx + (unsigned)k * C.pl;
+}
+__device__ __forceinline__ bool pair_is_refused(const GbfPairConsts& C, const GbfF64Step& s, unsigned t) {
+  int i, j, k;
+  return __double2hiint(s.Sn[pair_cell(C, t, i, j, k)]) == kPairRefused;
+}
+// A cell that gbf_pair_step_cell refused; its part of the masses.
+template <bool MASS>
+static __device__ __noinline__ double2 pair_cell_again(const GbfPairConsts& C, const gbf_model& m, const GbfDerived& d,
+                                                       const gbf_cells& cells, const GbfF64Step& s,
+                                                       const GbfPairWork& w, unsigned t) {
+  int i, j, k;
+  const unsigned c = pair_cell(C, t, i, j, k);
+  if (__double2loint(s.Sn[c])) {
+    GbfPairMass acc;
+    unsigned bad = 0;
+    if (gbf_pair_step_cell<MASS, true>(C, cells, s, w, i, j, k, c, acc, bad)) {
+      if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
+      return make_double2(acc.m1 - pf_to_double(acc.r1), acc.m2);
+    }
+  }
   return pair_cell_f64(m, d, cells, s, i, j, k);
 }
-// Pass 2 at interior cells t0, t0 + stride, .. below t1, summed into acc. The
-// cells that the pairs refuse are taken after the others: calls among the pair
-// arithmetic cost it registers (256^3, none refused: pass 2 488 us with them there,
-// 466 after the others).
+// Pass 2 at interior cells t0, t0 + stride, .. below t1, summed into acc; every
+// thread of the block calls it. The cells that the pairs refuse are taken after
+// the others: calls among the pair arithmetic cost it registers (256^3, none
+// refused: pass 2 488 us with them there, 456 after the others). Up to an eighth
+// of a block's cells, they are listed and shared out evenly, in a fixed order: a
+// warp pays for the FP64 of one lane what it pays for 32. More than that, a
+// thread takes its own, whose neighbours' are in its warp.
 template <bool MASS>
 __device__ __forceinline__ void gbf_pair_step_cells(const GbfPairConsts& C, const gbf_model& m, const GbfDerived& d,
                                                     const gbf_cells& cells, const GbfF64Step& s, const GbfPairWork& w,
                                                     unsigned t0, unsigned stride, unsigned t1, GbfPairMass& acc) {
   unsigned bad = 0, first = t1, last = 0;  // of the refused cells
   for (unsigned t = t0; t < t1; t += stride) {
-    const unsigned r = gbf_div(t, C.dix), q = gbf_div(r, C.diy);
-    const unsigned i = 1u + t - r * C.dix.d, j = 1u + r - q * C.diy.d, k = 1u + q;
-    if (!gbf_pair_step_cell<MASS>(C, cells, s, w, (int)i, (int)j, (int)k, i + j * (unsigned)C.nx + k * C.pl, acc, bad)) {
+    int i, j, k;
+    const unsigned c = pair_cell(C, t, i, j, k);
+    if (!gbf_pair_step_cell<MASS, false>(C, cells, s, w, i, j, k, c, acc, bad)) {
       first = min(first, t);
       last = t;
     }
   }
   if (bad) atomicOr(s.status, GBF_DEV_NONFINITE);
-  for (unsigned t = first; t < t1 && t <= last; t += stride) {
-    const double2 phiA = pair_cell_again(C, m, d, cells, s, t);
+  auto again = [&](unsigned t) {
+    const double2 phiA = pair_cell_again<MASS>(C, m, d, cells, s, w, t);
     if (MASS) {
       acc.m1 += phiA.x;
       acc.m2 += phiA.y;
     }
+  };
+#ifdef __CUDACC__
+  if (!__syncthreads_or(first < t1)) return;
+  constexpr unsigned kList = 128;
+  __shared__ unsigned list[kList], warps[32];
+  unsigned n = 0;  // this thread's
+  for (unsigned t = first; t < t1 && t <= last; t += stride) n += pair_is_refused(C, s, t);
+  const unsigned lane = threadIdx.x & 31u;
+  unsigned rank = n;  // cells of the threads before, in the warp and in the block
+  for (unsigned o = 1; o < 32u; o <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, rank, o);
+    if (lane >= o) rank += v;
   }
+  if (lane == 31u) warps[threadIdx.x >> 5] = rank;
+  __syncthreads();
+  rank -= n;
+  unsigned total = 0;
+  for (unsigned q = 0; q < blockDim.x >> 5; q++) {
+    if (q < threadIdx.x >> 5) rank += warps[q];
+    total += warps[q];
+  }
+  if (total * 8u > (t1 - (t0 - threadIdx.x) + stride - 1u) / stride * blockDim.x) {  // the block's cells: t0 is its first plus threadIdx.x
+    for (unsigned t = first; t < t1 && t <= last; t += stride)
+      if (pair_is_refused(C, s, t)) again(t);
+    return;
+  }
+  unsigned t = first;
+  for (unsigned base = 0; base < total; base += kList) {
+    for (; t < t1 && t <= last && rank < base + kList; t += stride)
+      if (pair_is_refused(C, s, t)) list[rank++ - base] = t;
+    __syncthreads();
+    for (unsigned q = threadIdx.x; q < kList && base + q < total; q += blockDim.x) again(list[q]);
+    __syncthreads();
+  }
+#else
+  for (unsigned t = first; t < t1 && t <= last; t += stride)
+    if (pair_is_refused(C, s, t)) again(t);
+#endif
 }

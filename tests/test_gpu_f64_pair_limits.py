@@ -1,5 +1,6 @@
 """The FP64 step on a GPU where its increments do not fit FP32 pairs: near
-residual water and for small lambda (single domains, and an ensemble of them), and a drop-in whose parameters move from the pair step to
+residual water and for small lambda (single domains, and an ensemble of them),
+far from hydrostatic, and a drop-in whose parameters move from the pair step to
 the plain passes and back. Against the oracle at the plain FP64 paths' tolerances."""
 from importlib import import_module
 from types import SimpleNamespace
@@ -8,7 +9,7 @@ import numpy as np
 import pytest
 
 from gpu_util import assert_field, p_tol
-from test_pair_cells import residual_state
+from test_pair_cells import overpressure, residual_state
 
 pytestmark = pytest.mark.gpu
 
@@ -60,6 +61,23 @@ def test_residual_water(gpu_lib, abi, O, oracle, pkg, lam, iterations):
     for r, (m, _, _, want) in enumerate(members):
         check(m, ens.download(r, "P1"), ens.download(r, "S2"), masses[:, r], want)
     ens.close()
+
+
+@pytest.mark.parametrize("smooth", [True, False])
+@pytest.mark.parametrize("uniform", [0.0, 1e4, 1e6])
+@pytest.mark.parametrize("amp", [100.0, 1e4])
+@pytest.mark.parametrize("ini", [True, False])
+def test_overpressure(gpu_lib, abi, O, oracle, pkg, ini, amp, uniform, smooth):
+    Domain = import_module(pkg.__name__ + ".domain").Domain
+    m, media, P, S = overpressure(abi, O, ini, amp, uniform, smooth)
+    want = oracle_step(O, oracle, m, P, S, media)
+    dom = Domain(m, media)
+    dom.set_outputs(abi.GBF_OUT_MASS, 1)
+    dom.upload(P, S)
+    dom.step(1)
+    assert dom.status() == abi.GBF_OK
+    check(m, dom.download("P1"), dom.download("S2"), dom.mass_history(1), want)
+    dom.close()
 
 
 def test_dropin_parameters_change_the_step(gpu_lib, abi, O, oracle, pkg):
