@@ -189,7 +189,7 @@ struct GbfPairWork {
 };
 
 __device__ __forceinline__ GbfPf pf_ld(const float2* p) {
-  const float2 v = __ldg(p);
+  const float2 v = *p;  // written by pass 1, which may still run when this kernel starts: no __ldg
   return {v.x, v.y};
 }
 __device__ __forceinline__ void pf_st(float2* p, GbfPf a) { *p = make_float2(a.h, a.l); }
@@ -231,8 +231,8 @@ __device__ __forceinline__ void gbf_pair_props_cell(const GbfPairConsts& C, cons
     s.ro1[c] = C.ro1_d * (1. + C.beta1_d * (P - C.Patm_d));
     s.ro2[c] = C.ro2_d * (1. + C.beta2_d * (P - C.Patm_d));
   } else {
-    P = __ldg(s.P + c);
-    S = __ldg(s.S + c);
+    P = s.P[c];
+    S = s.S[c];
   }
   const GbfPairRow R = w.rows[j];
   const GbfPf D = pf_from_double(__dsub_rn(P, R.phs));
@@ -554,7 +554,7 @@ __device__ __forceinline__ bool gbf_pair_step_cell(const GbfPairConsts& C, const
     most = change(r1, mag, C.rro1);
     mag = 0.f;
   }
-  const double Sd = __ldg(s.S + c);
+  const double Sd = s.S[c];
   const bool src = C.rn > 0 && j == 1 && (unsigned)(i - C.ri0) < (unsigned)C.rn && (unsigned)(k - C.rk0) < (unsigned)C.rn;
   const GbfPf Lc = pf_ld(w.L2 + c), Lxm = pf_ld(w.L2 + c - 1), Lxp = pf_ld(w.L2 + c + 1);
   const GbfPf Lyu = pf_ld(w.L2 + c - nx), Lyd = pf_ld(w.L2 + c + nx);

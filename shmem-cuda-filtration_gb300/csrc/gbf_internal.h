@@ -232,10 +232,12 @@ void gbf_timer_free(GbfTimer* t);
 // A step's kernels follow each other on one stream. Launched with programmatic
 // stream serialization, a kernel's blocks may become resident while the kernel
 // before it finishes; gbf_pdl_begin at its start lets the next one in and waits
-// until everything before is complete and visible, so the order of all memory
-// accesses is that of plain launches and the gap between two kernels (about
-// 1 us) shrinks. Every kernel launched with pdl calls it before its first
-// access to global memory. The ensembles' steps are launched without: as edges
+// until everything before is complete and visible, so the order of all plain
+// memory accesses is that of plain launches and the gap between two kernels
+// (about 1 us) shrinks. Every kernel launched with pdl calls it before its first
+// access to global memory, and reads what a step's kernels write by plain loads:
+// a non-coherent one (__ldg) is for data that nothing writes while the kernel is
+// resident. The ensembles' steps are launched without: as edges
 // of their CUDA graphs the programmatic launches cost more than the gaps (a
 // step of two FP64 members 187 us plain, 245 us with them); so are a caller's
 // captures of a domain's stream.

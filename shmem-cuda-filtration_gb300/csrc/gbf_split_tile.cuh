@@ -1157,8 +1157,8 @@ __device__ bool split_tile(const GbfSplitConsts& C, const GbfSplitGrid& G, int i
       rP[s] = 0.f; rS[s] = 0.f; rK[s] = 0.f; rM[s] = 0;
       if (hcol[s] >= 0 && k < nz) {
         const unsigned c = (unsigned)hcol[s] + (unsigned)k * pln;
-        rP[s] = __ldg(G.dP + c);
-        rS[s] = __ldg(G.S + c);
+        rP[s] = G.dP[c];
+        rS[s] = G.S[c];
         rM[s] = G.media ? __ldg(G.media + c) : 0;
         rK[s] = G.K ? __ldg(G.K + c) : split_of(C.K, rM[s]);
       }
