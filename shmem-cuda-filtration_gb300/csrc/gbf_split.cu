@@ -461,7 +461,8 @@ int gbf_split_alloc(gbf_domain* d) {
   if (!s) s |= gbf_domain_alloc(d, (void**)&d->M1, n * mb);
   if (!s) s |= gbf_domain_alloc(d, (void**)&d->M2, n * mb);
   d->split_cells = d->cells;
-  if (!s && d->px != m.nx) {  // the cell fields in padded rows
+  // the cell fields in padded rows; a drop-in's media array that TMA cannot take in place is copied too
+  if (!s && (d->px != m.nx || (tma && ((uintptr_t)d->cells.media & 15) != 0))) {
     auto padded = [&](const void* src, const void** dst) {
       if (!src || s) return;
       s |= gbf_domain_alloc(d, (void**)dst, n * 4);
