@@ -58,7 +58,7 @@ __device__ __forceinline__ bool is_zero(double d) {
 }
 __device__ __forceinline__ bool is_finite(double d) { return ((unsigned)__double2hiint(d) & 0x7ff00000u) != 0x7ff00000u; }
 
-// A positive divisor and its correctly rounded reciprocal (r = 0: divide).
+// A divisor and its correctly rounded reciprocal (r = 0: divide).
 struct Recip {
   double b, r;
 };
@@ -68,7 +68,8 @@ __device__ __noinline__ double plain_div(double a, double b) { return a / b; }
 // the quotient by the reciprocal is within two units in the last place; a
 // residual step brings it within one, and by Markstein's theorem (IBM J. Res.
 // Dev. 34, 1990) the next is then correctly rounded. The residuals are exact
-// away from underflow and overflow; other dividends (but zeros) are divided.
+// away from underflow and overflow; other dividends (but zeros, over a positive
+// number) are divided.
 __device__ __forceinline__ double exact_div(double a, const Recip& d) {
   const unsigned e = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
   if (e - 200u < 1600u && d.r != 0.0) {
@@ -76,7 +77,7 @@ __device__ __forceinline__ double exact_div(double a, const Recip& d) {
     q = __fma_rn(__fma_rn(-q, d.b, a), d.r, q);
     return __fma_rn(__fma_rn(-q, d.b, a), d.r, q);
   }
-  if (is_zero(a)) return a;  // b > 0
+  if (is_zero(a) && d.b > 0.) return a;
   return plain_div(a, d.b);
 }
 
@@ -86,9 +87,11 @@ struct EagerConsts {
   double e1[2], e2[2], mil[2], mil1[2];  // Brooks-Corey exponents; -1/lambda, -1/lambda - 1
   Recip om_swr[2], lam_swr[2];           // 1 - S_wr, lambda (1 - S_wr)
   double PkS1[2];                        // dP_k/dS at S_e = 1
+  bool one[2];                           // S = 0 is S_e = 1, its P_k and slope finite (no model of use is not so)
   double Xi1w[2];                        // Xi1 of the table's K at S_e = 1
   Recip mu1, mu2, h1, h2, h3, hh1, hh2, hh3;  // hh: 2 h
   double dtphi[2];                       // dt / phi of the table
+  bool flux;                             // finite pressures have finite potentials: no zero mobility meets a NaN
 };
 EagerConsts eager_consts(const gbf_model& m) {
   EagerConsts C;
@@ -101,9 +104,11 @@ EagerConsts eager_consts(const gbf_model& m) {
     C.om_swr[md] = recip(1 - swr);
     C.lam_swr[md] = recip(lam * (1 - swr));
     C.PkS1[md] = m.P_d[md] / (lam * (1 - swr));
+    C.one[md] = (1. - swr) / (1. - swr) == 1. && isfinite(C.PkS1[md]) && isfinite(m.P_d[md]);
     C.Xi1w[md] = -1. * m.K[md] / m.mu1;
     C.dtphi[md] = m.dt / m.m[md];
   }
+  C.flux = fabs(m.h1) > 0. && fabs(m.h2) > 0. && fabs(m.h3) > 0. && isfinite(m.g) && isfinite(m.kv);
   C.mu1 = recip(m.mu1);
   C.mu2 = recip(m.mu2);
   C.h1 = recip(m.h1);
@@ -166,7 +171,7 @@ __global__ void k_props(const gbf_model m, const EagerConsts C, gbf_arrays a, gb
       S2 = a.S2[c];
       P1 = a.P1[c];
     }
-    const bool wet = mine && !is_zero(S2);
+    const bool wet = mine && !(is_zero(S2) && C.one[md]);
     const bool some = pow_jobs(jobs, wet, wet, S2, md, m, C, C.e1, C.e2, [](int k, int, double S_e, double p) {
       return k ? (1. - S_e) * (1. - S_e) * (1 - p) : p;
     });
@@ -316,7 +321,7 @@ __global__ void k_mass(const gbf_model m, const EagerConsts C, gbf_arrays a, gbf
     const double roS2 = a.ro2[c] * a.S2[c];
     const bool closed = noflow_bottom && j == g.ny - 2;
     // P2 equal to P1 at the seven cells; DNAPL immobile there, and every number that its zero mobility multiplies finite
-    bool same = true, still = true;
+    bool same = true, still = C.flux;
 #pragma unroll
     for (int q = 0; q < 7; q++) {
       const double p2 = a.P2[nb[q]];
@@ -374,7 +379,7 @@ __global__ void k_newton(const gbf_model m, const EagerConsts C, gbf_arrays a, g
     const double pd = m.P_d[md];
     // Without DNAPL (S2 = 0, roS2 = 0) every product with S2 is zero, dS too,
     // and the step in P1 is the one of the general form with those zeros left out.
-    if (mine && is_zero(S2) && is_zero(roS2) && is_finite(P1) && is_finite(roS1) && !tol) {
+    if (mine && C.one[md] && is_zero(S2) && is_zero(roS2) && is_finite(P1) && is_finite(roS1) && !tol) {
       const double F1P = m.ro01 * (m.beta1);
       double Pb = P1;
       for (int w = 1; w <= N; w++) {
@@ -395,7 +400,7 @@ __global__ void k_newton(const gbf_model m, const EagerConsts C, gbf_arrays a, g
     }
     double Pb = P1, Sb = S2, Sk = 0., P_k = 0., SPkS = 0., omS = 0., F1P = 0., F2P = 0.;  // b: the point before
     for (int w = 1; w <= N; w++) {
-      const bool moved = active && (w == 1 || !same_bits(S2, Sk)), wet = moved && !is_zero(S2);
+      const bool moved = active && (w == 1 || !same_bits(S2, Sk)), wet = moved && !(is_zero(S2) && C.one[md]);
       // P_k and dP_k/dS where S2 moved (at S_e = 1 without pow)
       if (!pow_jobs(jobs, active, wet, S2, md, m, C, C.mil, C.mil1, [&](int k, int d, double, double p) {
             const double v = m.P_d[d] * p;
