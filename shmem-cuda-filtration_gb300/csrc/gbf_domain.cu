@@ -128,6 +128,14 @@ int f64_step(gbf_domain* d, int props_flags) {
   return GBF_OK;
 }
 
+// The derived arrays that pass 1 of an FP64 step writes too.
+int props_flags(const gbf_domain* d) {
+  int pf = 0;
+  if (d->outs.Xi1) pf |= GBF_PF_WRITE_XI_P2;
+  if (d->outs.u1x && (d->out_flags & GBF_OUT_VELOCITY)) pf |= GBF_PF_WRITE_U;
+  return pf;
+}
+
 int copy_cells(gbf_domain* d, const gbf_cells* hc) {
   const size_t n = gbf_geo(d->m).n;
   if (!hc) return GBF_OK;
@@ -286,9 +294,7 @@ int gbf_domain_advance_host(gbf_domain* d, const double* P_in, const double* S_i
 int gbf_domain_step(gbf_domain* d, int nsteps) {
   if (!d || nsteps < 0) return gbf_fail(GBF_ERR_ARG, "gbf_domain_step");
   if (!d->uploaded) return gbf_fail(GBF_ERR_STATE, "gbf_domain_step before upload");
-  int pf = 0;
-  if (d->outs.Xi1) pf |= GBF_PF_WRITE_XI_P2;
-  if (d->outs.u1x && (d->out_flags & GBF_OUT_VELOCITY)) pf |= GBF_PF_WRITE_U;
+  const int pf = props_flags(d);
   for (int s = 0; s < nsteps; s++) {
     int st = (d->precision != GBF_PREC_F64) ? gbf_split_step(d) : f64_step(d, pf);
     if (st) return st;
@@ -299,7 +305,7 @@ int gbf_domain_step(gbf_domain* d, int nsteps) {
 int gbf_domain_launches_per_step(gbf_domain* d) {
   if (!d) return 0;
   if (d->precision != GBF_PREC_F64) return gbf_split_launches_per_step(d);
-  return 3;
+  return 3 + (d->pair && props_flags(d) ? 1 : 0);  // beside the pair step, a pass of their own forms them
 }
 
 int gbf_domain_sync(gbf_domain* d) {

@@ -757,7 +757,7 @@ int gbf_split_advance_host(gbf_domain* d, const double* P_in, const double* S_in
 }
 
 int gbf_split_launches_per_step(gbf_domain* d) {
-  return 2 + (d->split_patch ? 1 : 0);
+  return 2 + (d->split_patch ? 1 : 0) + (d->borrowed && d->split_cells.media != d->cells.media ? 1 : 0);
 }
 
 // ----------------------------------------------------------- diagnostics
