@@ -38,7 +38,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
-#include "gbf_internal.h"
+#include "gbf_pair.cuh"
 
 namespace {
 
@@ -53,11 +53,6 @@ __device__ __forceinline__ double phi_at(const gbf_model& m, const gbf_cells& c,
 }
 
 __device__ __forceinline__ bool same_bits(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
-__device__ __forceinline__ bool is_zero(double d) {
-  return (((unsigned)__double2hiint(d) << 1) | (unsigned)__double2loint(d)) == 0u;
-}
-__device__ __forceinline__ bool is_finite(double d) { return ((unsigned)__double2hiint(d) & 0x7ff00000u) != 0x7ff00000u; }
-
 // A divisor and its correctly rounded reciprocal (r = 0: divide).
 struct Recip {
   double b, r;
@@ -77,7 +72,7 @@ __device__ __forceinline__ double exact_div(double a, const Recip& d) {
     q = __fma_rn(__fma_rn(-q, d.b, a), d.r, q);
     return __fma_rn(__fma_rn(-q, d.b, a), d.r, q);
   }
-  if (is_zero(a) && d.b > 0.) return a;
+  if (gbf_is_zero(a) && d.b > 0.) return a;
   return plain_div(a, d.b);
 }
 
@@ -171,7 +166,7 @@ __global__ void k_props(const gbf_model m, const EagerConsts C, gbf_arrays a, gb
       S2 = a.S2[c];
       P1 = a.P1[c];
     }
-    const bool wet = mine && !(is_zero(S2) && C.one[md]);
+    const bool wet = mine && !(gbf_is_zero(S2) && C.one[md]);
     const bool some = pow_jobs(jobs, wet, wet, S2, md, m, C, C.e1, C.e2, [](int k, int, double S_e, double p) {
       return k ? (1. - S_e) * (1. - S_e) * (1 - p) : p;
     });
@@ -258,7 +253,7 @@ __device__ __noinline__ double plain_upwind(double x1, double x2, double Xc, dou
 }
 __device__ __forceinline__ double upwind_div(double x1, double x2, double Xc, double rc, double Xm, double rm,
                                              double Xp, double rp, const Recip& h) {
-  if (!is_finite(x1) || !is_finite(x2)) return plain_upwind(x1, x2, Xc, rc, Xm, rm, Xp, rp, h.b);
+  if (!gbf_is_finite(x1) || !gbf_is_finite(x2)) return plain_upwind(x1, x2, Xc, rc, Xm, rm, Xp, rp, h.b);
   // (x + |x|) / 2 and (x - |x|) / 2 of a finite x are x or +0, by its sign bit (-0: +0 and -0)
   const bool n1 = __double2hiint(x1) < 0, n2 = __double2hiint(x2) < 0;
   const double p1 = n1 ? 0. : x1, m1 = n1 ? x1 : 0., p2 = n2 ? 0. : x2, m2 = n2 ? x2 : 0.;
@@ -326,7 +321,7 @@ __global__ void k_mass(const gbf_model m, const EagerConsts C, gbf_arrays a, gbf
     for (int q = 0; q < 7; q++) {
       const double p2 = a.P2[nb[q]];
       same = same && same_bits(p2, a.P1[nb[q]]);
-      still = still && is_zero(a.Xi2[nb[q]]) && is_finite(p2) && is_finite(a.ro2[nb[q]]);
+      still = still && gbf_is_zero(a.Xi2[nb[q]]) && gbf_is_finite(p2) && gbf_is_finite(a.ro2[nb[q]]);
     }
     const Faces f = eager_faces(a.P1, c, nx, pl, C);
     const double f1 = eager_divergence(m, C, f, closed, a.Xi1, a.ro1, c, nx, pl);
@@ -334,7 +329,7 @@ __global__ void k_mass(const gbf_model m, const EagerConsts C, gbf_arrays a, gbf
     double A1 = roS1 - dtphi * f1, A2;
     const bool in_src = src != 0.0 && j == 1 && gbf_in_rate_patch(m, i, k);
     // roS2 - dtphi (+-0): roS2 itself, but for roS2 = -0
-    if (still && !in_src && __double_as_longlong(roS2) != (long long)0x8000000000000000ull && is_finite(dtphi)) {
+    if (still && !in_src && __double_as_longlong(roS2) != (long long)0x8000000000000000ull && gbf_is_finite(dtphi)) {
       A2 = roS2;
     } else {
       const double gsum = eager_divergence2(m, C, a, f, same, closed, c, nx, pl);
@@ -379,7 +374,7 @@ __global__ void k_newton(const gbf_model m, const EagerConsts C, gbf_arrays a, g
     const double pd = m.P_d[md];
     // Without DNAPL (S2 = 0, roS2 = 0) every product with S2 is zero, dS too,
     // and the step in P1 is the one of the general form with those zeros left out.
-    if (mine && C.one[md] && is_zero(S2) && is_zero(roS2) && is_finite(P1) && is_finite(roS1) && !tol) {
+    if (mine && C.one[md] && gbf_is_zero(S2) && gbf_is_zero(roS2) && gbf_is_finite(P1) && gbf_is_finite(roS1) && !tol) {
       const double F1P = m.ro01 * (m.beta1);
       double Pb = P1;
       for (int w = 1; w <= N; w++) {
@@ -400,7 +395,7 @@ __global__ void k_newton(const gbf_model m, const EagerConsts C, gbf_arrays a, g
     }
     double Pb = P1, Sb = S2, Sk = 0., P_k = 0., SPkS = 0., omS = 0., F1P = 0., F2P = 0.;  // b: the point before
     for (int w = 1; w <= N; w++) {
-      const bool moved = active && (w == 1 || !same_bits(S2, Sk)), wet = moved && !(is_zero(S2) && C.one[md]);
+      const bool moved = active && (w == 1 || !same_bits(S2, Sk)), wet = moved && !(gbf_is_zero(S2) && C.one[md]);
       // P_k and dP_k/dS where S2 moved (at S_e = 1 without pow)
       if (!pow_jobs(jobs, active, wet, S2, md, m, C, C.mil, C.mil1, [&](int k, int d, double, double p) {
             const double v = m.P_d[d] * p;

@@ -112,7 +112,7 @@ const void* gbf_mapped_host(const void* p) {
 extern "C" {
 
 const char* gbf_kernel_name(int kind) {
-  static const char* names[GBF_K_COUNT] = {"f64_props", "f64_flux_newton", "f64_boundary", "mass_tail",
+  static const char* names[GBF_K_COUNT] = {"f64_props", "f64_flux_newton", "f64_boundary",
                                            "split_step", "split_boundary", "ensemble_step", "ensemble_boundary",
                                            "ensemble_f64_props", "ensemble_f64_flux_newton"};
   return (kind >= 0 && kind < GBF_K_COUNT) ? names[kind] : "";

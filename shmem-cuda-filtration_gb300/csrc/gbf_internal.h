@@ -209,7 +209,7 @@ GBF_HD T gbf_sweep_P(const gbf_model& m, const GbfGeo& g, const T* cur, const T*
 // ------------------------------------------------------- kernel timing
 // Optional CUDA-event spans around each kernel launch, on the launching
 // stream (bench accounting of the dominant kernel). Kinds index gbf_kernel_name().
-enum { GBF_K_PROPS = 0, GBF_K_FLUX_NEWTON, GBF_K_BOUNDARY, GBF_K_MASS_TAIL, GBF_K_SPLIT_STEP, GBF_K_SPLIT_BOUNDARY,
+enum { GBF_K_PROPS = 0, GBF_K_FLUX_NEWTON, GBF_K_BOUNDARY, GBF_K_SPLIT_STEP, GBF_K_SPLIT_BOUNDARY,
        GBF_K_ENS_STEP, GBF_K_ENS_BOUNDARY, GBF_K_ENS_PROPS, GBF_K_ENS_FLUX_NEWTON, GBF_K_COUNT };
 
 struct GbfTimer {

@@ -41,11 +41,6 @@ __device__ __forceinline__ GbfPf pf_addf(GbfPf a, float b) {
   const GbfPf s = pf_two_sum(a.h, b);
   return pf_fast(s.h, __fadd_rn(s.l, a.l));
 }
-// a + b with |a.h| >= |b.h|
-__device__ __forceinline__ GbfPf pf_add_big(GbfPf a, GbfPf b) {
-  const GbfPf s = pf_fast(a.h, b.h);
-  return pf_fast(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
-}
 // a product, its parts not renormalised (|l| up to about 2^-22 |h|)
 __device__ __forceinline__ GbfPf pf_mul_raw(GbfPf a, GbfPf b) {
   const float p = __fmul_rn(a.h, b.h);

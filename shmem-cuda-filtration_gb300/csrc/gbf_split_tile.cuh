@@ -1552,7 +1552,6 @@ struct GbfPairSmem {
   Ring ring;
   float dP[kTmaStages][Ring::NP];
   float L1[kTmaStages][Ring::NP], L2[kTmaStages][Ring::NP];
-  int wet[kTmaStages];  // the last plane of each buffer with DNAPL (of another tile before: taken as wet, no harm)
 };
 // The mbarriers of the two rings (halo planes, interior rows), apart from the
 // ring data: a CTA that runs tiles of two shapes keeps one set of barriers,
@@ -1752,7 +1751,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
     md = has_media ? make_int2(__float_as_int(kv.x), __float_as_int(kv.y)) : make_int2(0, 0);
     return make_float2(split_of(C.K, md.x), split_of(C.K, md.y));
   };
-  auto build = [&](int s, int k) {  // plane buffer s (plane k) from halo stage s
+  auto build = [&](int s) {  // plane buffer s from halo stage s
 #pragma unroll
     for (int q = 0; q < SLOTS; q++) {
       // slot 0: the own pair of every thread in the tile; the first later
@@ -1790,7 +1789,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
   }
   {
     const bool ok = wait_bit(0);
-    if (ok) build(0, k0);
+    if (ok) build(0);
     if (__syncthreads_or(!ok)) {
       give_up();
       return false;
@@ -1824,7 +1823,7 @@ __device__ bool split_tile_x2(const GbfSplitConsts& C, const GbfSplitGrid& G, in
       const int sn = t_next;
       bool ok = wait_bit(sn);
       ok = ok && wait_bit(8 + t_rows);
-      if (ok) build(sn, k + 1);
+      if (ok) build(sn);
       if (__syncthreads_or(!ok)) {
         give_up();
         return false;
