@@ -4,15 +4,15 @@
                     [--workload NAME] [--cube N] [--no-compare] [--no-cpu-baseline]
 
 Workloads are <config>_<form>: config0..config4 (the benchmark configurations
-as seeded synthetic inputs, see workloads.py) and the forms f64 (plain FP64),
-split (FP32 state and fluxes, phase masses at FP64 precision as FP32-pair
-defects, one residual-correction Newton step per cell), splitdf (FP32-pair
+as seeded synthetic inputs, see workloads.py) and the forms f64 (FP64 state,
+increments from FP32 pairs), split (FP32 state and fluxes, phase masses at FP64
+precision as FP32-pair defects, one residual-correction Newton step per cell), splitdf (FP32-pair
 masses), splitdefect (FP32 mass defects, no correction step); and
 config1_dropin / config1_dropinsplit, config 1's grid through the reference's
 own host function set (defines.h: the five calls of time_step_function) in
 fused FP64 mode / split mode.
 The default, config4_split, is the combined precision + batching form on the
-256-member ensemble; the same line also reports plain FP64 and the other split
+256-member ensemble; the same line also reports the FP64 form and the other split
 forms on the same members.
 
 One JSON line on rank 0. `value` is device-resident throughput (inputs in
@@ -151,7 +151,8 @@ def barrier(world):
 
 # ------------------------------------------------------------------ workloads
 
-PRECISIONS = {"f64": ("GBF_PREC_F64", "plain FP64", "f64"),
+PRECISIONS = {"f64": ("GBF_PREC_F64", "FP64 state and inputs, a step's increments from FP32 pairs (cells that those do "
+                     "not hold: FP64)", "f64+f32x2"),
               "split": ("GBF_PREC_SPLIT", "FP32 state and fluxes, phase masses at FP64 precision (FP32-pair "
                         "defects over the state's mass at the row's hydrostatic density), one residual-"
                         "correction Newton step per cell with the residual in FP32 pairs", "f32+f32x2"),
@@ -159,8 +160,8 @@ PRECISIONS = {"f64": ("GBF_PREC_F64", "plain FP64", "f64"),
                           "f32+f32x2"),
               "splitdefect": ("GBF_PREC_SPLIT_DEFECT", "FP32 state and fluxes, phase masses as FP32 defects over "
                               "the state's mass at the row's hydrostatic density, no correction step", "f32"),
-              "dropin": ("GBF_PREC_F64", "plain FP64 through the reference's host function set (defines.h), "
-                         "fused mode", "f64"),
+              "dropin": ("GBF_PREC_F64", "the FP64 form (FP64 state and inputs, increments from FP32 pairs) through "
+                         "the reference's host function set (defines.h), fused mode", "f64+f32x2"),
               "dropinsplit": ("GBF_PREC_SPLIT", "the split form (FP32 state and fluxes, phase masses at FP64 "
                               "precision, one residual-correction Newton step per cell) through the reference's "
                               "host function set (defines.h), split mode", "f32+f32x2")}
@@ -357,14 +358,13 @@ class DropinRunner:
 
 
 # Algorithmic bytes per interior (or every) cell of each kernel: the
-# compulsory DRAM traffic of its inputs and outputs.
+# compulsory DRAM traffic of its inputs and outputs, in a cell with DNAPL.
 ALGO_BYTES = {
     "f64_props": (52.0, "all"),             # read P, S, K (20); write P - P_hs, L1, L2, P_k as FP32 pairs (32)
     "ensemble_f64_props": (52.0, "all"),
-    "f64_flux_newton": (60.0, "interior"),  # read P, S, P - P_hs, L1, L2 (40), phi (4); write P, S (16); 8 more with DNAPL
-    "ensemble_f64_flux_newton": (60.0, "interior"),
-    # read dP, S, K, phi (16), M1, M2 (16); write dP, S (8), M1, M2 (16). Cells without DNAPL leave M2
-    # unwritten: 8 bytes fewer (4 in the defect form)
+    "f64_flux_newton": (68.0, "interior"),  # read P, S, P - P_hs, L1, L2, P_k (48), phi (4); write P, S (16)
+    "ensemble_f64_flux_newton": (68.0, "interior"),
+    # read dP, S, K, phi (16), M1, M2 (16); write dP, S (8), M1, M2 (16)
     "split_step": (56.0, "interior"),
     "ensemble_step": (56.0, "interior"),
 }
@@ -373,8 +373,16 @@ ALGO_BYTES_DEFECT = {"split_step": (40.0, "interior"), "ensemble_step": (40.0, "
 # The drop-in's media-table grid reads an int media index instead of K, phi (props: P, S, media, and the
 # copy of the caller's state and its densities written; flux/Newton: media in place of phi).
 # Split mode: read dP, S (8), media (4), M1, M2 (16); write dP, S (8), M1, M2 (16).
-ALGO_BYTES_DROPIN = {"f64_props": (84.0, "all"), "f64_flux_newton": (60.0, "interior"),
+ALGO_BYTES_DROPIN = {"f64_props": (84.0, "all"), "f64_flux_newton": (68.0, "interior"),
                      "split_step": (52.0, "interior")}
+
+
+def algo_bytes(form, kernel):
+    """(bytes per cell, which cells) of the timed steps: the workloads hold DNAPL at their sources only, and a
+    cell without leaves P_k (FP64 passes) or the DNAPL mass (split forms) where they are."""
+    table = ALGO_BYTES_DROPIN if form in DROPIN_MODES else ALGO_BYTES_DEFECT if form == "splitdefect" else ALGO_BYTES
+    bpc, which = table.get(kernel, ALGO_BYTES.get(kernel, (0.0, "all")))
+    return max(0.0, bpc - (4.0 if form == "splitdefect" else 8.0)), which
 
 
 def timed(runner, steps, stream, world):
@@ -531,8 +539,7 @@ def run_ours(args, rank, world):
     hbm, peak_kind = peaks()
     kname, (kms, klaunch) = max(ktimes.items(), key=lambda kv: kv[1][0])
     per_launch_s = kms / 1e3 / max(klaunch, 1)
-    table = ALGO_BYTES_DROPIN if p in DROPIN_MODES else ALGO_BYTES_DEFECT if p == "splitdefect" else ALGO_BYTES
-    bpc, which = table.get(kname, ALGO_BYTES.get(kname, (0.0, "all")))
+    bpc, which = algo_bytes(p, kname)
     algo = bpc * (icells if which == "interior" else cells)
     achieved = algo / per_launch_s / 1e9 if per_launch_s > 0 else 0.0
     traffic = None
@@ -549,7 +556,7 @@ def run_ours(args, rank, world):
             "binding_resource": ("instruction issue, and beside it the FP64 pipe (ncu: 72% issue active, "
                                  "46% of FP64-pipe cycles active in the flux/Newton pass)") if f64 else
                                 ("instruction issue and the per-plane block barrier (algorithmic bytes are those of "
-                                 "a cell with DNAPL; others leave the DNAPL mass, 8 or 4 bytes, unwritten)"),
+                                 "a cell without DNAPL, which leaves its DNAPL mass, 8 or 4 bytes, unwritten)"),
             "ms_per_step_with_kernel_events": ms_k / args.steps}
     if f64:  # the FP64 pipe beside it, from the ncu capture of this pass
         roof["fp64_pipe"] = {"frac": 0.464, "metric": "sm__pipe_fp64_cycles_active",
@@ -672,7 +679,7 @@ def run_ours(args, rank, world):
 
 
 def compare(pkg, members, prec, ensemble, steps, flags=0):
-    """The same members advanced `steps` steps in form `prec` and in plain FP64
+    """The same members advanced `steps` steps in form `prec` and in FP64
     on the GPU: both states and both phase-mass histories."""
     abi = pkg.abi
 
@@ -698,7 +705,7 @@ def compare(pkg, members, prec, ensemble, steps, flags=0):
     moved = max(float(np.abs(b[1] - m.initial_state()[1]).max()) for b, m in zip(ref, members))
     scale = np.maximum(np.abs(mr), 1e-300)
     drift = float(np.max(np.abs(mg - mr) / scale * (np.abs(mr) > 0)))
-    block = {"vs": "plain FP64 GPU path of the same members (pinned to the oracle at 1e-12)", "steps": steps,
+    block = {"vs": "FP64 GPU path of the same members (pinned to the oracle at 1e-12)", "steps": steps,
              "max_dS": ds, "rel_l2_P": (num / den) ** 0.5, "phase_mass_rel_diff_max": drift, "S_moved_max": moved,
              "status": [int(s1), int(s2)]}
     if cfl is not None:
@@ -729,7 +736,7 @@ def accuracy_dropin(pkg, member, steps=20):
 
 
 def accuracy_block(pkg, O, members, prec, ensemble, steps=20):
-    """The measured form against plain FP64 on the same members and steps
+    """The measured form against FP64 on the same members and steps
     (the GPU FP64 path, itself pinned to the oracle at 1e-12), and against
     the oracle on the smallest member: max|dS|, relative L2 of P, relative
     phase-mass difference per step, and how far S moved (max|S - S0|)."""
