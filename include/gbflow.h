@@ -41,8 +41,9 @@ enum { GBF_SOURCE_DIRICHLET_PATCH = 0, /* reference: S2 = S2_gr on the top patch
 enum { GBF_BC_REFERENCE = 0,           /* reference Border_S2/Border_P1 rules           */
        GBF_BC_HYDROSTATIC_SIDES = 1 }; /* Dirichlet hydrostatic P on i/k sides,
                                           no-flow bottom face for both phases          */
-enum { GBF_PREC_F64 = 0,               /* FP64 state; a step's increments to FP64 accuracy of
-                                          the state (FP32 pairs where that is faster)   */
+enum { GBF_PREC_F64 = 0,               /* FP64 state; a step's increments from FP32 pairs (about
+                                          2^-46 of themselves) or, where that or FP32's range
+                                          would not do for FP64 results, in FP64        */
        GBF_PREC_SPLIT = 1,             /* FP32 P,S,K,fluxes; phase masses at least as precise
                                           as FP64: FP32-pair defects over the state's exact
                                           FP32-product mass; after the FP32 Newton step one
@@ -89,8 +90,10 @@ typedef struct gbf_model {
   double kv;                      /* vertical/horizontal permeability ratio (1 = isotropic) */
   double newton_tol;              /* 0: always run newton_iterations (reference);
                                      >0: stop once |dS| and |dP|/P_atm fall below it.
-                                     FP64 domains and ensembles of 7 or more iterations
-                                     solve to round-off whatever its value */
+                                     Where FP64 domains, ensembles and the fused drop-in
+                                     form a cell's increments from FP32 pairs (7 or more
+                                     iterations), its Newton runs to round-off instead,
+                                     in 7 steps at most, whatever both values */
 } gbf_model;
 
 /*

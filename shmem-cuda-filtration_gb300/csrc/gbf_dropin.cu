@@ -24,11 +24,12 @@
 //     calls as one fused step that writes P1, S2, ro1, ro2 only; the other
 //     arrays of the step (P2, Xi, velocities, roS, roS_old) are computed when
 //     the host reads one of them, from the state the step started from, with
-//     the same kernels as the one-call-per-stage mode. Its Newton stops once
-//     an iteration moves S by less than 1e-11 and P by less than 1e-11 P
-//     (at most the reference's 7 iterations): the same results to round-off
-//     (the tests hold both modes to the oracle at 1e-12) in about a third of
-//     the time, since every FP64 iteration costs a log and an exp per cell.
+//     the same kernels as the one-call-per-stage mode. Its Newton runs to
+//     round-off in FP32-pair increments; cells and models that those do not
+//     hold take FP64, which stops once an iteration moves S by less than 1e-11
+//     and P by less than 1e-11 P (at most the reference's 7 iterations): the
+//     same results to round-off (the tests hold both modes to the oracle at
+//     1e-12).
 #include <stdio.h>
 #include <stdlib.h>
 
@@ -59,7 +60,7 @@ int initial_mode() {
   return e[0] == '1' ? 1 : e[0] == '2' ? 2 : 0;
 }
 int g_mode = initial_mode();
-constexpr double kFusedNewtonTol = 1e-11;  // converge-and-exit Newton of the fused mode
+constexpr double kFusedNewtonTol = 1e-11;  // converge-and-exit Newton of the fused mode's FP64 cells and passes
 
 gbf_model model_from(const consts& def, int localNx) {
   gbf_model m;
