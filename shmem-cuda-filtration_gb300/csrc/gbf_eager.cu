@@ -72,7 +72,7 @@ __device__ __forceinline__ double exact_div(double a, const Recip& d) {
     q = __fma_rn(__fma_rn(-q, d.b, a), d.r, q);
     return __fma_rn(__fma_rn(-q, d.b, a), d.r, q);
   }
-  if (gbf_is_zero(a) && d.b > 0.) return a;
+  if (gbf_is_zero(a) && (unsigned)__double2hiint(d.b) - 1u < 0x7fefffffu) return a;  // b > 0 and finite, without the FP64 unit
   return plain_div(a, d.b);
 }
 
@@ -82,7 +82,7 @@ struct EagerConsts {
   double e1[2], e2[2], mil[2], mil1[2];  // Brooks-Corey exponents; -1/lambda, -1/lambda - 1
   Recip om_swr[2], lam_swr[2];           // 1 - S_wr, lambda (1 - S_wr)
   double PkS1[2];                        // dP_k/dS at S_e = 1
-  bool one[2];                           // S = 0 is S_e = 1, its P_k and slope finite (no model of use is not so)
+  bool one;                              // S = 0 is S_e = 1, its P_k and slope finite, in both media (every model of use)
   double Xi1w[2];                        // Xi1 of the table's K at S_e = 1
   Recip mu1, mu2, h1, h2, h3, hh1, hh2, hh3;  // hh: 2 h
   double dtphi[2];                       // dt / phi of the table
@@ -90,6 +90,7 @@ struct EagerConsts {
 };
 EagerConsts eager_consts(const gbf_model& m) {
   EagerConsts C;
+  C.one = true;
   for (int md = 0; md < 2; md++) {
     const double lam = m.lambda[md], swr = m.S_wr[md];
     C.e1[md] = (2. + 3. * lam) / lam;
@@ -99,7 +100,7 @@ EagerConsts eager_consts(const gbf_model& m) {
     C.om_swr[md] = recip(1 - swr);
     C.lam_swr[md] = recip(lam * (1 - swr));
     C.PkS1[md] = m.P_d[md] / (lam * (1 - swr));
-    C.one[md] = (1. - swr) / (1. - swr) == 1. && isfinite(C.PkS1[md]) && isfinite(m.P_d[md]);
+    C.one = C.one && (1. - swr) / (1. - swr) == 1. && isfinite(C.PkS1[md]) && isfinite(m.P_d[md]);
     C.Xi1w[md] = -1. * m.K[md] / m.mu1;
     C.dtphi[md] = m.dt / m.m[md];
   }
@@ -166,7 +167,7 @@ __global__ void k_props(const gbf_model m, const EagerConsts C, gbf_arrays a, gb
       S2 = a.S2[c];
       P1 = a.P1[c];
     }
-    const bool wet = mine && !(gbf_is_zero(S2) && C.one[md]);
+    const bool wet = mine && !(gbf_is_zero(S2) && C.one);
     const bool some = pow_jobs(jobs, wet, wet, S2, md, m, C, C.e1, C.e2, [](int k, int, double S_e, double p) {
       return k ? (1. - S_e) * (1. - S_e) * (1 - p) : p;
     });
@@ -374,7 +375,7 @@ __global__ void k_newton(const gbf_model m, const EagerConsts C, gbf_arrays a, g
     const double pd = m.P_d[md];
     // Without DNAPL (S2 = 0, roS2 = 0) every product with S2 is zero, dS too,
     // and the step in P1 is the one of the general form with those zeros left out.
-    if (mine && C.one[md] && gbf_is_zero(S2) && gbf_is_zero(roS2) && gbf_is_finite(P1) && gbf_is_finite(roS1) && !tol) {
+    if (mine && C.one && gbf_is_zero(S2) && gbf_is_zero(roS2) && gbf_is_finite(P1) && gbf_is_finite(roS1) && !tol) {
       const double F1P = m.ro01 * (m.beta1);
       double Pb = P1;
       for (int w = 1; w <= N; w++) {
@@ -395,7 +396,7 @@ __global__ void k_newton(const gbf_model m, const EagerConsts C, gbf_arrays a, g
     }
     double Pb = P1, Sb = S2, Sk = 0., P_k = 0., SPkS = 0., omS = 0., F1P = 0., F2P = 0.;  // b: the point before
     for (int w = 1; w <= N; w++) {
-      const bool moved = active && (w == 1 || !same_bits(S2, Sk)), wet = moved && !(gbf_is_zero(S2) && C.one[md]);
+      const bool moved = active && (w == 1 || !same_bits(S2, Sk)), wet = moved && !(gbf_is_zero(S2) && C.one);
       // P_k and dP_k/dS where S2 moved (at S_e = 1 without pow)
       if (!pow_jobs(jobs, active, wet, S2, md, m, C, C.mil, C.mil1, [&](int k, int d, double, double p) {
             const double v = m.P_d[d] * p;
