@@ -4,7 +4,8 @@
 // DFMA against 6.7 TB/s of HBM): any step whose arithmetic is FP64 is bound
 // by that pipe (measured 8.73 ms a step at 256^3: 85% of it active, DRAM at
 // 4%). The step therefore forms its increments in FP32 pairs
-// (gbf_f64_pair.cuh) and touches the FP64 pipe for five additions a cell:
+// (gbf_f64_pair.cuh) and takes the FP64 pipe 6 warp instructions per 32 cells
+// without DNAPL (with phase masses), about 25 with:
 //   pass 1 (k_pair_props, every cell): pressure against the row's hydrostatic
 //     value, mobility x density of both phases, capillary pressure, as pairs
 //     (32 bytes a cell written, 24 without DNAPL);
@@ -15,9 +16,10 @@
 // Newton, so they are not computed again for halos, and the 64 bytes a cell
 // that this moves beside the state are hidden behind the arithmetic. Both are
 // bound by instruction issue, with the FP64 pipe about half busy; 256^3,
-// heterogeneous, a fifth of the cells with DNAPL: pass 1 204 us (223 with the
-// DNAPL mobility formed and P_k stored in every cell), pass 2 445 us (2.2 and
-// 2.4 TB/s of 44 and 62 bytes a cell), where the FP64 passes took 2460 and
+// heterogeneous, a fifth of the cells with DNAPL: pass 1 201 us (223 with the
+// DNAPL mobility formed and P_k stored in every cell), pass 2 456 us (3.7 and
+// 2.2 TB/s of 44 and 62 bytes a cell; 445 without the looks for cells that
+// pairs do not hold), where the FP64 passes took 2460 and
 // 6270. Pass 1 keeps to 32 registers for eight blocks an SM: at 40 it takes 226
 // us, and on small grids fewer blocks of the next kernel fit beside it (40
 // steps of 40^3 778 -> 881 us). Pass 2 takes 64 registers for four blocks an SM:
@@ -25,9 +27,10 @@
 // (627, 764).
 //   face pass (k_f64_boundary): the reference's sweep-ordered boundary
 //     values (cpu.cpp:44-54, 323-403) into the next state.
-// A model with fewer Newton iterations than the reference's 7 runs the plain
-// FP64 passes (k_f64_props, k_f64_flux_newton; per-cell code in
-// gbf_f64_cell.cuh): its iterates stop before convergence.
+// A model with fewer Newton iterations than the reference's 7, whose iterates
+// stop before convergence, and one whose constants do not fit FP32 pairs run the
+// plain FP64 passes (k_f64_props, k_f64_flux_newton; per-cell code in
+// gbf_f64_cell.cuh).
 #include "gbf_f64_cell.cuh"
 #include "gbf_f64_pair.cuh"
 
@@ -108,7 +111,9 @@ __global__ void __launch_bounds__(kThreads) k_f64_boundary(const gbf_model m, co
 namespace {
 // Block size of the pair step's passes over n cells: 64 where 256 would leave
 // less than a few blocks an SM. Time of a step with 256, 128, 64, 32 threads:
-// 40^3 17.3, 15.9, 15.1, 14.8 us; 64^3 25.5, 23.8, 23.4, 26.4 us.
+// 40^3 17.3, 15.9, 15.1, 14.8 us; 64^3 25.5, 23.8, 23.4, 26.4 us; with 256 and
+// 64 threads 68^3 (the cut) 28.9, 26.3, 80^3 34.7, 34.0, 96^3 51.2, 50.6,
+// 112^3 74.7, 75.1.
 unsigned pair_threads(size_t n) { return n < (size_t)gbf_num_sms() * 2048 ? 64u : (unsigned)kThreads; }
 }  // namespace
 
@@ -140,7 +145,8 @@ int gbf_f64_launch_step(const gbf_model& m, const GbfDerived& d, const gbf_cells
   const unsigned fg = gbf_f64_flux_grid(m);
   const bool mass = s.mass_partials && mass_out;
   cudaError_t err = cudaSuccess;
-  // programmatic launches up to 4M cells (256^3: 613 us a step without, 619 with)
+  // programmatic launches up to 4M cells. us a step with, without: 40^3 15.0, 20.1; 96^3 51.2, 54.1; 128^3 108.7,
+  // 104.9; 144^3 150.9, 151.1; 160^3 (4.1M) 181.3, 186.8; 176^3 242, 237; 256^3 669, 661
   const bool pdl = g.n < (4u << 20);
   unsigned threads = kThreads;
   auto go = [&](auto kern, unsigned blocks, auto... args) {

@@ -34,11 +34,12 @@
 //     away the cell's face potentials are taken from FP64 differences. So are
 //     those at pressures above 32 / beta1, where the water's weight is that of
 //     32 times its density and fluxes of 2^3 of the limit above cancel.
-// What the looks for these cost where no cell is refused: 256^3 640 -> 655 us a
-// step. Where many are (192^3, all wet, us a step; 613 with none): all of them
-// 10,000 Pa off hydrostatic with the reference's compressibilities 1020; noise
-// of 10,000 Pa 20,900; S_e 1e-6 17,800, more than the plain passes' (about 3700),
-// which form each mobility once.
+// The looks for these cost 20 of 650 us a step at 256^3 where no cell is refused.
+// Where many are (192^3, us a step): 10,000 Pa off hydrostatic everywhere with
+// the reference's compressibilities, all wet 624 -> 1030, all dry 176 -> 460;
+// noise of 10,000 Pa 20,800 and 2400; S_e 1e-6 everywhere 18,200. The plain
+// passes take about 3700, since they form each mobility once; cells like these
+// are few in a state that time steps have smoothed.
 // S below about 1e-13 has no mobility in pairs (om^3 is below FP32's range; in
 // FP64 it would move 1e-26 of itself a step).
 #pragma once
