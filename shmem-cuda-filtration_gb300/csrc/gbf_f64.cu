@@ -17,8 +17,8 @@
 // that this moves beside the state are hidden behind the arithmetic. Both are
 // bound by instruction issue, with the FP64 pipe about half busy; 256^3,
 // heterogeneous, a fifth of the cells with DNAPL: pass 1 201 us (223 with the
-// DNAPL mobility formed and P_k stored in every cell), pass 2 456 us (3.7 and
-// 2.2 TB/s of 44 and 62 bytes a cell; 445 without the looks for cells that
+// DNAPL mobility formed and P_k stored in every cell), pass 2 470 us (3.7 and
+// 2.2 TB/s of 44 and 62 bytes a cell; 447 without the looks for cells that
 // pairs do not hold), where the FP64 passes took 2460 and
 // 6270. Pass 1 keeps to 32 registers for eight blocks an SM: at 40 it takes 226
 // us, and on small grids fewer blocks of the next kernel fit beside it (40

@@ -34,7 +34,7 @@
 //     away the cell's face potentials are taken from FP64 differences. So are
 //     those at pressures above 32 / beta1, where the water's weight is that of
 //     32 times its density and fluxes of 2^3 of the limit above cancel.
-// The looks for these cost 20 of 650 us a step at 256^3 where no cell is refused.
+// The looks for these cost 24 of 660 us a step at 256^3 where no cell is refused.
 // Where many are (192^3, us a step): 10,000 Pa off hydrostatic everywhere with
 // the reference's compressibilities, all wet 624 -> 1030, all dry 176 -> 460;
 // noise of 10,000 Pa 20,800 and 2400; S_e 1e-6 everywhere 18,200. The plain
@@ -640,10 +640,11 @@ static __device__ __noinline__ double2 pair_cell_again(const GbfPairConsts& C, c
 // Pass 2 at interior cells t0, t0 + stride, .. below t1, summed into acc; every
 // thread of the block calls it. The cells that the pairs refuse are taken after
 // the others: calls among the pair arithmetic cost it registers (256^3, none
-// refused: pass 2 488 us with them there, 456 after the others). Up to an eighth
-// of a block's cells, they are listed and shared out evenly, in a fixed order: a
-// warp pays for the FP64 of one lane what it pays for 32. More than that, a
-// thread takes its own, whose neighbours' are in its warp.
+// refused: pass 2 488 us with them there, 470 after the others, 447 without
+// any). Up to an eighth of a block's cells, they are listed and shared out
+// evenly, in a fixed order: a warp pays for the FP64 of one lane what it pays
+// for 32. More than that, a thread takes its own, whose neighbours' are in its
+// warp.
 template <bool MASS>
 __device__ __forceinline__ void gbf_pair_step_cells(const GbfPairConsts& C, const gbf_model& m, const GbfDerived& d,
                                                     const gbf_cells& cells, const GbfF64Step& s, const GbfPairWork& w,
@@ -667,6 +668,7 @@ __device__ __forceinline__ void gbf_pair_step_cells(const GbfPairConsts& C, cons
   };
 #ifdef __CUDACC__
   if (!__syncthreads_or(first < t1)) return;
+  // 512 B: with 2 KB a block programmatic launches no longer overlap (40 steps of 40^3 788 -> 942 us)
   constexpr unsigned kList = 128;
   __shared__ unsigned list[kList], warps[32];
   unsigned n = 0;  // this thread's
